@@ -49,10 +49,14 @@ constexpr int QBLK_BYTES = 128 * 128;    // 128 rows x 64 bf16
 constexpr int QN_BYTES = 4096;           // 128 rows x 16 bf16 (padded to 4 KB)
 constexpr int BN_BYTES = 256 * 32;       // 256 rows x 16 bf16
 constexpr int TMEM_COLS = 512;
+constexpr int HQ_LD = 36;  // floats per row of a hit queue: 32 values, threshold, lane, column
+// rows of a selection warp's hit queue (THRESH); fewer where the resident
+// query tile of a split pass leaves no room beside three stages
+__host__ __device__ constexpr int hq_rows(int nkb) { return nkb <= 4 ? 8 : 4; }
 
 struct Layout {
   int nkb, S, C, mode;
-  size_t q_off, qn_off, stg_off, stage_bytes, list_off, bar_off, total;
+  size_t q_off, qn_off, stg_off, stage_bytes, list_off, hq_off, bar_off, total;
 };
 
 // qs: the query tile is streamed with each K block (stage = B block + A block)
@@ -73,6 +77,8 @@ __host__ __device__ inline Layout make_layout(int nkb, int S, int mode, int C, b
   L.list_off = off;
   if (mode != SCAN_THRESH) off += (size_t)(C > 16 ? N_EPI : 128) * C * 8;
   off = (off + 15) & ~(size_t)15;
+  L.hq_off = off;
+  if (mode == SCAN_THRESH) off += (size_t)(N_EPI / 32) * hq_rows(nkb) * HQ_LD * 4;
   L.bar_off = off; off += (size_t)(2 * S + 8) * 8 + 16;
   L.total = off + 1024;  // alignment slack for the 1024-byte aligned base
   return L;
@@ -329,23 +335,29 @@ __global__ void __launch_bounds__(NT_TC, 1)
       }
     }
   } else if (warp == 1) {
-    // ---------------- MMA issuer (the leader's, for a pair)
-    if (lane == 0 && leader) {
+    // ---------------- MMA issuer (the leader's, for a pair).  The whole warp
+    // runs the loop and one elected lane issues: the operands stay in uniform
+    // registers.
+    if (leader) {
+      const bool el = elect_one();
       const uint32_t idesc = idesc_16_f32(PAIR ? 2 * TC_TILE_M : TC_TILE_M, TC_TILE_N, sel.f16 != 0);
       bool ok = true, any = false;
       int sn = 0;
       uint32_t phn = 0;
       int it = 0, ui = 0;
+      const uint32_t stg0 = smem_u32(Stg), q0s = smem_u32(Qs), qns = smem_u32(Qn);
       for (int w = w0; w < nunits && ok; w += wstep, ui++) {
       const UnitInfo un = unit_info(w);
+      const int t_begin = __shfl_sync(0xffffffffu, un.t_begin, 0);
+      const int t_end = __shfl_sync(0xffffffffu, un.t_end, 0);
       if (!QS) {
-        if (!mbar_wait(qfull, (uint32_t)(ui & 1), abort_flag, wl)) { ok = false; break; }
+        if (!mbar_wait_warp(qfull, (uint32_t)(ui & 1), abort_flag, wl)) { ok = false; break; }
         tc_fence_after();
       }
-      for (int t = un.t_begin; t < un.t_end && ok; t++, it++) {
+      for (int t = t_begin; t < t_end; t++, it++) {
         const int a = it & 1;
         const uint32_t u = (uint32_t)(it >> 1);
-        if (!mbar_wait(&tempty[a], (u & 1) ^ 1, abort_flag, wl)) { ok = false; break; }
+        if (!mbar_wait_warp(&tempty[a], (u & 1) ^ 1, abort_flag, wl)) { ok = false; break; }
         tc_fence_after();
         const uint32_t dt = tmem + (uint32_t)(a * TC_TILE_N);
         for (int ks = 0; ks < nks; ks++) {
@@ -355,13 +367,17 @@ __global__ void __launch_bounds__(NT_TC, 1)
           // TMA data: its arrival is tracked by the barrier's transaction
           // count, no tcgen05 fence is needed (a fence here would stall the
           // MMA pipe once per stage)
-          if (!mbar_wait(&full[s], ph, abort_flag, wl)) { ok = false; break; }
-          const uint32_t sb = smem_u32(Stg + (size_t)s * SB);
+          if (!mbar_wait_warp(&full[s], ph, abort_flag, wl)) { ok = false; break; }
+          const uint32_t sb = stg0 + (uint32_t)s * (uint32_t)SB;
           // a descriptor's start address field is addr >> 4 in its low 14 bits
           // (shared addresses < 256 KB): offsets are added to a base descriptor
-          {
-            const uint32_t sa = QS ? sb + BHALF : smem_u32(Qs + ks * QBLK_BYTES);
-            const uint64_t da = desc_k_sw128(sa), db = desc_k_sw128(sb);
+          const uint32_t sa = QS ? sb + BHALF : q0s + (uint32_t)(ks * QBLK_BYTES);
+          const uint64_t da = desc_k_sw128(sa), db = desc_k_sw128(sb);
+          const uint32_t sn_ = sb + BHALF + (QS ? QBLK_BYTES : 0);
+          const uint64_t dq = desc_k_sw32(QS ? sn_ + BN_BYTES : qns);
+          const uint64_t dbn = desc_k_sw32(sn_);
+          const bool lastk = L2 && ks == nkb - 1;
+          if (el) {
 #pragma unroll
             for (int kk = 0; kk < 4; kk++) {
               const uint32_t acc = (ks > 0 || kk > 0) ? 1u : 0u;
@@ -370,32 +386,31 @@ __global__ void __launch_bounds__(NT_TC, 1)
               else
                 umma_bf16(dt, da + (uint64_t)(kk * 2), db + (uint64_t)(kk * 2), idesc, acc);
             }
-            if (L2 && ks == nkb - 1) {  // the norm fold: one more K=16 step
-              const uint32_t sn_ = sb + BHALF + (QS ? QBLK_BYTES : 0);
-              const uint64_t dq = desc_k_sw32(QS ? sn_ + BN_BYTES : smem_u32(Qn));
-              const uint64_t dbn = desc_k_sw32(sn_);
+            if (lastk) {  // the norm fold: one more K=16 step
               if (PAIR)
                 umma_bf16_pair(dt, dq, dbn, idesc, 1u);
               else
                 umma_bf16(dt, dq, dbn, idesc, 1u);
             }
+            if (PAIR)
+              umma_commit_pair_mc(&empty[s], 3);
+            else
+              umma_commit(&empty[s]);
           }
           any = true;
-          if (PAIR)
-            umma_commit_pair_mc(&empty[s], 3);
-          else
-            umma_commit(&empty[s]);
         }
         if (!ok) break;
-        if (PAIR)
-          umma_commit_pair_mc(&tfull[a], 3);
-        else
-          umma_commit(&tfull[a]);
+        if (el) {
+          if (PAIR)
+            umma_commit_pair_mc(&tfull[a], 3);
+          else
+            umma_commit(&tfull[a]);
+        }
       }
       // release the resident query tile once this unit's MMAs are done
-      if (!QS && PERSIST && ok) umma_commit(qempty);
+      if (!QS && PERSIST && ok && el) umma_commit(qempty);
       }
-      if (!PAIR && any) {
+      if (!PAIR && any && el) {
         // every MMA issued has finished with TMEM and shared memory
         umma_commit(mdone);
         mbar_wait_drain(mdone, 0);
@@ -406,9 +421,10 @@ __global__ void __launch_bounds__(NT_TC, 1)
         for (int e = it; e < it + 2 && ok; e++) {
           const int a = e & 1;
           const uint32_t u = (uint32_t)(e >> 1);
-          if (!mbar_wait(&tempty[a], (u & 1) ^ 1, abort_flag, wl)) ok = false;
+          if (!mbar_wait_warp(&tempty[a], (u & 1) ^ 1, abort_flag, wl)) ok = false;
         }
       }
+      __syncwarp();
     }
   } else {
     // ---------------- selection warps
@@ -418,6 +434,9 @@ __global__ void __launch_bounds__(NT_TC, 1)
     const int row = grp * 32 + lane;
     const int tslot = ew * 32 + lane;      // 0..255
     const uint32_t lane_base = (uint32_t)(grp * 32) << 16;
+    const int hqn = hq_rows(nkb);
+    float *Hq = reinterpret_cast<float *>(base + lay.hq_off) + ew * (hqn * HQ_LD);
+    int hq = 0;  // rows queued (THRESH)
     int it = 0;
     bool ok = true;
     for (int w = w0; w < nunits && ok; w += wstep) {
@@ -494,33 +513,78 @@ __global__ void __launch_bounds__(NT_TC, 1)
       }
     };
 
-    // One 32-column chunk already in registers.  The loop body must stay small
-    // (the selection warps run it from the instruction cache): a min tree and
-    // one warp vote per chunk; only when some lane's chunk minimum passes its
-    // bound (true when min < bound or min is NaN) does the warp build each
-    // lane's hit mask and walk its hits, extracting each value with a select
-    // tree instead of unrolled per-element code.
-    auto process = [&](const uint32_t (&r)[32], int jc) {
+    // THRESH: the queued rows of 32 columns, each with a value <= its lane's
+    // threshold.  The whole warp looks at a row at a time (lane = column): the
+    // hits, in column order, go to the next slots of the row's region.
+    // (cbase of lane l is that of lane 0 plus l * cap.)
+    const long cbase0 = MODE == SCAN_THRESH ? __shfl_sync(0xffffffffu, cbase, 0) : 0;
+    auto drain = [&]() {
+      __syncwarp();
+#pragma unroll 2
+      for (int e = 0; e < hq; e++) {
+        const float *xr = Hq + e * HQ_LD;
+        const float4 meta = *reinterpret_cast<const float4 *>(xr + 32);
+        const int src = __float_as_int(meta.y), j = __float_as_int(meta.z) + lane;
+        const float x = xr[lane];
+        const bool hit = x <= meta.x && j < nbv;
+        const uint32_t m = __ballot_sync(0xffffffffu, hit);
+        const int pos = __shfl_sync(0xffffffffu, rcount, src) + __popc(m & ((1u << lane) - 1u));
+        if (hit && pos < cap) {
+          const long o = cbase0 + (long)src * cap + pos;
+          sel.candv[o] = x;
+          sel.candi[o] = j + id_off;
+        }
+        if (lane == src) rcount += __popc(m);
+      }
+      hq = 0;
+      __syncwarp();
+    };
+
+    // THRESH: one 32-column chunk in registers with a chunk minimum <= the
+    // lane's threshold in the lanes of pm.  They only write their values to the
+    // warp's hit queue, which is drained while the next accumulator is not
+    // ready: the accumulators are handed back at the pace of the slowest of
+    // eight warps, so a hit costs the pass less the shorter it holds its warp.
+    auto push = [&](const uint32_t (&r)[32], uint32_t pm, int jc) {
+      while (pm) {
+        const int rank = hq + __popc(pm & ((1u << lane) - 1u));
+        const bool on = pm >> lane & 1u;
+        if (on && rank < hqn) {
+          float4 *xr = reinterpret_cast<float4 *>(Hq + rank * HQ_LD);
+#pragma unroll
+          for (int i = 0; i < 8; i++)
+            xr[i] = make_float4(__uint_as_float(r[4 * i]), __uint_as_float(r[4 * i + 1]),
+                                __uint_as_float(r[4 * i + 2]), __uint_as_float(r[4 * i + 3]));
+          xr[8] = make_float4(thr, __int_as_float(lane), __int_as_float(jc), 0.f);
+        }
+        hq += __popc(pm);
+        if (hq < hqn) break;
+        pm = __ballot_sync(0xffffffffu, on && rank >= hqn);
+        hq = hqn;
+        drain();
+      }
+    };
+
+    // Lists: one 32-column chunk already in registers, mc its minimum.  The
+    // loop body must stay small (the selection warps run it from the
+    // instruction cache): one warp vote per chunk; only when some lane's chunk
+    // minimum passes its bound (true when min < bound or min is NaN) does the
+    // warp build each lane's hit mask and walk its hits, extracting each value
+    // with a select tree instead of unrolled per-element code.
+    auto process = [&](const uint32_t (&r)[32], float mc, int jc) {
       float v[32];
 #pragma unroll
       for (int i = 0; i < 32; i++) v[i] = __uint_as_float(r[i]);
+      // lists: a superset filter (update() keeps the strict x < lmax)
+      const float bnd = fminf(lmax, tb);
+      const bool pass = rvalid && !(mc > bnd);
+      if (!__any_sync(0xffffffffu, pass)) return;
+      if (!pass) return;
       if (jc + 32 > nbv) {
 #pragma unroll
         for (int i = 0; i < 32; i++)
           if (jc + i >= nbv) v[i] = NAN;
       }
-      float m8[4];
-#pragma unroll
-      for (int g = 0; g < 4; g++)
-        m8[g] = fmin3(fmin3(v[8 * g], v[8 * g + 1], v[8 * g + 2]),
-                      fmin3(v[8 * g + 3], v[8 * g + 4], v[8 * g + 5]),
-                      fminf(v[8 * g + 6], v[8 * g + 7]));
-      const float mc = fminf(fminf(m8[0], m8[1]), fminf(m8[2], m8[3]));
-      // lists: a superset filter (update() keeps the strict x < lmax)
-      const float bnd = MODE == SCAN_THRESH ? thr : fminf(lmax, tb);
-      const bool pass = rvalid && !(mc > bnd);
-      if (!__any_sync(0xffffffffu, pass)) return;
-      if (!pass) return;
       uint32_t bits = 0;
 #pragma unroll
       for (int i = 0; i < 32; i++) {
@@ -555,14 +619,15 @@ __global__ void __launch_bounds__(NT_TC, 1)
       // two register sets: the load of chunk c+1 is in flight while chunk c is
       // scanned; the loop keeps one copy of the chunk code per register set
       uint32_t r0[32], r1[32], r2[32], r3[32];
-      tmem_ld32(tcol, r0);
-      tmem_ld32(tcol + 32, r1);
-      tmem_ld32(tcol + 64, r2);
-      tmem_ld32(tcol + 96, r3);
-      tmem_ld_wait(r0);
-      tmem_ld_wait(r1);
-      tmem_ld_wait(r2);
-      tmem_ld_wait(r3);
+      uint32_t m0, m1, m2, m3;
+      tmem_ld32_min(tcol, r0, m0);
+      tmem_ld32_min(tcol + 32, r1, m1);
+      tmem_ld32_min(tcol + 64, r2, m2);
+      tmem_ld32_min(tcol + 96, r3, m3);
+      tmem_ld_wait(r0, m0);
+      tmem_ld_wait(r1, m1);
+      tmem_ld_wait(r2, m2);
+      tmem_ld_wait(r3, m3);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) {
@@ -577,11 +642,33 @@ __global__ void __launch_bounds__(NT_TC, 1)
         tb = INFINITY;
         if (t == t_begin && j0 + 128 <= nbv) tb = cth_bound<C>(r0, r1, r2, r3);
       }
-      process(r0, j0);
-      process(r1, j0 + 32);
-      process(r2, j0 + 64);
-      process(r3, j0 + 96);
+      if (MODE == SCAN_THRESH) {
+        // (thr is NaN in lanes without a query; an all-NaN chunk has no hit)
+        const float f0 = __uint_as_float(m0), f1 = __uint_as_float(m1);
+        const float f2 = __uint_as_float(m2), f3 = __uint_as_float(m3);
+        if (__any_sync(0xffffffffu, fminf(fminf(f0, f1), fminf(f2, f3)) <= thr)) {
+          const uint32_t p0 = __ballot_sync(0xffffffffu, f0 <= thr);
+          const uint32_t p1 = __ballot_sync(0xffffffffu, f1 <= thr);
+          const uint32_t p2 = __ballot_sync(0xffffffffu, f2 <= thr);
+          const uint32_t p3 = __ballot_sync(0xffffffffu, f3 <= thr);
+          push(r0, p0, j0);
+          push(r1, p1, j0 + 32);
+          push(r2, p2, j0 + 64);
+          push(r3, p3, j0 + 96);
+        }
+        if (hq) {
+          const int it1 = it + 1;
+          const bool ready = mbar_test_wait(&tfull[it1 & 1], (uint32_t)((it1 >> 1) & 1));
+          if (!__any_sync(0xffffffffu, ready)) drain();
+        }
+      } else {
+        process(r0, __uint_as_float(m0), j0);
+        process(r1, __uint_as_float(m1), j0 + 32);
+        process(r2, __uint_as_float(m2), j0 + 64);
+        process(r3, __uint_as_float(m3), j0 + 96);
+      }
     }
+    if (MODE == SCAN_THRESH && hq) drain();
     // a failed wait ends this unit's scan; the merge below still runs, so that
     // every selection warp reaches each named barrier
     if (MODE == SCAN_THRESH && rvalid) sel.cnt[rbase] = rcount;

@@ -48,6 +48,18 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity) {
   return ok != 0;
 }
 
+// whether the phase has completed, without waiting
+__device__ __forceinline__ bool mbar_test_wait(uint64_t *bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n .reg .pred p;\n mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+      " selp.u32 %0, 1, 0, p;\n}\n"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+
 // try_wait that may suspend the thread (no instruction issue) until the phase
 // completes or hint_ns elapse
 __device__ __forceinline__ bool mbar_try_wait_sleep(uint64_t *bar, uint32_t parity,
@@ -180,6 +192,26 @@ __device__ __forceinline__ void umma_commit(uint64_t *bar) {
       : "memory");
 }
 
+// true in one lane of a converged warp.  A warp that runs its issue loop with
+// all lanes and predicates only the tcgen05 instructions on this keeps their
+// operands (descriptors, TMEM address, instruction descriptor) warp-uniform;
+// inside an `if (lane == 0)` region each of them is moved to a uniform
+// register for every instruction.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t r;
+  asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n"
+               : "=r"(r));
+  return r != 0;
+}
+
+// mbar_wait by a whole converged warp; the result is the same in every lane
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t *bar, uint32_t parity,
+                                               volatile int *abort_flag, uint64_t limit_ns) {
+  bool ok = mbar_try_wait(bar, parity);
+  if (!__all_sync(0xffffffffu, ok)) ok = mbar_wait(bar, parity, abort_flag, limit_ns);
+  return __all_sync(0xffffffffu, ok);
+}
+
 // 32 consecutive fp32 columns of this thread's TMEM lane; the values are only
 // valid after tmem_ld_wait() on the same registers.
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
@@ -196,6 +228,20 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
       : "r"(taddr));
 }
 
+// tmem_ld32 that also returns the smallest of the 32 values (numbers only: NaN
+// where all of them are NaN), reduced by the load itself; as bits in m.
+__device__ __forceinline__ void tmem_ld32_min(uint32_t taddr, uint32_t (&r)[32], uint32_t &m) {
+  asm volatile(
+      "tcgen05.ld.red.sync.aligned.32x32b.x32.min.f32 "
+      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
+      "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, %32, [%33];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
+        "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
+        "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31]), "=r"(m)
+      : "r"(taddr));
+}
+
 // waits for this thread's outstanding tcgen05.ld; the registers are threaded
 // through so no use can be scheduled before the wait
 __device__ __forceinline__ void tmem_ld_wait(uint32_t (&r)[32]) {
@@ -208,6 +254,11 @@ __device__ __forceinline__ void tmem_ld_wait(uint32_t (&r)[32]) {
                  "+r"(r[27]), "+r"(r[28]), "+r"(r[29]), "+r"(r[30]), "+r"(r[31])
                :
                : "memory");
+}
+
+__device__ __forceinline__ void tmem_ld_wait(uint32_t (&r)[32], uint32_t &m) {
+  tmem_ld_wait(r);
+  asm volatile("" : "+r"(m)::"memory");
 }
 
 // ---- CTA-pair (cta_group::2) forms: one MMA spans the TMEM of two CTAs of a

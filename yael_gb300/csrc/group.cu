@@ -31,7 +31,7 @@ namespace yg {
 namespace {
 
 constexpr int kGroupTiles = 128;       // base tiles per main-pass unit
-constexpr int kSampleC = 12;           // threshold rank in the sample (knn.cu)
+constexpr int kSampleC = 13;           // threshold rank in the sample (knn.cu)
 
 // workspace slots of the grouped pipeline (disjoint from the per-call ones)
 enum GroupSlot : int {
@@ -126,7 +126,7 @@ struct Wave {
 // pair table for the final checks.  Two sets of buffers alternate between
 // consecutive waves, so wave i + 1 is packed while wave i's passes run.
 struct WaveState {
-  int np = 0, nq_all = 0, stride = 1, max_cand = 0;
+  int np = 0, nq_all = 0, stride = 1, max_cand = 0, blockmin = 0;
   long brows = 0;
   std::vector<GroupPair> hp;
   size_t n_mu = 0, n_su = 0;
@@ -158,6 +158,7 @@ int wave_prepare(const yael_gpu_knn_pair *pairs, const Wave &w, int d, int k, in
   const long P = (long)TC_TILE_N * stride;
   S.np = np;
   S.stride = stride;
+  S.blockmin = 0;
   // ---- layout
   std::vector<GroupPair> &hp = S.hp;
   hp.assign(np, GroupPair());
@@ -259,7 +260,7 @@ int wave_prepare(const yael_gpu_knn_pair *pairs, const Wave &w, int d, int k, in
         u.bend = g.boff + g.nb;
         u.pair = i;
         u.chunk = c;
-        u.pad_ = 0;
+        u.blockmin = 0;
         mu.push_back(u);
       }
     if (!hinf[i]) {  // the sample view: every stride-th row, tiles of 256 sampled rows
@@ -270,11 +271,13 @@ int wave_prepare(const yael_gpu_knn_pair *pairs, const Wave &w, int d, int k, in
         u.q0 = g.qoff + qt * TC_TILE_M;
         u.qend = g.qoff + g.nq;
         u.t_begin = sb0 / TC_TILE_N;
-        u.t_end = u.t_begin + (int)ceil_div(ns, TC_TILE_N);
-        u.bend = sb0 + ns;
+        u.blockmin = ns >= kSampleMin ? 1 : 0;  // whole super tiles of the sample
+        const int nsu = u.blockmin ? ns - ns % kSampleSuper : ns;
+        u.t_end = u.t_begin + (int)ceil_div(nsu, TC_TILE_N);
+        u.bend = sb0 + nsu;
         u.pair = i;
         u.chunk = 0;
-        u.pad_ = 0;
+        S.blockmin |= u.blockmin;
         su.push_back(u);
       }
     }
@@ -347,6 +350,7 @@ int wave_execute(WaveState &S, int d, int k, int metric, int max_ctas, cudaStrea
     ss.units = S.dsu;
     ss.nunits = (int)S.n_su;
     ss.gpairs = S.dpairs;
+    ss.blockmin = S.blockmin;
     ss.max_ctas = max_ctas;
     TcOperands ops;
     YG_CHECK(tc_base_view(op, S.stride, (int)(S.brows / S.stride), &ops));

@@ -351,16 +351,22 @@ int knn_batch(KnnJob &job, Ctx *ctx, cudaStream_t st, Small *dsmall, BaseOps *bo
   } else {
     // ---- THRESH: per-query thresholds from a strided sample of the base.
     // The c-th smallest of a 1/stride sample lies below ~c*stride base values;
-    // with stride = k/3 the chance that fewer than k fall below it is the
-    // chance that a Poisson(3) exceeds c-1 (c = 12: ~1.7e-4 per query; such a
-    // query fails its certificate and the band pass settles it).  The sample
-    // pass keeps 16 values per row; the c-th of them is the threshold.
+    // with stride = k/m the chance that fewer than k fall below it is the
+    // chance that a Poisson(m) reaches c: 1.6e-5 per query for m = 3, c = 13,
+    // 1.8e-5 for m = 6, c = 19.  (Such a query fails its certificate and a band
+    // pass with the sample's value of rank 2c settles it, ~0.3 ms a call; with
+    // c = 12, and the exhaustive pass behind it, most calls of 10k queries paid
+    // 6.9 ms.)  The larger sample costs the pass twice the sample and leaves
+    // 3.2k candidates instead of 4.3k: it pays where the sample is a small part
+    // of the base and its pass takes block minima (k = 100: 1/16 of the base).
+    // The sample pass keeps 16 values per row and chunk.
     sel.mode = SCAN_THRESH;
     sel.halves = 2;
     float *thr;
     YG_CHECK(ws_get(ws, WS_THR, nq, &thr));
-    const int c = 12;
-    int stride = k / 3;
+    const bool big = bf16 && k >= 96 && nb / (k / 6) >= kSampleMin;
+    const int c = big ? 19 : 13;
+    int stride = k / (big ? 6 : 3);
     if (stride < 1) stride = 1;
     const int ns = nb / stride;
     if (up) {
@@ -388,6 +394,9 @@ int knn_batch(KnnJob &job, Ctx *ctx, cudaStream_t st, Small *dsmall, BaseOps *bo
       sstride = (int)std::max<long>(1, (long)((double)stride * n0 / nb));
       sns = (int)(n0 / sstride);
     }
+    // a long sample is read in blocks (whole super tiles of it)
+    const bool blockmin = bf16 && sns >= kSampleMin;
+    if (blockmin) sns -= sns % kSampleSuper;
     if (band) {
       // thresholds from the k-th exact distance an earlier pass found
       const BandLayout L = band_layout(nq, nb, k, tile_m, tile_n, sel.halves, ctx->num_sms);
@@ -405,16 +414,19 @@ int knn_batch(KnnJob &job, Ctx *ctx, cudaStream_t st, Small *dsmall, BaseOps *bo
       fill_f32<<<(unsigned)ceil_div(nq, 256), 256, 0, st>>>(thr, nq, INFINITY);
       YG_LAUNCH_CHECK();
     } else {
-      ra.m_expect = c * stride;
-      const double er = (double)c * stride / nreg;  // expected hits per region
+      // base rows per sampled row (part 0 stands for the whole base)
+      const double per = (double)nb / sns;
+      ra.m_expect = (int)(c * per);
+      const double er = c * per / nreg;  // expected hits per region
       sel.cap = pow2_at_least((int)(2.0 * er + 6.0 * sqrt(er) + 16.0));
       ScanSel ss;
       ss.mode = SCAN_TOPV;  // only the c-th value is needed
       ss.C = 16;
       const int nts = (int)ceil_div(sns, tile_n);
-      const int nch = tune_chunks(TuneKey{2, job.prec, nqt, nts, ss.C},
+      int nch = tune_chunks(TuneKey{2, job.prec, nqt, nts, ss.C},
                                   choose_chunks(nqt, nts, ctx->num_sms, ctas_per_sm, 2), 64,
                                   ctx->num_sms * ctas_per_sm, &sample_ticket);
+      if (c > ss.C) nch = imax(nch, 2);  // the lists together hold the c-th value
       ss.tiles_per_chunk = (int)ceil_div(nts, nch);
       ss.nchunk = (int)ceil_div(nts, ss.tiles_per_chunk);
       YG_CHECK(ws_get(ws, WS_STOPV, (size_t)ss.nchunk * nq * ss.C, &ss.topv));
@@ -422,6 +434,7 @@ int knn_batch(KnnJob &job, Ctx *ctx, cudaStream_t st, Small *dsmall, BaseOps *bo
       tm_sample.reset(new PassTimer(timed || sample_ticket >= 0, st, &job.ms_sample));
       if (bf16) {
         TcOperands tcs = tcq;
+        ss.blockmin = blockmin ? 1 : 0;
         YG_CHECK(tc_base_view(tcq, sstride, sns, &tcs));
         YG_CHECK(tc_scan(tcs, nq, sns, ss, st));
       } else {
@@ -430,6 +443,11 @@ int knn_batch(KnnJob &job, Ctx *ctx, cudaStream_t st, Small *dsmall, BaseOps *bo
       }
       tm_sample->stop(st);
       YG_CHECK(thresh_from_sample(nq, ss.nchunk, ss.C, c, ss.topv, eps, thr, st));
+      ra.sample_topv = ss.topv;
+      ra.sample_nchunk = ss.nchunk;
+      ra.sample_C = ss.C;
+      ra.sample_c = c;
+      ra.sample_stride = nq;
     }
     sel.thr = thr;
     const int nr = sel.nregion();

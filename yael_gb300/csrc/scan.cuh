@@ -35,7 +35,7 @@ struct GroupUnit {
   int bend;            // end of the pair's valid columns in this view
   int pair;            // index into the pair table
   int chunk;           // chunk of the pair's base (THRESH region; 0 for lists)
-  int pad_;
+  int blockmin;        // TOPV: the unit reads the sample in blocks (ScanSel::blockmin)
 };
 
 // Per pair: where its candidates go (THRESH) and what the re-rank needs.
@@ -79,6 +79,9 @@ struct ScanSel {
   int nunits = 0;
   const GroupPair *gpairs = nullptr;
   int max_ctas = 0;         // persistent passes: grid limit (0 = one CTA per SM)
+  // TOPV (tc_scan): the list holds minima of 32-row blocks of the sample
+  // instead of single values; see kSampleSuper
+  int blockmin = 0;
   int f16 = 0;              // tensor-core passes: fp16 operands (else bf16)
   // tensor-core passes: bound of every wait (0: kWaitLimitNs), and a test
   // switch under which the producer issues no load, so that the consumers'
@@ -87,6 +90,17 @@ struct ScanSel {
   int withhold = 0;
   __host__ __device__ int nregion() const { return nchunk * halves; }
 };
+
+// Block minima of a threshold sample.  The c-th smallest of the minima of
+// disjoint blocks is an upper bound of the c-th smallest sampled value, and the
+// minimum of 32 columns comes with the tensor-core pass's accumulator load, so
+// the sample's lists take one insertion attempt per 32 values.  A block's rows
+// are kSampleD sample rows apart inside super tiles of kSampleSuper rows, so
+// that neighbours stored next to one another fall into different blocks; a
+// sample is cut to whole super tiles and used this way from kSampleMin rows on
+// (there the c <= 20 smallest values share a block rarely enough that the
+// threshold's rank grows by less than a tenth).
+constexpr int kSampleD = 32, kSampleSuper = 32 * kSampleD, kSampleMin = 4 * kSampleSuper;
 
 // FP32 CUDA-core producer.  q: nq rows (stride ldq floats); b: nb rows (stride
 // ldb floats); bn: ||b||^2 as float with stride bn_stride (L2 only).

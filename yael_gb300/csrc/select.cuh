@@ -43,6 +43,11 @@ struct RerankArgs {
   // sized for a few times this rather than for every region's capacity, and a
   // query with more candidates fails its certificate (the band pass follows)
   int m_expect = 0;
+  // THRESH with thresholds from a sample: its lists and rank, from which a
+  // query with fewer than k candidates gets the bound its band pass starts from
+  const float *sample_topv = nullptr;
+  int sample_nchunk = 0, sample_C = 0, sample_c = 0;
+  int sample_stride = 0;         // queries per list chunk
   // grouped re-rank (many pairs, THRESH): row q belongs to pair qpair[q], whose
   // table entry gives its candidate regions, base rows, statistics and outputs
   // (q, qn64, eps, qexact, thr, fail_list and kth_out stay indexed by q)

@@ -144,7 +144,9 @@ __global__ void __launch_bounds__(NT_TC, 1)
     tc_scan_kernel(const __grid_constant__ CUtensorMap mapQ,
                    const __grid_constant__ CUtensorMap mapQn,
                    const __grid_constant__ CUtensorMap mapB,
-                   const __grid_constant__ CUtensorMap mapBn, int nq, int nb, int nkb,
+                   const __grid_constant__ CUtensorMap mapBn,
+                   const __grid_constant__ CUtensorMap mapB3,
+                   const __grid_constant__ CUtensorMap mapBn3, int nq, int nb, int nkb,
                    int S, ScanSel sel, int *err) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   // aligned by pointer arithmetic on smem_raw (not through an integer), so
@@ -186,14 +188,14 @@ __global__ void __launch_bounds__(NT_TC, 1)
   const int w0 = PERSIST ? (int)blockIdx.x : 0, wstep = PERSIST ? (int)gridDim.x : 1;
   struct UnitInfo {
     long q0, qend;
-    int t_begin, t_end, bend, chunk, pair;
+    int t_begin, t_end, bend, chunk, pair, blockmin;
   };
   auto unit_info = [&](int w) -> UnitInfo {
     UnitInfo u;
     if (grouped) {
       const GroupUnit g = sel.units[w];
       u.q0 = g.q0; u.qend = g.qend; u.t_begin = g.t_begin; u.t_end = g.t_end;
-      u.bend = g.bend; u.chunk = g.chunk; u.pair = g.pair;
+      u.bend = g.bend; u.chunk = g.chunk; u.pair = g.pair; u.blockmin = g.blockmin;
       return u;
     }
     u.q0 = PERSIST ? (long)(w % nqt) * TC_TILE_M : (long)blockIdx.x * TC_TILE_M;
@@ -203,6 +205,7 @@ __global__ void __launch_bounds__(NT_TC, 1)
     u.t_end = imin(ntb, u.t_begin + sel.tiles_per_chunk);
     u.bend = nb;
     u.pair = -1;
+    u.blockmin = sel.blockmin;
     return u;
   };
   const uint32_t crank = PAIR ? cluster_ctarank() : 0;
@@ -279,6 +282,11 @@ __global__ void __launch_bounds__(NT_TC, 1)
       }
       for (int t = un.t_begin; t < un.t_end && ok; t++) {
         const int brow = t * TC_TILE_N + (int)crank * (TC_TILE_N / 2) * (PAIR ? 1 : 0);
+        // sample blocks: 8 consecutive rows of each of a super tile's 32 row groups
+        const bool b3 = MODE == SCAN_TOPV && !PAIR && un.blockmin;
+        const int lt = grouped ? t - un.t_begin : t;
+        const int brow3 = (grouped ? un.t_begin * TC_TILE_N : 0) + (lt >> 2) * kSampleSuper +
+                          (lt & 3) * (TC_TILE_N / 32);
         for (int ks = 0; ks < nks; ks++) {
           const int s = sn;
           const uint32_t ph = phn;
@@ -302,10 +310,12 @@ __global__ void __launch_bounds__(NT_TC, 1)
             }
           } else {
             mbar_arrive_expect_tx(&full[s], tx);
-            tma_load_2d(&mapB, &full[s], sp, ks * 64, brow);
+            if (b3) tma_load_3d(&mapB3, &full[s], sp, ks * 64, 0, brow3);
+            else tma_load_2d(&mapB, &full[s], sp, ks * 64, brow);
             if (QS) tma_load_2d(&mapQ, &full[s], sp + BHALF, ks * 64, (int)q0);
             if (lastk) {
-              tma_load_2d(&mapBn, &full[s], np_, 0, brow);
+              if (b3) tma_load_3d(&mapBn3, &full[s], np_, 0, 0, brow3);
+              else tma_load_2d(&mapBn, &full[s], np_, 0, brow);
               if (QS) tma_load_2d(&mapQn, &full[s], np_ + BN_BYTES, 0, (int)q0);
             }
             issued |= 1u << s;
@@ -640,7 +650,8 @@ __global__ void __launch_bounds__(NT_TC, 1)
       // hit; a bound of this half tile's C-th smallest filters them instead
       if (MODE != SCAN_THRESH && C <= 16) {
         tb = INFINITY;
-        if (t == t_begin && j0 + 128 <= nbv) tb = cth_bound<C>(r0, r1, r2, r3);
+        if (t == t_begin && j0 + 128 <= nbv && !(MODE == SCAN_TOPV && un.blockmin))
+          tb = cth_bound<C>(r0, r1, r2, r3);
       }
       if (MODE == SCAN_THRESH) {
         // (thr is NaN in lanes without a query; an all-NaN chunk has no hit)
@@ -660,6 +671,15 @@ __global__ void __launch_bounds__(NT_TC, 1)
           const int it1 = it + 1;
           const bool ready = mbar_test_wait(&tfull[it1 & 1], (uint32_t)((it1 >> 1) & 1));
           if (!__any_sync(0xffffffffu, ready)) drain();
+        }
+      } else if (MODE == SCAN_TOPV && un.blockmin) {
+        // the four chunk minima are the values (no partial tile here)
+        float mv[4] = {__uint_as_float(m0), __uint_as_float(m1), __uint_as_float(m2),
+                       __uint_as_float(m3)};
+#pragma unroll 1
+        for (int c = 0; c < 4; c++) {
+          const float x = c & 2 ? (c & 1 ? mv[3] : mv[2]) : (c & 1 ? mv[1] : mv[0]);
+          if (__any_sync(0xffffffffu, x < lmax)) update(x, 0);
         }
       } else {
         process(r0, __uint_as_float(m0), j0);
@@ -772,6 +792,33 @@ static int make_map(CUtensorMap *m, const void *ptr, uint64_t cols, uint64_t row
   return OK;
 }
 
+// The block view of a sample (kSampleSuper): rows kSampleD apart in the middle
+// dimension, consecutive rows in the last; one box is 32 x 8 rows, the 32 of a
+// block first.
+static int make_map3(CUtensorMap *m, const void *ptr, uint64_t cols, uint64_t rows,
+                     uint64_t row_bytes, uint32_t box_cols, CUtensorMapSwizzle sw) {
+  YG_CHECK(get_encode());
+  if (!ptr || (reinterpret_cast<uintptr_t>(ptr) & 15) || (row_bytes & 15) ||
+      rows < kSampleSuper) {
+    set_error(E_ARG, "tensor map: null / misaligned / short sample operand");
+    return E_ARG;
+  }
+  // the last start row keeps all 32 groups inside the operand
+  cuuint64_t dims[3] = {cols, 32, rows - 31 * kSampleD};
+  cuuint64_t strides[2] = {row_bytes * kSampleD, row_bytes};
+  cuuint32_t box[3] = {box_cols, 32, TC_TILE_N / 32};
+  cuuint32_t es[3] = {1, 1, 1};
+  CUresult r = g_encode(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void *>(ptr), dims,
+                        strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, sw,
+                        CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) {
+    set_error(E_CUDA, "cuTensorMapEncodeTiled failed (%d): sample blocks, rows=%llu pitch=%llu",
+              (int)r, (unsigned long long)rows, (unsigned long long)row_bytes);
+    return E_CUDA;
+  }
+  return OK;
+}
+
 template <int MODE, int C, bool L2, bool QS, bool PAIR>
 int launch(const TcOperands &op, int nq, int nb, const ScanSel &sel, cudaStream_t st) {
   const int nkb = op.Kp / 64;
@@ -788,7 +835,7 @@ int launch(const TcOperands &op, int nq, int nb, const ScanSel &sel, cudaStream_
     return E_UNSUPPORTED;
   }
   YG_CHECK(ensure_smem((const void *)tc_scan_kernel<MODE, C, L2, QS, PAIR>, lay.total));
-  CUtensorMap mq, mqn, mb, mbn;
+  CUtensorMap mq, mqn, mb, mbn, mb3, mbn3;
   YG_CHECK(make_map(&mq, op.q, op.Kp, nq, (uint64_t)op.Kp * 2, 64, 128,
                     CU_TENSOR_MAP_SWIZZLE_128B));
   // a pair CTA loads 128 of the 256 rows of each base block
@@ -803,6 +850,15 @@ int launch(const TcOperands &op, int nq, int nb, const ScanSel &sel, cudaStream_
     mqn = mq;
     mbn = mb;
   }
+  mb3 = mb;
+  mbn3 = mbn;
+  if (MODE == SCAN_TOPV && sel.blockmin) {
+    YG_CHECK(make_map3(&mb3, op.b, op.Kp, nb, (uint64_t)op.Kp * 2 * op.b_step, 64,
+                       CU_TENSOR_MAP_SWIZZLE_128B));
+    if (L2)
+      YG_CHECK(make_map3(&mbn3, op.bn, 16, nb, (uint64_t)32 * op.b_step, 16,
+                         CU_TENSOR_MAP_SWIZZLE_32B));
+  }
   if (!PAIR && (QS || sel.units)) {
     // persistent: one CTA per SM (the ring fills shared memory), units strided
     int dev = 0, nsm = 0;
@@ -815,12 +871,12 @@ int launch(const TcOperands &op, int nq, int nb, const ScanSel &sel, cudaStream_
     }
     if (sel.max_ctas > 0 && sel.max_ctas < nsm) nsm = sel.max_ctas;
     const unsigned g = (unsigned)(nunits < nsm ? nunits : nsm);
-    tc_scan_kernel<MODE, C, L2, QS, PAIR><<<g, NT_TC, lay.total, st>>>(mq, mqn, mb, mbn, nq, nb,
-                                                                        nkb, S, sel, op.err);
+    tc_scan_kernel<MODE, C, L2, QS, PAIR><<<g, NT_TC, lay.total, st>>>(
+        mq, mqn, mb, mbn, mb3, mbn3, nq, nb, nkb, S, sel, op.err);
   } else if (!PAIR) {
     dim3 grid((unsigned)ceil_div(nq, TC_TILE_M), (unsigned)sel.nchunk);
     tc_scan_kernel<MODE, C, L2, QS, PAIR><<<grid, NT_TC, lay.total, st>>>(
-        mq, mqn, mb, mbn, nq, nb, nkb, S, sel, op.err);
+        mq, mqn, mb, mbn, mb3, mbn3, nq, nb, nkb, S, sel, op.err);
   } else {
     // query tiles padded to whole pairs (a padding CTA has no valid rows)
     cudaLaunchConfig_t cfg = {};
@@ -835,8 +891,8 @@ int launch(const TcOperands &op, int nq, int nb, const ScanSel &sel, cudaStream_
     at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    YG_CUDA(cudaLaunchKernelEx(&cfg, tc_scan_kernel<MODE, C, L2, QS, PAIR>, mq, mqn, mb, mbn, nq,
-                               nb, nkb, S, sel, op.err));
+    YG_CUDA(cudaLaunchKernelEx(&cfg, tc_scan_kernel<MODE, C, L2, QS, PAIR>, mq, mqn, mb, mbn,
+                               mb3, mbn3, nq, nb, nkb, S, sel, op.err));
   }
   YG_LAUNCH_CHECK();
   return OK;

@@ -148,7 +148,7 @@ int tc_scan(const TcOperands &op, int nq, int nb, const ScanSel &sel_in, cudaStr
     const char *e = getenv("YAEL_GPU_TC_PAIR");
     return e && e[0] == '1';
   }();
-  const bool pair = pair_env && nq > TC_TILE_M;
+  const bool pair = pair_env && nq > TC_TILE_M && !sel.blockmin;
   // the query tile stays resident in shared memory when a ring of at least
   // three stages still fits beside it (always for K <= 256; for the 3xBF16
   // split of d <= 128, K = 384, with short lists); else it is streamed with

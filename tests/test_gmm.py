@@ -329,3 +329,48 @@ def test_port_restatement_bit_identical_to_reference(nt):
                                ctypes.byref(it)) == 0
         for a, b in zip((gw, gm, gs), exp):
             np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,d,k", [(1, 1, 1), (31, 3, 5), (65, 64, 64), (2433, 65, 33),
+                                   (5003, 100, 17), (4900, 130, 65), (10001, 32, 129),
+                                   (40, 9, 2500)])
+def test_gpu_mixture_tile_edges(n, d, k):
+    """Vectors, dimensions and components at the edges of the posterior and
+    moment tiles (k = 2500: rows too long for shared memory)."""
+    L_ = bind(yg.lib())
+    v, w, mu, sigma = mixture(n + d, n, d, k)
+    g, keep = make_gmm(w, mu, sigma)
+    np.testing.assert_allclose(run_p(L_, v, g, go.FLAGS_W),
+                               go.compute_p(v, w, mu, sigma, go.FLAGS_W), rtol=0, atol=P_ATOL)
+    # posteriors with many exact zeros, whole rows of them included
+    rng = np.random.default_rng(n)
+    p = rng.random((n, k), dtype=np.float32)
+    p[rng.random((n, k)) < 0.9] = 0
+    p[rng.random(n) < 0.3] = 0
+    flags = go.FLAGS_W * (k > 1) | go.FLAGS_MU | go.FLAGS_SIGMA
+    close(run_fisher(L_, v, g, flags, p),
+          go.fisher_from_posteriors(v, w, mu, sigma, p.astype(np.float64), flags),
+          FV_RTOL, FV_ATOL)
+
+
+@pytest.mark.gpu
+def test_gpu_moments_non_finite():
+    """A zero posterior does not hide an infinity or a NaN of its vector: the
+    entries that FP64 moments make non-finite are non-finite."""
+    L_ = bind(yg.lib())
+    v, w, mu, sigma = mixture(5, 700, 70, 40)
+    g, keep = make_gmm(w, mu, sigma)
+    p = np.zeros((700, 40), np.float32)
+    p[np.arange(700), np.arange(700) % 40] = 1
+    v[123, 7], v[400, 66], v[500, 11], p[650, 3] = np.inf, np.nan, -np.inf, np.inf
+    got = run_fisher(L_, v, g, go.FLAGS_MU, p)
+    with np.errstate(invalid="ignore"):
+        p64, v64, s64 = p.astype(np.float64), v.astype(np.float64), sigma.astype(np.float64)
+        s0, s1 = p64.sum(0)[:, None], np.einsum("ij,il->jl", p64, v64)
+        exp = (s1 - mu.astype(np.float64) * s0) / s64 / np.sqrt(700 * w[:, None] / s64)
+        exp = exp.reshape(-1)
+    np.testing.assert_array_equal(np.isnan(got), np.isnan(exp))
+    np.testing.assert_array_equal(np.isinf(got), np.isinf(exp))
+    fin = np.isfinite(exp)
+    close(got[fin], exp[fin].astype(np.float64), FV_RTOL, FV_ATOL)

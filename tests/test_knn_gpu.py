@@ -13,7 +13,8 @@ import numpy as np
 import pytest
 
 import yael_gb300 as yg
-from _util import GOLDEN, check_knn_ties, exact_dist64, knn_exact, knn_port, ptr
+from _util import (GOLDEN, assign_mismatches, check_knn_ties, exact_dist64, knn_exact, knn_port,
+                   ptr)
 from yael_gb300 import synth
 
 pytestmark = pytest.mark.gpu
@@ -321,3 +322,40 @@ def test_host_upload_in_parts(k):
     if len(mism):
         assert check_knn_ties(idx, exact_dist64(b, q, idx), ridx, r64) == 0
     np.testing.assert_allclose(dis, rdis, rtol=2e-6, atol=1e-5)
+
+
+@pytest.mark.parametrize("prec", ["bf16", "fp16", "bf16x3"])
+@pytest.mark.parametrize("nq,nb", [(19_500, 200), (20_001, 287), (40_000, 1031), (77_900, 2049),
+                                   (20_000, 4099), (80_000, 3900)])
+def test_nearest_running_thresholds(nq, nb, prec):
+    """k = 1 over enough queries for the running thresholds, at the edges of
+    tiles, chunks and regions: rows in ascending and in descending distance, many
+    equal rows (more than a region holds), NaN and infinite queries."""
+    d = 20
+    rng = np.random.default_rng(nb)
+    b = rng.standard_normal((nb, d)).astype(np.float32)
+    q = (b[rng.integers(0, nb, nq)] + 0.3 * rng.standard_normal((nq, d))).astype(np.float32)
+    m = nq // 8
+    b[nb // 2:nb // 2 + 40] = b[nb // 2]              # equal rows, near all of these queries
+    q[:m] = b[nb // 2] + 0.01 * q[:m]
+    b[40:120] = np.linspace(4, 0.1, 80, dtype=np.float32)[:, None]   # ever nearer, then farther
+    b[120:200] = np.linspace(0.1, 4, 80, dtype=np.float32)[:, None]
+    q[m:2 * m] = 1e-3 * q[m:2 * m]
+    idx, dis, _ = gpu_knn(b, q, 1, prec)
+    assert assign_mismatches(q, b, idx[:, 0].copy(), NT)[0] == 0
+    np.testing.assert_allclose(dis[:, 0], ((q - b[idx[:, 0]]) ** 2).sum(1), rtol=2e-5, atol=1e-6)
+    # integers: exact values, the lowest id of each group of equal rows
+    bi = rng.integers(0, 3, (nb, d)).astype(np.float32)
+    bi[nb - 60:] = bi[:60]
+    qi = rng.integers(0, 3, (nq, d)).astype(np.float32)
+    qi[:m] = bi[nb - 1]
+    idx, _, st = gpu_knn(bi, qi, 1, prec)
+    assert st["exact_class"] == 1
+    assert assign_mismatches(qi, bi, idx[:, 0].copy(), NT)[0] == 0
+    # queries without a nearest row
+    q[5], q[nq - 1, 3] = np.nan, np.inf
+    idx2, dis2, _ = gpu_knn(b, q, 1, prec)
+    sel = np.setdiff1d(np.arange(nq), [5, nq - 1])
+    ref1, _, _ = gpu_knn(b, q[[5, nq - 1]], 1, prec)
+    np.testing.assert_array_equal(idx2[[5, nq - 1]], ref1)
+    assert assign_mismatches(q[sel], b, idx2[sel, 0].copy(), NT)[0] == 0

@@ -14,7 +14,8 @@
 namespace yg {
 
 struct TuneKey {
-  int kind;   // pass: 0 TOPC main, 1 THRESH main, 2 threshold sample, 3 grouped assignment
+  int kind;   // pass: 0 TOPC main, 1 THRESH main, 2 threshold sample, 3 grouped assignment,
+              // 4 running thresholds
   int prec;   // distance precision
   int nqt;    // query tiles
   int ntb;    // base tiles

@@ -107,6 +107,20 @@ __global__ void gather_kth_kernel(const float *in_kth, const float *out_kth, con
 // as many as the short re-rank's 32 slots hold (two regions per chunk)
 int prior_cap(int nchunk) { return imax(8, 32 / (2 * nchunk)); }
 
+// Nearest neighbours (k = 1) by running thresholds: chunks of the base, 0 where
+// lists do better.  A region keeps the few rows within the error band of
+// the smallest value it has seen (ScanSel::run_eps), so the pass takes one
+// comparison per 32 values where a list of eight takes an insertion for
+// every value among its best eight so far: 200k x 10k, d = 128: 1.11 ms -> 0.49.
+// All regions of a query fit the short re-rank's 32 slots, so at most four
+// chunks: with fewer query tiles than that fills, more chunks (and lists) do
+// better.
+int running_chunks(int nqt, int ntb, int num_sms) {
+  const int c = choose_chunks(nqt, ntb, num_sms, 1, 4);
+  return c <= 4 ? c : 0;
+}
+int running_cap(int nchunk) { return imin(8, 32 / (2 * nchunk)); }
+
 int list_length(int k, int exact, int nb) {
   (void)nb;
   if (k == 1) return 8;
@@ -332,6 +346,26 @@ int knn_batch(KnnJob &job, Ctx *ctx, cudaStream_t st, Small *dsmall, BaseOps *bo
     YG_CHECK(scan_parts(job, *up, *bops, dsmall, tcq, nq, sel, pnch, ptpc, pfirst, ptm, st));
     tm_scan->stop(st);
     job.scan_launches += up->nparts;
+  } else if (const int rc = !band && !prior && bf16 && k == 1
+                                ? running_chunks(nqt, ntb, ctx->num_sms) : 0) {
+    // ---- the nearest row, thresholds running with the smallest value seen
+    sel.mode = SCAN_THRESH;
+    sel.halves = 2;
+    sel.run_eps = eps;
+    const int nchunk = tune_chunks(TuneKey{4, job.prec, nqt, ntb, 0}, rc,
+                                   imax(1, imin(4, ntb / 4)), ctx->num_sms * ctas_per_sm,
+                                   &scan_ticket);
+    sel.tiles_per_chunk = (int)ceil_div(ntb, nchunk);
+    sel.nchunk = (int)ceil_div(ntb, sel.tiles_per_chunk);
+    sel.cap = running_cap(sel.nchunk);
+    const long nr = sel.nregion();
+    YG_CHECK(ws_get(ws, WS_CNT, (size_t)nr * nq, &sel.cnt));
+    YG_CHECK(ws_get(ws, WS_TOPV, (size_t)nr * nq * sel.cap, &sel.candv));
+    YG_CHECK(ws_get(ws, WS_TOPI, (size_t)nr * nq * sel.cap, &sel.candi));
+    tm_scan.reset(new PassTimer(timed || scan_ticket >= 0, st, &job.ms_scan));
+    YG_CHECK(scan(job, job.q, nq, job.b, job.ldb, nb, bn32, 1, &tcq, sel, st));
+    tm_scan->stop(st);
+    job.scan_launches++;
   } else if (!band && !prior && c_needed <= 16) {
     // ---- TOPC over the full base (register lists)
     sel.mode = SCAN_TOPC;
@@ -407,16 +441,20 @@ int knn_batch(KnnJob &job, Ctx *ctx, cudaStream_t st, Small *dsmall, BaseOps *bo
     } else if (prior) {
       // every row whose exact distance can be <= the known bound
       sel.cap = prior_cap(sel.nchunk);
+      sel.queue = nb >= 8192;  // a few rows in the band of the bound
       YG_CHECK(band_thresholds(nq, job.metric, job.prior_kth, qn64, eps, thr, st));
     } else if (nb <= kMaxCandidates || sns < 4 * c) {
       // every base row is a candidate; a region holds at most its share of the chunk
       sel.cap = pow2_at_least(imax(1, sel.tiles_per_chunk * tile_n / sel.halves));
+      sel.queue = 1;
       fill_f32<<<(unsigned)ceil_div(nq, 256), 256, 0, st>>>(thr, nq, INFINITY);
       YG_LAUNCH_CHECK();
     } else {
       // base rows per sampled row (part 0 stands for the whole base)
       const double per = (double)nb / sns;
       ra.m_expect = (int)(c * per);
+      // (under half a hit expected in 32 rows x 32 columns)
+      sel.queue = 1024.0 * c * per < 0.5 * nb;
       const double er = c * per / nreg;  // expected hits per region
       sel.cap = pow2_at_least((int)(2.0 * er + 6.0 * sqrt(er) + 16.0));
       ScanSel ss;
@@ -518,7 +556,8 @@ int knn_batch(KnnJob &job, Ctx *ctx, cudaStream_t st, Small *dsmall, BaseOps *bo
             "[yael_gpu] knn level=%d prec=%d pass=%s nq=%d nb=%d d=%d k=%d chunks=%d "
             "scan=%.3fms sample=%.3fms rerank=%.3fms rejected=%d\n",
             job.level, job.prec,
-            band ? "band" : prior ? "prior" : (sel.mode == SCAN_TOPC ? "topc" : "thresh"), nq,
+            band ? "band" : prior ? "prior" : sel.run_eps ? "running"
+                 : (sel.mode == SCAN_TOPC ? "topc" : "thresh"), nq,
             nb, d, k, sel.nchunk, job.ms_scan, job.ms_sample, job.ms_rerank, nf);
   if (nf == 0) return OK;
   // A regular pass's rejections go to a band pass at the same precision: its

@@ -16,6 +16,11 @@
 //             candv/candi[(r * nq + q) * cap + s], count cnt[r * nq + q] (all
 //             hits, including those that did not fit in cap).  No atomics:
 //             each (region, query) has exactly one writer.
+//             With run_eps (tc_scan, k = 1) the threshold is not given but runs:
+//             the smallest v the region has seen plus run_slack(eps).  A
+//             region starts over when its threshold falls below all its
+//             candidates, so it ends with the few rows that can still be the
+//             nearest; every row it left out is above its last threshold.
 #pragma once
 #include "common.cuh"
 
@@ -67,6 +72,7 @@ struct ScanSel {
   float *topv = nullptr;
   int *topi = nullptr;
   const float *thr = nullptr;
+  const float *run_eps = nullptr;  // THRESH: eps per query, thresholds run (thr unused)
   int *cnt = nullptr;
   float *candv = nullptr;
   int *candi = nullptr;
@@ -82,6 +88,9 @@ struct ScanSel {
   // TOPV (tc_scan): the list holds minima of 32-row blocks of the sample
   // instead of single values; see kSampleSuper
   int blockmin = 0;
+  // THRESH (tc_scan): well under one hit in 32 rows x 32 columns expected, or
+  // nearly all of them hits: both are best drained a row of 32 at a time
+  int queue = 0;
   int f16 = 0;              // tensor-core passes: fp16 operands (else bf16)
   // tensor-core passes: bound of every wait (0: kWaitLimitNs), and a test
   // switch under which the producer issues no load, so that the consumers'
@@ -90,6 +99,14 @@ struct ScanSel {
   int withhold = 0;
   __host__ __device__ int nregion() const { return nchunk * halves; }
 };
+
+// What a running threshold leaves above the smallest value: two error bounds
+// (the row of the smallest exact distance is within them) and a little for the
+// certificate's roundings.  Where no bound holds the rows nearest by value are
+// kept all the same: they give the later passes a distance to start from.
+__host__ __device__ inline float run_slack(float eps) {
+  return eps < INFINITY ? 2.0005f * eps : 0.f;
+}
 
 // Block minima of a threshold sample.  The c-th smallest of the minima of
 // disjoint blocks is an upper bound of the c-th smallest sampled value, and the

@@ -701,16 +701,19 @@ __device__ __forceinline__ unsigned rerank_small_k1(const RerankArgs &a, int q) 
   unsigned key = 0xffffffffu;  // f2ord of the approximate value
   int id = 0x7fffffff;         // 0x7fffffff: no candidate in this lane
   unsigned long long tkey = ~0ull;
+  float vraw = INFINITY;       // THRESH: the value of the distance pass
   bool overflow = false;
   if (thresh) {
     if (gl < s.nregion() * s.cap) {
       const int r = gl / s.cap, sl = gl - r * s.cap;
       const int cnt = s.cnt[(long)r * a.nq + q];
-      overflow = cnt > s.cap;
+      // (running thresholds: exact values past the region's end tie its
+      // least, with larger ids)
+      overflow = cnt > s.cap && !(s.run_eps && ex);
       if (sl < cnt && sl < s.cap) {
         const long o = ((long)r * a.nq + q) * s.cap + sl;
-        const float v = s.candv[o];
-        key = f2ord(L2 ? (float)((double)v + qn) : v);
+        vraw = s.candv[o];
+        key = f2ord(L2 ? (float)((double)vraw + qn) : vraw);
         id = s.candi[o];
       }
     }
@@ -858,7 +861,10 @@ __device__ __forceinline__ unsigned rerank_small_k1(const RerankArgs &a, int q) 
       // settled; the few it may reject at the edge go to the band pass.
       if (thresh) {
         // every non-candidate has approx > thr, so exact > thr + ||q||^2 - eps
-        const float t = s.thr[q];
+        // (a running threshold ends at or above the least value plus its slack)
+        const float t = s.run_eps ? __fadd_rd(ord2f(__reduce_min_sync(gm, f2ord(vraw))),
+                                              run_slack(eps))
+                                  : s.thr[q];
         float blo = t, babs = fabsf(t);
         if (L2) {
           const double bd = (double)t + qn;
@@ -1211,6 +1217,10 @@ __global__ void __launch_bounds__(RT) fb_select_kernel(const int *qlist, int q0,
 
 int rerank(const RerankArgs &a, cudaStream_t st) {
   if (a.nq <= 0) return OK;
+  if (a.sel.run_eps && (a.k != 1 || a.gpairs || a.sel.nregion() * a.sel.cap > 32)) {
+    set_error(E_UNSUPPORTED, "rerank: running thresholds are for k = 1 and short regions");
+    return E_UNSUPPORTED;
+  }
   // short candidate sets: a group of 8 to 32 lanes per query
   const bool small_topc = a.sel.mode == SCAN_TOPC && a.sel.nchunk * a.sel.C <= 32;
   const bool small_thresh = a.sel.mode == SCAN_THRESH && !a.gpairs && a.sel.cap > 0 &&

@@ -49,6 +49,20 @@ constexpr int QBLK_BYTES = 128 * 128;    // 128 rows x 64 bf16
 constexpr int QN_BYTES = 4096;           // 128 rows x 16 bf16 (padded to 4 KB)
 constexpr int BN_BYTES = 256 * 32;       // 256 rows x 16 bf16
 constexpr int TMEM_COLS = 512;
+// Template mode of a THRESH pass with running thresholds (ScanSel::run_eps): a
+// kernel of its own, so that the fixed-threshold pass keeps its code.
+constexpr int SCAN_RUN = 3;
+// And of a THRESH pass with ScanSel::queue: the hit queue alone, without the
+// code that walks a chunk's hits lane by lane (which the loop's instruction
+// cache does not hold for nothing: 1M x 10k, k = 100: 1.51 ms without, 1.60 with).
+constexpr int SCAN_QUEUE = 4;
+constexpr int kWalkLanes = 2;  // more hit lanes than this walk their own hits
+// A running unit goes through its first kRunLead tiles twice: the first time
+// only for their least values.  Rows whose threshold has nothing to stand on
+// yet would queue a chunk per tile (1 + 1/2 + 1/3 + ... of them); a tile
+// scanned again costs about what 0.27 queued chunks a row cost, so the sum
+// kRunLead + 3.7 ln(tiles / kRunLead) is least at four tiles.
+constexpr int kRunLead = 4, kRunLeadMin = 12;
 constexpr int HQ_LD = 36;  // floats per row of a hit queue: 32 values, threshold, lane, column
 // rows of a selection warp's hit queue (THRESH); fewer where the resident
 // query tile of a split pass leaves no room beside three stages
@@ -75,10 +89,13 @@ __host__ __device__ inline Layout make_layout(int nkb, int S, int mode, int C, b
                   (qs ? QBLK_BYTES + QN_BYTES : 0);
   L.stg_off = off; off += (size_t)S * L.stage_bytes;
   L.list_off = off;
-  if (mode != SCAN_THRESH) off += (size_t)(C > 16 ? N_EPI : 128) * C * 8;
+  if (mode == SCAN_RUN) off += N_EPI * 4;  // the least value of each row and column half
+  else if (mode != SCAN_THRESH && mode != SCAN_QUEUE)
+    off += (size_t)(C > 16 ? N_EPI : 128) * C * 8;
   off = (off + 15) & ~(size_t)15;
   L.hq_off = off;
-  if (mode == SCAN_THRESH) off += (size_t)(N_EPI / 32) * hq_rows(nkb) * HQ_LD * 4;
+  if (mode == SCAN_THRESH || mode == SCAN_RUN || mode == SCAN_QUEUE)
+    off += (size_t)(N_EPI / 32) * hq_rows(nkb) * HQ_LD * 4;
   L.bar_off = off; off += (size_t)(2 * S + 8) * 8 + 16;
   L.total = off + 1024;  // alignment slack for the 1024-byte aligned base
   return L;
@@ -139,7 +156,7 @@ __device__ __forceinline__ void reg_insert(float (&L)[C], int (&I)[C], float x, 
   }
 }
 
-template <int MODE, int C, bool L2, bool QS, bool PAIR>
+template <int KMODE, int C, bool L2, bool QS, bool PAIR>
 __global__ void __launch_bounds__(NT_TC, 1)
     tc_scan_kernel(const __grid_constant__ CUtensorMap mapQ,
                    const __grid_constant__ CUtensorMap mapQn,
@@ -152,7 +169,10 @@ __global__ void __launch_bounds__(NT_TC, 1)
   // aligned by pointer arithmetic on smem_raw (not through an integer), so
   // that the compiler keeps these pointers in the shared address space
   uint8_t *base = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-  const Layout lay = make_layout(nkb, S, MODE, C, QS, PAIR);
+  constexpr bool RUN = KMODE == SCAN_RUN;
+  constexpr int MODE = RUN || KMODE == SCAN_QUEUE ? (int)SCAN_THRESH : KMODE;
+  constexpr bool WALK = KMODE == SCAN_THRESH;
+  const Layout lay = make_layout(nkb, S, KMODE, C, QS, PAIR);
   const size_t SB = lay.stage_bytes;
   constexpr int BHALF = PAIR ? STAGE_BYTES / 2 : STAGE_BYTES;  // base bytes per stage, this CTA
   constexpr int BNHALF = PAIR ? BN_BYTES / 2 : BN_BYTES;
@@ -208,6 +228,8 @@ __global__ void __launch_bounds__(NT_TC, 1)
     u.blockmin = sel.blockmin;
     return u;
   };
+  // tiles of a unit of n that are scanned twice
+  auto lead_tiles = [](int n) { return RUN && n >= kRunLeadMin ? kRunLead : 0; };
   const uint32_t crank = PAIR ? cluster_ctarank() : 0;
   const bool leader = crank == 0;
 
@@ -227,6 +249,7 @@ __global__ void __launch_bounds__(NT_TC, 1)
     *abort_flag = 0;
     fence_mbar_init();
   }
+  if (RUN && warp >= 2) Lv[(warp - 2) * 32 + lane] = INFINITY;
   if (warp == 1) {
     if (PAIR) {
       tmem_alloc_pair(tmem_holder, TMEM_COLS);
@@ -280,7 +303,9 @@ __global__ void __launch_bounds__(NT_TC, 1)
         }
         qloads++;
       }
-      for (int t = un.t_begin; t < un.t_end && ok; t++) {
+      const int lead = lead_tiles(un.t_end - un.t_begin);
+      for (int tt = un.t_begin - lead; tt < un.t_end && ok; tt++) {
+        const int t = RUN && tt < un.t_begin ? tt + lead : tt;
         const int brow = t * TC_TILE_N + (int)crank * (TC_TILE_N / 2) * (PAIR ? 1 : 0);
         // sample blocks: 8 consecutive rows of each of a super tile's 32 row groups
         const bool b3 = MODE == SCAN_TOPV && !PAIR && un.blockmin;
@@ -359,7 +384,7 @@ __global__ void __launch_bounds__(NT_TC, 1)
       for (int w = w0; w < nunits && ok; w += wstep, ui++) {
       const UnitInfo un = unit_info(w);
       const int t_begin = __shfl_sync(0xffffffffu, un.t_begin, 0);
-      const int t_end = __shfl_sync(0xffffffffu, un.t_end, 0);
+      const int t_end = __shfl_sync(0xffffffffu, un.t_end + lead_tiles(un.t_end - un.t_begin), 0);
       if (!QS) {
         if (!mbar_wait_warp(qfull, (uint32_t)(ui & 1), abort_flag, wl)) { ok = false; break; }
         tc_fence_after();
@@ -466,7 +491,17 @@ __global__ void __launch_bounds__(NT_TC, 1)
     if (MODE != SCAN_THRESH && C > 16) {
       for (int s = 0; s < C; s++) { Lv[s * N_EPI + tslot] = INFINITY; Li[s * N_EPI + tslot] = 0x7fffffff; }
     }
-    if (MODE == SCAN_THRESH && rvalid) thr = sel.thr[qrow];
+    // running threshold: the least value seen plus the query's slack
+    float rmin = -INFINITY, slack = 0.f;
+    volatile float *lv_own = Lv + half * 128 + row, *lv_other = Lv + (half ^ 1) * 128 + row;
+    if (RUN) {
+      if (rvalid) {
+        thr = rmin = INFINITY;
+        slack = run_slack(sel.run_eps[qrow]);
+      }
+    } else if (MODE == SCAN_THRESH && rvalid) {
+      thr = sel.thr[qrow];
+    }
     int rcount = 0;  // THRESH: hits of this thread's region (chunk, half, query)
     float tb = INFINITY;  // lists: bound of the current half tile's C-th smallest
     // THRESH region of this thread: counter index and first slot
@@ -536,7 +571,8 @@ __global__ void __launch_bounds__(NT_TC, 1)
         const float4 meta = *reinterpret_cast<const float4 *>(xr + 32);
         const int src = __float_as_int(meta.y), j = __float_as_int(meta.z) + lane;
         const float x = xr[lane];
-        const bool hit = x <= meta.x && j < nbv;
+        // (a running threshold may have come down since the row was queued)
+        const bool hit = x <= (RUN ? __shfl_sync(0xffffffffu, thr, src) : meta.x) && j < nbv;
         const uint32_t m = __ballot_sync(0xffffffffu, hit);
         const int pos = __shfl_sync(0xffffffffu, rcount, src) + __popc(m & ((1u << lane) - 1u));
         if (hit && pos < cap) {
@@ -555,7 +591,40 @@ __global__ void __launch_bounds__(NT_TC, 1)
     // warp's hit queue, which is drained while the next accumulator is not
     // ready: the accumulators are handed back at the pace of the slowest of
     // eight warps, so a hit costs the pass less the shorter it holds its warp.
+    // Where several lanes of a chunk have hits (short bases) draining them one by
+    // one costs more than a walk of all lanes over their own: 52 pairs of up to
+    // 34k rows, k = 50: 0.58 ms queued, 0.25 walked; 64 pairs of up to 1M rows,
+    // k = 32: 3.72 and 3.01.
     auto push = [&](const uint32_t (&r)[32], uint32_t pm, int jc) {
+      if (WALK && __popc(pm) > kWalkLanes) {
+        if (pm >> lane & 1u) {
+          uint32_t bits = 0;
+#pragma unroll
+          for (int i = 0; i < 32; i++) bits |= __uint_as_float(r[i]) <= thr ? (1u << i) : 0u;
+          if (jc + 32 > nbv) bits &= jc < nbv ? (1u << (nbv - jc)) - 1u : 0u;
+#pragma unroll 1
+          while (bits) {
+            const int i = __ffs(bits) - 1;
+            bits &= bits - 1;
+            uint32_t t16[16], t8[8], t4[4], t2[2];
+#pragma unroll
+            for (int z = 0; z < 16; z++) t16[z] = (i & 1) ? r[2 * z + 1] : r[2 * z];
+#pragma unroll
+            for (int z = 0; z < 8; z++) t8[z] = (i & 2) ? t16[2 * z + 1] : t16[2 * z];
+#pragma unroll
+            for (int z = 0; z < 4; z++) t4[z] = (i & 4) ? t8[2 * z + 1] : t8[2 * z];
+#pragma unroll
+            for (int z = 0; z < 2; z++) t2[z] = (i & 8) ? t4[2 * z + 1] : t4[2 * z];
+            if (rcount < cap) {
+              sel.candv[cbase + rcount] = __uint_as_float((i & 16) ? t2[1] : t2[0]);
+              sel.candi[cbase + rcount] = jc + i + id_off;
+            }
+            rcount++;
+          }
+        }
+        __syncwarp();
+        return;
+      }
       while (pm) {
         const int rank = hq + __popc(pm & ((1u << lane) - 1u));
         const bool on = pm >> lane & 1u;
@@ -617,7 +686,9 @@ __global__ void __launch_bounds__(NT_TC, 1)
       }
     };
 
-    for (int t = t_begin; t < t_end; t++, it++) {
+    const int lead = lead_tiles(t_end - t_begin);
+    for (int tt = t_begin - lead; tt < t_end; tt++, it++) {
+      const int t = RUN && tt < t_begin ? tt + lead : tt;
       const int a = it & 1;
       const uint32_t u = (uint32_t)(it >> 1);
       ok = mbar_wait(&tfull[a], u & 1, abort_flag, wl);
@@ -657,6 +728,38 @@ __global__ void __launch_bounds__(NT_TC, 1)
         // (thr is NaN in lanes without a query; an all-NaN chunk has no hit)
         const float f0 = __uint_as_float(m0), f1 = __uint_as_float(m1);
         const float f2 = __uint_as_float(m2), f3 = __uint_as_float(m3);
+        if (RUN) {
+          float m = fminf(fminf(f0, f1), fminf(f2, f3));
+          if (j0 + 128 > nbv) {
+            // the unit's last columns: past them the operands are zeros
+            const int left = nbv - j0, c = left >> 5;
+            m = left >= 32 ? f0 : INFINITY;
+            if (left >= 64) m = fminf(m, f1);
+            if (left >= 96) m = fminf(m, f2);
+            if (left > 0) {
+#pragma unroll
+              for (int i = 0; i < 31; i++) {
+                const uint32_t x = c == 0 ? r0[i] : c == 1 ? r1[i] : c == 2 ? r2[i] : r3[i];
+                if (i < (left & 31)) m = fminf(m, __uint_as_float(x));
+              }
+            }
+          }
+          // The two column halves of a row share what they have seen, one unit
+          // per CTA at a time only (a persistent grid's next unit would read the
+          // last one's): a late read costs some candidates, never one of
+          // them, as every value read is one of the row's.
+          if (!PERSIST) {
+            if (m < rmin) *lv_own = m;
+            m = fminf(m, *lv_other);
+          }
+          if (m < rmin) {
+            thr = __fadd_ru(m, slack);
+            // every candidate so far is above the new threshold: start over
+            if (thr < rmin) rcount = 0;
+            rmin = m;
+          }
+          if (tt < t_begin) continue;
+        }
         if (__any_sync(0xffffffffu, fminf(fminf(f0, f1), fminf(f2, f3)) <= thr)) {
           const uint32_t p0 = __ballot_sync(0xffffffffu, f0 <= thr);
           const uint32_t p1 = __ballot_sync(0xffffffffu, f1 <= thr);
@@ -819,7 +922,7 @@ static int make_map3(CUtensorMap *m, const void *ptr, uint64_t cols, uint64_t ro
   return OK;
 }
 
-template <int MODE, int C, bool L2, bool QS, bool PAIR>
+template <int MODE, int C, bool L2, bool QS, bool PAIR>  // MODE: the kernel's KMODE
 int launch(const TcOperands &op, int nq, int nb, const ScanSel &sel, cudaStream_t st) {
   const int nkb = op.Kp / 64;
   int S = 12;
@@ -900,6 +1003,15 @@ int launch(const TcOperands &op, int nq, int nb, const ScanSel &sel, cudaStream_
 
 template <bool L2, bool QS, bool PAIR>
 int dispatch(const TcOperands &op, int nq, int nb, const ScanSel &sel, cudaStream_t st) {
+  if (sel.mode == SCAN_THRESH && sel.run_eps) {
+    if (sel.units) {
+      set_error(E_UNSUPPORTED, "tc_scan: grouped pass with running thresholds");
+      return E_UNSUPPORTED;
+    }
+    return launch<SCAN_RUN, 1, L2, QS, PAIR>(op, nq, nb, sel, st);
+  }
+  if (sel.mode == SCAN_THRESH && sel.queue)
+    return launch<SCAN_QUEUE, 1, L2, QS, PAIR>(op, nq, nb, sel, st);
   if (sel.mode == SCAN_THRESH) return launch<SCAN_THRESH, 1, L2, QS, PAIR>(op, nq, nb, sel, st);
   switch (sel.C) {
     case 1: return launch<SCAN_TOPC, 1, L2, QS, PAIR>(op, nq, nb, sel, st);

@@ -359,3 +359,19 @@ def test_nearest_running_thresholds(nq, nb, prec):
     ref1, _, _ = gpu_knn(b, q[[5, nq - 1]], 1, prec)
     np.testing.assert_array_equal(idx2[[5, nq - 1]], ref1)
     assert assign_mismatches(q[sel], b, idx2[sel, 0].copy(), NT)[0] == 0
+
+
+@pytest.mark.parametrize("prec", PRECS)
+@pytest.mark.parametrize("nq,nb,k", [(300, 420, 20), (257, 8192, 100), (513, 1716, 100),
+                                     (130, 3000, 20), (129, 8193, 50)])
+def test_short_base_thresholds(nq, nb, k, prec):
+    """More than sixteen neighbours in bases of a few thousand rows: thresholds
+    from the shortest samples, clustered and sorted rows (samples that mislead)."""
+    rng = np.random.default_rng(nb + k)
+    b = rng.standard_normal((nb, 24)).astype(np.float32)
+    q = rng.standard_normal((nq, 24)).astype(np.float32)
+    assert_exact(b, q, k, prec)
+    b[::max(1, k // 3)] *= 3                      # the sampled rows are the far ones
+    assert_exact(b, q, k, prec)
+    b = b[np.argsort((b ** 2).sum(1), kind="stable")].copy()
+    assert_exact(b, q, k, prec)

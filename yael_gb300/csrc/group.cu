@@ -116,7 +116,8 @@ void pair_layout(int nb, int stride, bool inf, int *nreg, int *cap, int *tpc) {
   }
 }
 
-bool pair_inf(int nb, int stride) { return nb <= kMaxCandidates || nb / stride < 4 * kSampleC; }
+// a pair whose sample is too short for a threshold (knn.cu)
+bool pair_inf(int nb, int stride) { return nb / stride < 4 * kSampleC; }
 
 struct Wave {
   std::vector<int> pairs;  // indices into the caller's pair array

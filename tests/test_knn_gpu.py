@@ -375,3 +375,25 @@ def test_short_base_thresholds(nq, nb, k, prec):
     assert_exact(b, q, k, prec)
     b = b[np.argsort((b ** 2).sum(1), kind="stable")].copy()
     assert_exact(b, q, k, prec)
+
+
+@pytest.mark.parametrize("nq,nb,d,k", [(1, 130, 7, 1), (33, 1, 5, 1), (31, 600, 16, 2),
+                                       (129, 127, 33, 1), (700, 9000, 17, 1), (64, 5000, 100, 5),
+                                       (2000, 40_000, 12, 10), (300, 2200, 65, 3)])
+def test_fp32_row_tiles(nq, nb, d, k):
+    """The FP32 pass at the edges of its tiles, slices and chunks: aligned and
+    unaligned rows, running thresholds in one and in many regions, samples in
+    single values and in minima; clustered, integer and repeated rows."""
+    rng = np.random.default_rng(nq + nb)
+    b = rng.standard_normal((nb, d)).astype(np.float32)
+    q = rng.standard_normal((nq, d)).astype(np.float32)
+    assert_exact(b, q, k, "fp32")
+    bi, qi = np.round(b).astype(np.float32), np.round(q).astype(np.float32)
+    bi[nb // 2:] = bi[:nb - nb // 2]
+    st = assert_exact(bi, qi, k, "fp32")
+    assert st["exact_class"] == 1
+    b = b[np.argsort(-(b ** 2).sum(1), kind="stable")].copy()
+    assert_exact(b, q, k, "fp32")
+    idx, _, _ = gpu_knn(b, q, k, "fp32", dt=16)
+    dots = q.astype(np.float64) @ b.astype(np.float64).T
+    np.testing.assert_array_equal(idx, np.argsort(dots, axis=1, kind="stable")[:, :k])

@@ -121,11 +121,52 @@ int running_chunks(int nqt, int ntb, int num_sms) {
 }
 int running_cap(int nchunk) { return imin(8, 32 / (2 * nchunk)); }
 
+// the smallest c that a Poisson(m) reaches with a probability of 2e-5 at most
+int sample_rank(double m) {
+  double p = exp(-m), tail = 1.0 - p;  // P(X >= 1)
+  int c = 1;
+  while (tail > 2e-5 && c < 64) {
+    p *= m / c;
+    tail -= p;
+    c++;
+  }
+  return c;
+}
+
+// stride and rank of the threshold sample (knn_batch)
+struct SamplePlan {
+  int stride, c;
+  SamplePlan(int k, int nb, bool bf16) {
+    const bool big = bf16 && k >= 96 && nb / (k / 6) >= kSampleMin;
+    c = big ? 19 : 13;
+    stride = imax(1, k / (big ? 6 : 3));
+    // The FP32 pass costs its sample more than its candidates: at least a
+    // 1/16 sample while it keeps 256 rows.  1,000 x 100k, d = 100, k = 20: 1/6
+    // of the base and 78 candidates 270 us, 1/16 and 144 candidates 52 (the
+    // re-rank 6 us longer).
+    const int s = imin(16, nb / 256);
+    if (!bf16 && s > stride) {
+      stride = s;
+      c = sample_rank((double)k / s);
+    }
+  }
+  bool usable(int nb) const { return stride > 1 && nb / stride >= 4 * c; }
+};
+
 int list_length(int k, int exact, int nb) {
   (void)nb;
   if (k == 1) return 8;
   if (exact) return k;
   return k <= 4 ? 8 : 2 * k;
+}
+
+// out[q] = the least of n rows of nq values
+__global__ void min_rows_kernel(const float *v, int nq, int n, float *out) {
+  const int q = blockIdx.x * blockDim.x + threadIdx.x;
+  if (q >= nq) return;
+  float m = INFINITY;
+  for (int r = 0; r < n; r++) m = fminf(m, v[(long)r * nq + q]);
+  out[q] = m;
 }
 
 __global__ void fill_f32(float *p, long n, float v) {
@@ -315,10 +356,12 @@ int knn_batch(KnnJob &job, Ctx *ctx, cudaStream_t st, Small *dsmall, BaseOps *bo
 
   const bool timed = job.timing || trace_enabled();
   const int tile_n = bf16 ? TC_TILE_N : SIMT_TILE_N;
-  const int tile_m = bf16 ? TC_TILE_M : 128;
+  const int tile_m = bf16 ? TC_TILE_M : simt_tile_m(nq, nb, ctx->num_sms);
   const int nqt = (int)ceil_div(nq, tile_m);
   const int ntb = (int)ceil_div(nb, tile_n);
-  const int ctas_per_sm = 1;
+  const int ctas_per_sm = bf16 ? 1 : 2;
+  // (few CTAs in all: single tiles, so that every SM has some)
+  const int min_tiles = bf16 || (long)nqt * ntb > 8L * ctx->num_sms ? 4 : 1;
   // oversampling for inexact distances: the certificate needs a margin between
   // the k-th exact value and the first excluded candidate
   const int c_needed = list_length(k, bstats_exact, nb);
@@ -346,27 +389,45 @@ int knn_batch(KnnJob &job, Ctx *ctx, cudaStream_t st, Small *dsmall, BaseOps *bo
     YG_CHECK(scan_parts(job, *up, *bops, dsmall, tcq, nq, sel, pnch, ptpc, pfirst, ptm, st));
     tm_scan->stop(st);
     job.scan_launches += up->nparts;
-  } else if (const int rc = !band && !prior && bf16 && k == 1
-                                ? running_chunks(nqt, ntb, ctx->num_sms) : 0) {
+  } else if (const int rc = band || prior || k != 1 ? 0
+                            : bf16 ? running_chunks(nqt, ntb, ctx->num_sms)
+                                   : choose_chunks(nqt, ntb, ctx->num_sms, ctas_per_sm,
+                                                   min_tiles)) {
     // ---- the nearest row, thresholds running with the smallest value seen
     sel.mode = SCAN_THRESH;
-    sel.halves = 2;
+    sel.halves = bf16 ? 2 : 1;
+    sel.tile_m = tile_m;
     sel.run_eps = eps;
     const int nchunk = tune_chunks(TuneKey{4, job.prec, nqt, ntb, 0}, rc,
-                                   imax(1, imin(4, ntb / 4)), ctx->num_sms * ctas_per_sm,
-                                   &scan_ticket);
+                                   bf16 ? imax(1, imin(4, ntb / 4)) : imin(1024, ntb),
+                                   ctx->num_sms * ctas_per_sm, &scan_ticket);
     sel.tiles_per_chunk = (int)ceil_div(ntb, nchunk);
     sel.nchunk = (int)ceil_div(ntb, sel.tiles_per_chunk);
-    sel.cap = running_cap(sel.nchunk);
+    sel.cap = bf16 ? running_cap(sel.nchunk) : 8;
     const long nr = sel.nregion();
     YG_CHECK(ws_get(ws, WS_CNT, (size_t)nr * nq, &sel.cnt));
     YG_CHECK(ws_get(ws, WS_TOPV, (size_t)nr * nq * sel.cap, &sel.candv));
     YG_CHECK(ws_get(ws, WS_TOPI, (size_t)nr * nq * sel.cap, &sel.candi));
     tm_scan.reset(new PassTimer(timed || scan_ticket >= 0, st, &job.ms_scan));
+    // more regions than the short re-rank's slots: their last thresholds' least
+    // one is the query's
+    const bool many = sel.nregion() * sel.cap > 32;
+    if (many) {
+      YG_CHECK(ws_get(ws, WS_STOPV, (size_t)nr * nq, &sel.run_thr));
+      ra.m_expect = (int)nr;
+    }
     YG_CHECK(scan(job, job.q, nq, job.b, job.ldb, nb, bn32, 1, &tcq, sel, st));
     tm_scan->stop(st);
+    if (many) {
+      float *thr;
+      YG_CHECK(ws_get(ws, WS_THR, nq, &thr));
+      min_rows_kernel<<<(unsigned)ceil_div(nq, 256), 256, 0, st>>>(sel.run_thr, nq, (int)nr, thr);
+      YG_LAUNCH_CHECK();
+      sel.thr = thr;
+      sel.run_eps = nullptr;
+    }
     job.scan_launches++;
-  } else if (!band && !prior && c_needed <= 16) {
+  } else if (bf16 && !band && !prior && c_needed <= 16) {
     // ---- TOPC over the full base (register lists)
     sel.mode = SCAN_TOPC;
     sel.C = pow2_at_least(c_needed);
@@ -395,13 +456,12 @@ int knn_batch(KnnJob &job, Ctx *ctx, cudaStream_t st, Small *dsmall, BaseOps *bo
     // of the base and its pass takes block minima (k = 100: 1/16 of the base).
     // The sample pass keeps 16 values per row and chunk.
     sel.mode = SCAN_THRESH;
-    sel.halves = 2;
+    sel.halves = bf16 ? 2 : 1;
+    sel.tile_m = tile_m;
     float *thr;
     YG_CHECK(ws_get(ws, WS_THR, nq, &thr));
-    const bool big = bf16 && k >= 96 && nb / (k / 6) >= kSampleMin;
-    const int c = big ? 19 : 13;
-    int stride = k / (big ? 6 : 3);
-    if (stride < 1) stride = 1;
+    const SamplePlan plan(k, nb, bf16);
+    const int c = plan.c, stride = plan.stride;
     const int ns = nb / stride;
     if (up) {
       sel.nchunk = part_chunks(*up, 1, job.prec, 0, nqt, tile_n, ctx->num_sms * ctas_per_sm,
@@ -412,7 +472,8 @@ int knn_batch(KnnJob &job, Ctx *ctx, cudaStream_t st, Small *dsmall, BaseOps *bo
       sel.nchunk = band    ? 1
                    : prior ? choose_chunks(nqt, ntb, ctx->num_sms, ctas_per_sm, 4)
                            : tune_chunks(TuneKey{1, job.prec, nqt, ntb, 0},
-                                         choose_chunks(nqt, ntb, ctx->num_sms, ctas_per_sm, 4),
+                                         choose_chunks(nqt, ntb, ctx->num_sms, ctas_per_sm,
+                                                       min_tiles),
                                          1024, ctx->num_sms * ctas_per_sm, &scan_ticket);
       sel.tiles_per_chunk = (int)ceil_div(ntb, sel.nchunk);
       sel.nchunk = (int)ceil_div(ntb, sel.tiles_per_chunk);
@@ -429,8 +490,9 @@ int knn_batch(KnnJob &job, Ctx *ctx, cudaStream_t st, Small *dsmall, BaseOps *bo
       sns = (int)(n0 / sstride);
     }
     // a long sample is read in blocks (whole super tiles of it)
-    const bool blockmin = bf16 && sns >= kSampleMin;
-    if (blockmin) sns -= sns % kSampleSuper;
+    // (FP32: minima of 8 rows, from a few hundred of them on)
+    const bool blockmin = sns >= (bf16 ? kSampleMin : 4096);
+    if (blockmin && bf16) sns -= sns % kSampleSuper;
     if (band) {
       // thresholds from the k-th exact distance an earlier pass found
       const BandLayout L = band_layout(nq, nb, k, tile_m, tile_n, sel.halves, ctx->num_sms);
@@ -443,7 +505,7 @@ int knn_batch(KnnJob &job, Ctx *ctx, cudaStream_t st, Small *dsmall, BaseOps *bo
       sel.cap = prior_cap(sel.nchunk);
       sel.queue = nb >= 8192;  // a few rows in the band of the bound
       YG_CHECK(band_thresholds(nq, job.metric, job.prior_kth, qn64, eps, thr, st));
-    } else if (sns < 4 * c) {
+    } else if (up ? sns < 4 * c : !plan.usable(nb)) {
       // The sample is too short for a threshold: every base row is a candidate,
       // a region holds at most its share of the chunk.  (A sample pays on
       // short bases too: the re-rank sorts what it is given.  10k x 8,000,
@@ -464,9 +526,12 @@ int knn_batch(KnnJob &job, Ctx *ctx, cudaStream_t st, Small *dsmall, BaseOps *bo
       ScanSel ss;
       ss.mode = SCAN_TOPV;  // only the c-th value is needed
       ss.C = 16;
+      ss.tile_m = tile_m;
+      ss.blockmin = blockmin ? 1 : 0;
       const int nts = (int)ceil_div(sns, tile_n);
       int nch = tune_chunks(TuneKey{2, job.prec, nqt, nts, ss.C},
-                                  choose_chunks(nqt, nts, ctx->num_sms, ctas_per_sm, 2), 64,
+                                  choose_chunks(nqt, nts, ctx->num_sms, ctas_per_sm,
+                                                imin(2, min_tiles)), 64,
                                   ctx->num_sms * ctas_per_sm, &sample_ticket);
       if (c > ss.C) nch = imax(nch, 2);  // the lists together hold the c-th value
       ss.tiles_per_chunk = (int)ceil_div(nts, nch);
@@ -476,7 +541,6 @@ int knn_batch(KnnJob &job, Ctx *ctx, cudaStream_t st, Small *dsmall, BaseOps *bo
       tm_sample.reset(new PassTimer(timed || sample_ticket >= 0, st, &job.ms_sample));
       if (bf16) {
         TcOperands tcs = tcq;
-        ss.blockmin = blockmin ? 1 : 0;
         YG_CHECK(tc_base_view(tcq, sstride, sns, &tcs));
         YG_CHECK(tc_scan(tcs, nq, sns, ss, st));
       } else {
@@ -662,7 +726,19 @@ int knn_batches(KnnJob &job, Ctx *ctx, cudaStream_t st, Small *dsmall, BaseOps *
     const int nqt = (int)ceil_div(nq, tile_m), ntb = (int)ceil_div(nb, tile_n);
     const int C = pow2_at_least(cn);
     size_t per_query;
-    if (cn <= 16) {
+    if (!bf16) {
+      // running thresholds: 8 slots a region; else the regions' share of the
+      // candidates, or the whole base where it is too short for a sample
+      const int m = simt_tile_m(nq, nb, ctx->num_sms), nt = (int)ceil_div(nq, m);
+      const int nch = imin(imin(1024, ntb), 3 * choose_chunks(nt, ntb, ctx->num_sms, 2, 1) + 2);
+      const SamplePlan plan(k, nb, false);
+      const double er = (double)plan.c * plan.stride / nch;
+      const size_t cap = k == 1 ? 8
+                         : plan.usable(nb)
+                             ? pow2_at_least((int)(2.0 * er + 6.0 * sqrt(er) + 16.0))
+                             : 2 * (size_t)ceil_div(nb, nch) + 2 * tile_n;
+      per_query = (size_t)nch * (cap * 8 + 8) + 64 * 16 * 4 + 64;
+    } else if (cn <= 16) {
       // the autotuner may try up to 3x the heuristic's chunk count
       const int nch = imin(imin(1024, kMaxCandidates / C),
                            3 * choose_chunks(nqt, ntb, ctx->num_sms, 1, 4) + 2);

@@ -11,12 +11,12 @@
 //             topv/topi[(chunk * nq + q) * C + s], ascending.
 //   THRESH -- every (q, j) with v <= thr[q] is appended to a candidate
 //             region owned by one thread: region r = chunk * halves + column
-//             half (halves = 2 for the CUDA-core producer, whose two threads
-//             of a row split the columns; 1 for the tensor-core one), slots
+//             half (halves = 2 for the tensor-core producer, whose two warps
+//             of a row split the columns; 1 for the CUDA-core one), slots
 //             candv/candi[(r * nq + q) * cap + s], count cnt[r * nq + q] (all
 //             hits, including those that did not fit in cap).  No atomics:
 //             each (region, query) has exactly one writer.
-//             With run_eps (tc_scan, k = 1) the threshold is not given but runs:
+//             With run_eps (k = 1) the threshold is not given but runs:
 //             the smallest v the region has seen plus run_slack(eps).  A
 //             region starts over when its threshold falls below all its
 //             candidates, so it ends with the few rows that can still be the
@@ -91,6 +91,10 @@ struct ScanSel {
   // THRESH (tc_scan): well under one hit in 32 rows x 32 columns expected, or
   // nearly all of them hits: both are best drained a row of 32 at a time
   int queue = 0;
+  // FP32 pass: query rows per tile (simt_tile_m); running thresholds: where a
+  // region's last threshold goes ([region][query], may be null)
+  int tile_m = 128;
+  float *run_thr = nullptr;
   int f16 = 0;              // tensor-core passes: fp16 operands (else bf16)
   // tensor-core passes: bound of every wait (0: kWaitLimitNs), and a test
   // switch under which the producer issues no load, so that the consumers'
@@ -122,7 +126,10 @@ constexpr int kSampleD = 32, kSampleSuper = 32 * kSampleD, kSampleMin = 4 * kSam
 // FP32 CUDA-core producer.  q: nq rows (stride ldq floats); b: nb rows (stride
 // ldb floats); bn: ||b||^2 as float with stride bn_stride (L2 only).
 // Base tiles are 128 rows.  Reported base ids are j (row index in this view).
+// THRESH regions are chunks (halves = 1); a TOPV pass with blockmin lists the
+// minima of 8 rows.  TOPC lists are the allocation-free call's.
 constexpr int SIMT_TILE_N = 128;
+int simt_tile_m(int nq, int nb, int num_sms);
 int simt_scan(const float *q, long ldq, int nq, const float *b, long ldb, int nb,
               int d, const float *bn, long bn_stride, int metric, const ScanSel &sel,
               cudaStream_t st);

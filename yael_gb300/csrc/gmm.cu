@@ -10,8 +10,8 @@
 //     component and dimension (FP32 within each step of 32 vectors, pairs of
 //     floats across steps, FP64 across vector slices, summed in a fixed order:
 //     every result is reproducible), skipping zero posteriors.
-// The EM update of the k x d parameters, the empty-component splits and the
-// Fisher-vector formulas are host code over those moments.  The posterior
+// Fisher vectors are formed on the device from those moments; the EM update of the
+// k x d parameters and the empty-component splits are host code over them.  The posterior
 // matrix (n x k) stays on the device between the passes of an EM iteration.
 #include <cuda_runtime.h>
 #include <math.h>
@@ -486,6 +486,97 @@ __global__ void sum_slices_kernel(const double *__restrict__ part, int nz, long 
   out[t] = s;
 }
 
+// --- parameters --------------------------------------------------------------
+// From a mixture's (w, mu, sigma): 1 / sigma, and the constant terms of the log
+// density of each component, log det + log w (yael/gmm.c:311-330, the
+// determinant accumulated in float as there), in two floats.  A warp per
+// component: the logarithms by its lanes, their sum in order.
+__global__ void params_kernel(const float *__restrict__ w, const float *__restrict__ sigma, int k,
+                              int d, float det0, int use_w, float *__restrict__ isig,
+                              float *__restrict__ hi, float *__restrict__ lo) {
+  const int lane = threadIdx.x & 31;
+  const int j = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (j >= k) return;  // whole warps leave together
+  float det = det0;
+  for (int l0 = 0; l0 < d; l0 += 32) {
+    const int l = l0 + lane;
+    double h = 0.0;
+    if (l < d) {
+      const double sg = sigma[(long)j * d + l];
+      isig[(long)j * d + l] = (float)(1.0 / sg);
+      h = 0.5 * log(sg);
+    }
+    const int m = min(32, d - l0);
+    for (int s = 0; s < m; s++) det = (float)((double)det - __shfl_sync(0xffffffffu, h, s));
+  }
+  if (lane == 0) {
+    const double base = (double)det + (use_w ? (double)(float)log((double)w[j]) : 0.0);
+    const float h = (float)base;
+    hi[j] = h;
+    lo[j] = isfinite(base) ? (float)(base - (double)h) : 0.f;
+  }
+}
+
+// --- Fisher vectors ------------------------------------------------------------
+// gmm_fisher_from_posteriors (yael/gmm.c:527-725) from the FP64 moments
+// (S1[k][d], S2[k][d], S0[k]), each operation rounded on its own as in C.  On the
+// device so that one image's vector comes back as floats: moving the moments
+// to the host and dividing there took longer than all the passes of 2,000
+// descriptors.  Thread t < k*d: dimension t % d of component t / d; the parts
+// that sum over dimensions (GMM_FLAGS_1SIGMA) go a component per thread.
+__device__ __forceinline__ double dev2_of(double mu, double s0, double s1, double s2) {
+  return __dadd_rn(__dsub_rn(s2, __dmul_rn(__dmul_rn(2.0, mu), s1)), __dmul_rn(__dmul_rn(mu, mu), s0));
+}
+
+__global__ void fisher_kernel(const double *__restrict__ sum, const float *__restrict__ w,
+                              const float *__restrict__ mu, const float *__restrict__ sigma,
+                              long n, int k, int d, int flags, float *__restrict__ out) {
+  const long kd = (long)k * d, t = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  const double *s1 = sum, *s2 = sum + kd, *s0 = sum + 2 * kd;
+  const bool norm = !(flags & YAEL_GMM_FLAGS_NO_NORM);
+  if (flags & YAEL_GMM_FLAGS_W) {
+    if (t >= 1 && t < k) {
+      const double accu = __dsub_rn(s0[t] / w[t], s0[0] / w[0]);
+      const double f = __dmul_rn((double)n, __dadd_rn(1.0 / w[t], 1.0 / w[0]));
+      out[t - 1] = (float)(accu / sqrt(f));
+    }
+    out += k - 1;
+  }
+  if (t >= kd) return;
+  const int j = (int)(t / d);
+  const double m = mu[t], sg = sigma[t], wj = w[j];
+  if (flags & YAEL_GMM_FLAGS_MU) {
+    double x = __dsub_rn(s1[t], __dmul_rn(m, s0[j])) / sg;
+    if (norm) {
+      const double nf = sqrt(__dmul_rn((double)n, wj) / sg);
+      if (nf > 0) x /= nf;
+    }
+    out[t] = (float)x;
+    out += kd;
+  }
+  if (flags & YAEL_GMM_FLAGS_1SIGMA) {
+    if (t != (long)j * d) return;
+    const bool each = flags & YAEL_GMM_FLAGS_SIGMA;
+    float *o = out + (each ? (long)j * (d + 1) : j);
+    double accu2 = 0;
+    for (int l = 0; l < d; l++) {
+      const long u = t + l;
+      const double su = sigma[u];
+      const double accu =
+          __dsub_rn(dev2_of(mu[u], s0[j], s1[u], s2[u]) / su, s0[j]) / sqrt(su);
+      if (each)
+        *o++ = (float)(accu / sqrt(norm ? __dmul_rn((double)(2 * n), wj) / su : 1.0));
+      accu2 = __dadd_rn(accu2, accu);
+    }
+    *o = (float)(accu2 / sqrt(norm ? __dmul_rn((double)(2 * d * n), wj) / sg : 1.0));
+  } else if (flags & YAEL_GMM_FLAGS_SIGMA) {
+    const double accu = __dsub_rn(dev2_of(m, s0[j], s1[t], s2[t]), __dmul_rn(s0[j], sg));
+    const double f =
+        norm ? 1 / __dmul_rn(sg, sqrt(__dmul_rn((double)(2 * n), wj))) : pow(sg, -1.5);
+    out[t] = (float)__dmul_rn(accu, f);
+  }
+}
+
 // nnz[j] += number of vectors of slice y with P[i*k + j] > 0.  Block 32 x 8:
 // thread (tx, ty) counts component j0 + tx over vectors ty, ty + 8, ...
 __global__ void nnz_kernel(const float *__restrict__ P, long n, int k, long chunk,
@@ -539,11 +630,38 @@ void launched(const char *where) {
   ok(where, cudaGetLastError());
 }
 
-// The moments of a posterior matrix against a set of vectors, as FP64:
-// s0[j] = sum_i p_ij, s1[j*d + l] = sum_i p_ij x_il, s2[j*d + l] = sum_i p_ij x_il^2
+// The moments of a posterior matrix against a set of vectors, as FP64, in
+// pinned memory of the context: s0[j] = sum_i p_ij, s1[j*d + l] = sum_i p_ij x_il,
+// s2[j*d + l] = sum_i p_ij x_il^2
 struct Moments {
-  std::vector<double> s0, s1, s2;
+  const double *s0, *s1, *s2;
 };
+
+// A device array of a call: workspace of the calling thread up to kKeepBytes
+// (one image's descriptors: allocating and freeing ten arrays took 0.4 of a
+// 0.6 ms call), an allocation of the call's own above (given back at its end).
+constexpr size_t kKeepBytes = (size_t)32 << 20;
+enum GmmSlot : int {
+  GM_V = 260, GM_P, GM_PRM, GM_ISIG, GM_HI, GM_LO, GM_PART, GM_SUM, GM_NNZ, GM_MOVED, GM_OUT,
+};
+template <typename T, int SLOT>
+struct GmmArray {
+  T *p = nullptr;
+  DevArray<T> own;
+  T *get(Ctx *ctx, const char *where, long want) {
+    const size_t bytes = sizeof(T) * (size_t)(want > 1 ? want : 1);
+    if (bytes > kKeepBytes) {
+      p = own.get(where, want);
+    } else {
+      void *q = nullptr;
+      if (ctx->ws.get(SLOT, bytes, &q) != OK) die(where);
+      p = static_cast<T *>(q);
+    }
+    return p;
+  }
+};
+// pinned buffers: parameters and small vectors on their way up, moments down
+enum GmmPinned : int { GP_PRM = 8, GP_V, GP_MOMENTS };
 
 // device state of one call: vectors, posteriors, parameters, moments
 struct GmmDev {
@@ -551,55 +669,75 @@ struct GmmDev {
   Ctx *ctx = nullptr;
   long n = 0;
   int d = 0, k = 0;
-  DevArray<float> v, P, mu, isig, dhi, dlo;
-  DevArray<double> part, sum;
-  DevArray<int> nnz, moved;
+  GmmArray<float, GM_V> v;
+  GmmArray<float, GM_P> P;
+  GmmArray<float, GM_PRM> prm;  // mu[k][d], sigma[k][d], w[k]
+  GmmArray<float, GM_ISIG> isig;
+  GmmArray<float, GM_HI> dhi;
+  GmmArray<float, GM_LO> dlo;
+  GmmArray<double, GM_PART> part;
+  GmmArray<double, GM_SUM> sum;
+  GmmArray<int, GM_NNZ> nnz;
+  GmmArray<int, GM_MOVED> moved;
+  GmmArray<float, GM_OUT> fv;
 
   GmmDev(const char *w, long n_, int d_, int k_) : where(w), n(n_), d(d_), k(k_) {
     if (ctx_get(&ctx) != OK) die(where);
   }
   void sync() { ok(where, cudaStreamSynchronize(ctx->stream)); }
+  void *pinned(int slot, size_t bytes) {
+    void *h = nullptr;
+    if (ctx->pinned.get(slot, bytes, &h) != OK) die(where);
+    return h;
+  }
   void upload_v(const float *hv) {
-    ok(where, cudaMemcpyAsync(v.get(where, n * d), hv, sizeof(float) * (size_t)(n * d),
-                              cudaMemcpyHostToDevice, ctx->stream));
+    const size_t bytes = sizeof(float) * (size_t)(n * d);
+    v.get(ctx, where, n * d);
+    const void *src = hv;
+    // (a small pageable copy goes through pinned memory here rather than by
+    // the driver's own staging, which waits for it)
+    if (bytes <= (size_t)1 << 20) src = memcpy(pinned(GP_V, bytes), hv, bytes);
+    ok(where, cudaMemcpyAsync(v.p, src, bytes, cudaMemcpyHostToDevice, ctx->stream));
   }
   void upload_P(const float *hp) {
-    ok(where, cudaMemcpyAsync(P.get(where, n * k), hp, sizeof(float) * (size_t)(n * k),
+    ok(where, cudaMemcpyAsync(P.get(ctx, where, n * k), hp, sizeof(float) * (size_t)(n * k),
                               cudaMemcpyHostToDevice, ctx->stream));
   }
   void download_P(float *hp) {
-    ok(where, cudaMemcpyAsync(hp, P.p, sizeof(float) * (size_t)(n * k), cudaMemcpyDeviceToHost,
-                              ctx->stream));
-    sync();
+    if (copy_to_host(ctx, ctx->stream, hp, P.p, sizeof(float) * (size_t)(n * k)) != OK) die(where);
   }
+
+  // the mixture on the device (one copy from pinned memory; the caller
+  // synchronises before the next)
+  void upload_params(const gmm_t *g) {
+    const size_t kd = (size_t)k * d, m = 2 * kd + k;
+    float *h = static_cast<float *>(pinned(GP_PRM, sizeof(float) * m));
+    memcpy(h, g->mu, sizeof(float) * kd);
+    memcpy(h + kd, g->sigma, sizeof(float) * kd);
+    memcpy(h + 2 * kd, g->w, sizeof(float) * k);
+    ok(where, cudaMemcpyAsync(prm.get(ctx, where, (long)m), h, sizeof(float) * m,
+                              cudaMemcpyHostToDevice, ctx->stream));
+  }
+  const float *mu_dev() const { return prm.p; }
+  const float *sigma_dev() const { return prm.p + (size_t)k * d; }
+  const float *w_dev() const { return prm.p + 2 * (size_t)k * d; }
 
   // P = p(component | vector) for the mixture (w, mu, sigma): gmm_compute_p
   // (yael/gmm.c:305-362); flags & GMM_FLAGS_W adds log w_j.  count: also leave
   // the number of vectors with a positive posterior per component in nnz.
   void posteriors(const gmm_t *g, int flags, bool count = false) {
-    std::vector<float> hhi((size_t)k), hlo((size_t)k), his((size_t)k * d);
     const long kd = (long)k * d;
-    for (long t = 0; t < kd; t++) his[t] = (float)(1.0 / g->sigma[t]);
-    for (int j = 0; j < k; j++) {
-      float det = (float)(-d / 2.0 * log(2 * M_PI));  // float accumulation as the reference
-      for (int l = 0; l < d; l++) det = (float)(det - 0.5 * log(g->sigma[(long)j * d + l]));
-      // the constant terms of the log density in two floats
-      const double base = (double)det + (double)((flags & YAEL_GMM_FLAGS_W) ? (float)log(g->w[j])
-                                                                              : 0.f);
-      hhi[j] = (float)base;
-      hlo[j] = isfinite(base) ? (float)(base - (double)hhi[j]) : 0.f;
-    }
     cudaStream_t st = ctx->stream;
-    ok(where, cudaMemcpyAsync(mu.get(where, kd), g->mu, sizeof(float) * kd,
-                              cudaMemcpyHostToDevice, st));
-    ok(where, cudaMemcpyAsync(isig.get(where, kd), his.data(), sizeof(float) * kd,
-                              cudaMemcpyHostToDevice, st));
-    ok(where, cudaMemcpyAsync(dhi.get(where, k), hhi.data(), sizeof(float) * k,
-                              cudaMemcpyHostToDevice, st));
-    ok(where, cudaMemcpyAsync(dlo.get(where, k), hlo.data(), sizeof(float) * k,
-                              cudaMemcpyHostToDevice, st));
-    P.get(where, n * k);
-    if (count) ok(where, cudaMemsetAsync(nnz.get(where, k), 0, sizeof(int) * k, st));
+    upload_params(g);
+    isig.get(ctx, where, kd);
+    dhi.get(ctx, where, k);
+    dlo.get(ctx, where, k);
+    params_kernel<<<(unsigned)((k + 3) / 4), 128, 0, st>>>(
+        w_dev(), sigma_dev(), k, d, (float)(-d / 2.0 * log(2 * M_PI)),
+        (flags & YAEL_GMM_FLAGS_W) != 0, isig.p, dhi.p, dlo.p);
+    launched(where);
+    P.get(ctx, where, n * k);
+    if (count) ok(where, cudaMemsetAsync(nnz.get(ctx, where, k), 0, sizeof(int) * k, st));
     int *cnt = count ? nnz.p : nullptr;
     // The largest tile of vectors whose rows fit in shared memory and that
     // still gives every SM a CTA; k above about 2,300 fits none.
@@ -616,7 +754,6 @@ struct GmmDev {
       launched(where);
       if (count) count_nonzeros();
     }
-    sync();  // the host arrays above are freed on return
   }
 
   bool fits(int vr) const { return maha_floats(vr, k) * sizeof(float) <= ctx->smem_optin; }
@@ -626,7 +763,7 @@ struct GmmDev {
     const size_t smem = maha_floats(VR, FUSED ? k : 0) * sizeof(float);
     if (ensure_smem((const void *)posterior_kernel<VR, FUSED>, smem) != OK) die(where);
     posterior_kernel<VR, FUSED><<<(unsigned)((n + 16 * VR - 1) / (16 * VR)), MT, smem,
-                                  ctx->stream>>>(v.p, mu.p, isig.p, dhi.p, dlo.p, n, k, d, P.p,
+                                  ctx->stream>>>(v.p, mu_dev(), isig.p, dhi.p, dlo.p, n, k, d, P.p,
                                                  cnt);
     launched(where);
   }
@@ -651,7 +788,7 @@ struct GmmDev {
 
   int transfer(int j, int j2, int sd, float thr) {
     cudaStream_t st = ctx->stream;
-    ok(where, cudaMemsetAsync(moved.get(where, 1), 0, sizeof(int), st));
+    ok(where, cudaMemsetAsync(moved.get(ctx, where, 1), 0, sizeof(int), st));
     transfer_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(P.p, v.p, n, k, d, j, j2, sd,
                                                                 thr, moved.p);
     launched(where);
@@ -672,18 +809,24 @@ struct GmmDev {
     const long chunk = (steps + nz - 1) / nz * 32;
     const long m = (long)k * (2L * d + 1);
     const long used = (n + chunk - 1) / chunk;
-    part.get(where, used * m);
+    part.get(ctx, where, used * m);
     const size_t smem = sizeof(float) * 2 * 32 * (XW + 2 * CT + 4);
     if (ensure_smem((const void *)moments_kernel<NW, DPL>, smem) != OK) die(where);
     moments_kernel<NW, DPL><<<dim3((unsigned)gx, (unsigned)gy, (unsigned)used), NW * 32, smem,
                               ctx->stream>>>(P.p, v.p, n, k, d, chunk, part.p);
     launched(where);
     sum_slices_kernel<<<(unsigned)((m + 255) / 256), 256, 0, ctx->stream>>>(
-        part.p, (int)used, m, sum.get(where, m));
+        part.p, (int)used, m, sum.get(ctx, where, m));
     launched(where);
   }
 
-  Moments moments() {
+  // the moments of P against v, in sum (S1, S2, S0)
+  void moments_dev() {
+    if (n == 0) {
+      const size_t m = (size_t)k * (2 * (size_t)d + 1);
+      ok(where, cudaMemsetAsync(sum.get(ctx, where, (long)m), 0, sizeof(double) * m, ctx->stream));
+      return;
+    }
     // Dimensions per lane by d.  16 warps to a CTA (fewer passes over the
     // vectors) where k gives the warps components of their own and n gives
     // every SM some steps; else 4-warp CTAs, four to an SM.
@@ -694,19 +837,34 @@ struct GmmDev {
     } else {
       if (k > 64 && many) launch_moments<16, 2>(); else launch_moments<4, 2>();
     }
-    const size_t kd = (size_t)k * d;
-    Moments r;
-    r.s1.resize(kd);
-    r.s2.resize(kd);
-    r.s0.resize((size_t)k);
-    cudaStream_t st = ctx->stream;
-    ok(where, cudaMemcpyAsync(r.s1.data(), sum.p, sizeof(double) * kd, cudaMemcpyDeviceToHost, st));
-    ok(where, cudaMemcpyAsync(r.s2.data(), sum.p + kd, sizeof(double) * kd,
-                              cudaMemcpyDeviceToHost, st));
-    ok(where, cudaMemcpyAsync(r.s0.data(), sum.p + 2 * kd, sizeof(double) * k,
-                              cudaMemcpyDeviceToHost, st));
+  }
+
+  Moments moments() {
+    moments_dev();
+    const size_t kd = (size_t)k * d, bytes = sizeof(double) * (2 * kd + k);
+    double *h = static_cast<double *>(pinned(GP_MOMENTS, bytes));
+    ok(where, cudaMemcpyAsync(h, sum.p, bytes, cudaMemcpyDeviceToHost, ctx->stream));
     sync();
-    return r;
+    return Moments{h + 2 * kd, h, h + kd};
+  }
+
+  // the Fisher vector of P (or of no vectors) under the mixture in prm
+  void fisher(int flags, float *out) {
+    const long m = (long)gmm_len(flags);
+    moments_dev();
+    if (m == 0) {
+      sync();
+      return;
+    }
+    const long t = std::max((long)k * d, (long)k);
+    fisher_kernel<<<(unsigned)((t + 127) / 128), 128, 0, ctx->stream>>>(
+        sum.p, w_dev(), mu_dev(), sigma_dev(), n, k, d, flags, fv.get(ctx, where, m));
+    launched(where);
+    if (copy_to_host(ctx, ctx->stream, out, fv.p, sizeof(float) * (size_t)m) != OK) die(where);
+  }
+  size_t gmm_len(int flags) const {
+    const gmm_t g{d, k, nullptr, nullptr, nullptr};
+    return gmm_fisher_sizeof(&g, flags);
   }
 };
 
@@ -834,70 +992,6 @@ void compute_params(GmmDev &dev, gmm_t *g, int flags) {
   printf(" imfac = %.3f\n", k * ss);
 }
 
-// gmm_fisher_from_posteriors (yael/gmm.c:527-725) from the moments
-void fisher_from_moments(const Moments &m, long n, const gmm_t *g, int flags, float *out) {
-  const long d = g->d, k = g->k;
-  long ii = 0;
-  auto MU = [&](long l, long j) { return (double)g->mu[j * d + l]; };
-  auto SG = [&](long l, long j) { return (double)g->sigma[j * d + l]; };
-  if (flags & YAEL_GMM_FLAGS_W) {
-    for (long j = 1; j < k; j++) {
-      const double accu = m.s0[j] / g->w[j] - m.s0[0] / g->w[0];
-      const double f = n * (1.0 / g->w[j] + 1.0 / g->w[0]);
-      out[ii++] = (float)(accu / sqrt(f));
-    }
-  }
-  if (flags & YAEL_GMM_FLAGS_MU) {
-    float *dmu = out + ii;
-    for (long j = 0; j < k; j++)
-      for (long l = 0; l < d; l++) {
-        double x = (m.s1[j * d + l] - MU(l, j) * m.s0[j]) / SG(l, j);
-        if (!(flags & YAEL_GMM_FLAGS_NO_NORM)) {
-          const double nf = sqrt(n * (double)g->w[j] / SG(l, j));
-          if (nf > 0) x /= nf;
-        }
-        dmu[j * d + l] = (float)x;
-      }
-    ii += d * k;
-  }
-  if (flags & (YAEL_GMM_FLAGS_SIGMA | YAEL_GMM_FLAGS_1SIGMA)) {
-    // sum_i p_ij (x_il - mu_jl)^2
-    auto dev2 = [&](long l, long j) {
-      const double mu = MU(l, j);
-      return m.s2[j * d + l] - 2.0 * mu * m.s1[j * d + l] + mu * mu * m.s0[j];
-    };
-    if (flags & YAEL_GMM_FLAGS_1SIGMA) {
-      for (long j = 0; j < k; j++) {
-        double accu2 = 0;
-        for (long l = 0; l < d; l++) {
-          const double sg = SG(l, j);
-          const double accu = (dev2(l, j) / sg - m.s0[j]) / sqrt(sg);
-          if (flags & YAEL_GMM_FLAGS_SIGMA) {
-            const double f = (flags & YAEL_GMM_FLAGS_NO_NORM) ? 1.0 : 2 * n * (double)g->w[j] / sg;
-            out[ii++] = (float)(accu / sqrt(f));
-          }
-          accu2 += accu;
-        }
-        const double f =
-            (flags & YAEL_GMM_FLAGS_NO_NORM) ? 1.0 : 2 * d * n * (double)g->w[j] / SG(0, j);
-        out[ii++] = (float)(accu2 / sqrt(f));
-      }
-    } else {
-      float *dsg = out + ii;
-      for (long j = 0; j < k; j++)
-        for (long l = 0; l < d; l++) {
-          const double sg = SG(l, j);
-          const double accu = dev2(l, j) - m.s0[j] * sg;
-          const double f = (flags & YAEL_GMM_FLAGS_NO_NORM)
-                               ? pow(sg, -1.5)
-                               : 1 / (sg * sqrt(2 * n * (double)g->w[j]));
-          dsg[l + j * d] = (float)(accu * f);
-        }
-      ii += d * k;
-    }
-  }
-}
-
 }  // namespace
 }  // namespace yg
 
@@ -983,33 +1077,24 @@ size_t gmm_fisher_sizeof(const gmm_t *g, int flags) {
 
 void gmm_fisher(int n, const float *v, const gmm_t *g, int flags, float *dp_dlambda) {
   GmmDev dev("gmm_fisher", n, g->d, g->k);
-  Moments m;
   if (n > 0) {
     dev.upload_v(v);
     dev.posteriors(g, flags | YAEL_GMM_FLAGS_W);
-    m = dev.moments();
   } else {
-    m.s0.assign((size_t)g->k, 0.0);
-    m.s1.assign((size_t)g->k * g->d, 0.0);
-    m.s2.assign((size_t)g->k * g->d, 0.0);
+    dev.upload_params(g);
   }
-  fisher_from_moments(m, n, g, flags, dp_dlambda);
+  dev.fisher(flags, dp_dlambda);
 }
 
 void gmm_fisher_from_posteriors(int n, const float *v, const gmm_t *g, int flags,
                                 const float *p, float *dp_dlambda) {
   GmmDev dev("gmm_fisher_from_posteriors", n, g->d, g->k);
-  Moments m;
   if (n > 0) {
     dev.upload_v(v);
     dev.upload_P(p);
-    m = dev.moments();
-  } else {
-    m.s0.assign((size_t)g->k, 0.0);
-    m.s1.assign((size_t)g->k * g->d, 0.0);
-    m.s2.assign((size_t)g->k * g->d, 0.0);
   }
-  fisher_from_moments(m, n, g, flags, dp_dlambda);
+  dev.upload_params(g);
+  dev.fisher(flags, dp_dlambda);
 }
 
 void gmm_fisher_spatial(int N, int K, int D, const float *Q, const float *sgmm, const float *ll,
@@ -1020,16 +1105,11 @@ void gmm_fisher_spatial(int N, int K, int D, const float *Q, const float *sgmm, 
   for (long i = 0; i < N; i++)
     for (long c = 0; c < D; c++) llt[i * D + c] = ll[c * N + i];
   GmmDev dev("gmm_fisher_spatial", N, D, K);
-  Moments m;
   if (N > 0) {
     dev.upload_v(llt.data());
     dev.upload_P(Q);
-    m = dev.moments();
-  } else {
-    m.s0.assign((size_t)K, 0.0);
-    m.s1.assign((size_t)K * D, 0.0);
-    m.s2.assign((size_t)K * D, 0.0);
   }
+  const Moments m = dev.moments();
   const float *mm = sgmm, *S = sgmm + D;
   float *d_mm = sdesc, *d_S = sdesc + (long)K * D;
   for (long c = 0; c < D; c++)

@@ -19,15 +19,20 @@
 //               the side blocks, so the accumulator holds
 //               v_j = ||c_j'||^2 - 2 x'.c_j' of every centroid j (x', c': the
 //               rows less their instance's mean).
-//   warps 2-9   epilogue.  Warps 2-5 (one TMEM lane quadrant each, a thread
-//               per point) find the smallest v and mark the band of centroids
-//               within 2 eps of it (eps: the rigorous error bound of the
-//               16-bit products, the k-NN certificate's bound with the
-//               instance's own centroid norms and errors); all eight warps
-//               then take sixteen points each (two lanes per point): FP32
-//               direct differences over the band, near ties settled by the
-//               sign of the distance difference or FP64, and the points that
-//               change centroid moved in the fixed-point sums (atomics).
+//   warps 2-5   band (one TMEM lane quadrant each, a thread per point): the
+//               smallest v and the band of centroids within 2 eps of it (eps:
+//               the rigorous error bound of the 16-bit products, the k-NN
+//               certificate's bound with the instance's own centroid norms and
+//               errors), one tile ahead of
+//   warps 6-21  decision, eight points each (four lanes per point): FP32 direct
+//               differences over the band, near ties settled by the sign of
+//               the distance difference or FP64, and the points that change
+//               centroid moved in the fixed-point sums (atomics).
+// Bound by latency in both: TMEM loads and votes in the band, rows gathered from
+// shared memory or L2 in the decision.  Hence warps of their own for each
+// (band lists double-buffered between them) and sixteen for the decision.  With
+// eight warps doing both in turn 100k points x 256 centroids, d = 128, took 73
+// us (38 now), 1M points of an hkm level of 32, d = 96, 133 to 480 (120 to 370).
 // Every wait is bounded (tc_ptx.cuh); on expiry *err is set, every role leaves
 // its loop, the copies and MMAs already issued are waited for, and TMEM is
 // freed.
@@ -42,14 +47,19 @@ namespace yg {
 namespace kmtc {
 using namespace ptx;
 
-constexpr int NT = 320;
-constexpr int BW = 9;  // band mask words per point (k <= 256: 8 used; odd: no bank conflicts)
+constexpr int NDEC = 16;              // decision warps
+constexpr int PPW = 128 / NDEC;       // points per decision warp
+constexpr int LPP = 32 / PPW;         // lanes per point
+constexpr int NT = (6 + NDEC) * 32;
+constexpr int PAIRS = 64;             // (point, member) pairs listed per decision warp
+// band mask words per point (odd: no bank conflicts)
+__host__ __device__ constexpr int band_words(int N) { return (N >> 5) | 1; }
 constexpr int A_BLK = 128 * 128;  // 128 rows x 64 16-bit columns
 constexpr int A_SIDE = 128 * 32;  // 128 rows x 16 16-bit columns
 
 struct Lay {
   int nkb, N, S, fuse, csm, xs;
-  size_t stage_bytes, x_off, ts_off, b_off, bside_off, cf_off, band_off, lst_off, acc_off, cnt_off,
+  size_t stage_bytes, x_off, ts_off, b_off, bside_off, cf_off, band_off, lst_off, pair_off, acc_off, cnt_off,
       bar_off, total;
 };
 
@@ -67,13 +77,14 @@ __host__ __device__ inline Lay make_lay(int nkb, int N, int S, int fuse, int k, 
   L.b_off = off;     off += (size_t)nkb * N * 128;  // N % 32 == 0: 1024-aligned blocks
   L.bside_off = off; off += (size_t)N * 32;
   L.cf_off = off;    off += csm ? (size_t)N * d * 4 : 0;  // FP32 centroid rows (d % 4 == 0)
-  L.band_off = off;  off += (size_t)2 * 128 * BW * 4;
+  L.band_off = off;  off += (size_t)2 * 128 * band_words(N) * 4;
   L.lst_off = off;   off += (size_t)256 * 4;  // the tile's moves: new and old centroids
+  L.pair_off = off;  off += (size_t)NDEC * PAIRS * 8;  // pairs, then their distances
   off = (off + 15) & ~(size_t)15;
   L.acc_off = off;   off += fuse ? (size_t)k * d * 8 : 0;
   L.cnt_off = off;   off += fuse ? (size_t)k * 4 : 0;
   off = (off + 15) & ~(size_t)15;
-  L.bar_off = off;   off += (size_t)(2 * S + 8) * 8 + 16;
+  L.bar_off = off;   off += (size_t)(2 * S + 12) * 8 + 16;
   L.total = off + 1024;  // alignment slack of the 1024-byte aligned base
   return L;
 }
@@ -143,13 +154,17 @@ __device__ __forceinline__ bool fixed_shift_ok(float x, int S) {
   return (ex >= 150 - S && ex != 0xff && ex != 0) || (__float_as_uint(x) << 1) == 0u;
 }
 
-// The exact decision for the sixteen points r0 .. r0 + 15 of a warp, two
-// lanes per point (lanes 2 p and 2 p + 1 for point p; h = lane & 1 takes the
-// float4 columns q = 2 i + h).  The lanes of point p start at i = p and wrap
-// around, so that any eight consecutive lanes (four points, both halves) read
-// eight different bank groups when the rows are a multiple of 128 bytes.
+// The exact decision for the PPW points r0 .. r0 + PPW - 1 of a warp, LPP
+// lanes per point (lanes LPP p + h for point p; h takes the float4 columns
+// q = LPP i + h).  The lanes of point p start at i = p and wrap around, so
+// that any eight consecutive lanes (two points of four) read eight different
+// bank groups when the rows are a multiple of 128 bytes.
 // Per band member the FP32 distance sum_c (x_c - c_c)^2 is summed in that
-// order (four partial sums, the two halves added last: deterministic); members come in increasing index order and
+// order (four partial sums, the lanes' added last: deterministic).  Where
+// a warp's longest band is well above its average one, its (point, member)
+// pairs are listed first and the lane groups take them in turn, not their own
+// point's only (100k points, k = 256: 44 -> 38 us; an hkm level with 3.8
+// members a point 360 -> 340).  Members come in increasing index order and
 // strict '<' keeps the lower index on equal values; a near tie of the best
 // two is settled by the sign of their distance difference when that clears
 // its rounding bound, by FP64 otherwise (lowest index on equal values).  Writes assign / dis and, for the fused sums, the
@@ -161,62 +176,99 @@ __device__ __forceinline__ bool fixed_shift_ok(float x, int S) {
 template <bool CSM>
 __device__ __forceinline__ void phase_b_decide(const Params &P, const unsigned *bm, int r0,
                                                int np, long p0, const float *X, const float *Ci,
-                                               int lane, int d, int k, float rho, int *toj) {
-  const int r = r0 + (lane >> 1), h = lane & 1;
+                                               int lane, int d, int k, float rho, int *toj,
+                                               int *pairs) {
+  const int p = lane / LPP, r = r0 + p, h = lane % LPP;
   const bool val = r < np;
   // the previous assignment, loaded first (its latency under the distances)
   const int oa = (P.delta && val && h == 0) ? P.assign[p0 + r] : -1;
   const int d4 = d >> 2;
-  const int nh = (d4 + 1 - h) >> 1;  // this half's float4 columns
+  const int nh = (d4 + LPP - 1 - h) / LPP;  // this lane's float4 columns
   // the band: a bit per centroid, words of 32
   const int nw = (k + 31) >> 5;
-  const unsigned *bw = bm + r * BW;
+  const unsigned *bw = bm + r * band_words(P.N);
   int nm = 0;
   for (int w = 0; w < nw; w++) nm += val ? __popc(bw[w]) : 0;
   unsigned mk = val ? bw[0] : 0u;
   int wi = 0;
-  const int mmax = (int)__reduce_max_sync(0xffffffffu, (unsigned)nm);
   const float4 *xr = reinterpret_cast<const float4 *>(X + (long)(val ? r : 0) * d);
-  const int i0 = (lane >> 1) % max(nh, 1);  // this lane's first column
+  const int i0 = p % max(nh, 1);  // this lane's first column
   float e1 = INFINITY, e2 = INFINITY, e3 = INFINITY;
   int j1 = -1, j2 = -1;
-  for (int m = 0; m < mmax; m++) {
-    int j = 0;
-    if (m < nm) {  // the next member (one is left)
-      while (mk == 0u) mk = bw[++wi];
-      j = wi * 32 + __ffs(mk) - 1;
-      mk &= mk - 1;
-    }
+  // this lane's part of ||x - c_j||^2
+  auto part = [&](const float4 *x, int j) {
+    const float4 *cr = reinterpret_cast<const float4 *>(Ci + (long)j * d);
     float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
-    if (m < nm) {
-      const float4 *cr = reinterpret_cast<const float4 *>(Ci + (long)j * d);
 #pragma unroll 4
-      for (int t = 0; t < nh; t++) {
-        int i = i0 + t;
-        if (i >= nh) i -= nh;
-        const int q = 2 * i + h;
-        const float4 xv = xr[q];
-        const float4 cv = CSM ? cr[q] : __ldg(cr + q);
-        float u = xv.x - cv.x;
-        s0 = fmaf(u, u, s0);
-        u = xv.y - cv.y;
-        s1 = fmaf(u, u, s1);
-        u = xv.z - cv.z;
-        s2 = fmaf(u, u, s2);
-        u = xv.w - cv.w;
-        s3 = fmaf(u, u, s3);
-      }
+    for (int t = 0; t < nh; t++) {
+      int i = i0 + t;
+      if (i >= nh) i -= nh;
+      const int q = LPP * i + h;
+      const float4 xv = x[q];
+      const float4 cv = CSM ? cr[q] : __ldg(cr + q);
+      float u = xv.x - cv.x;
+      s0 = fmaf(u, u, s0);
+      u = xv.y - cv.y;
+      s1 = fmaf(u, u, s1);
+      u = xv.z - cv.z;
+      s2 = fmaf(u, u, s2);
+      u = xv.w - cv.w;
+      s3 = fmaf(u, u, s3);
     }
-    float e = (s0 + s1) + (s2 + s3);
-    e += __shfl_xor_sync(0xffffffffu, e, 1);  // the other half (same sum in both lanes)
-    if (m < nm) {
-      if (e < e1) {
-        e3 = e2; e2 = e1; j2 = j1; e1 = e; j1 = j;
-      } else if (e < e2) {
-        e3 = e2; e2 = e; j2 = j;
-      } else if (e < e3) {
-        e3 = e;
+    return (s0 + s1) + (s2 + s3);
+  };
+  auto group_sum = [&](float e) {
+#pragma unroll
+    for (int o = 1; o < LPP; o <<= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
+    return e;  // (the same sum in all of the group's lanes)
+  };
+  auto take = [&](float e, int j) {
+    if (e < e1) {
+      e3 = e2; e2 = e1; j2 = j1; e1 = e; j1 = j;
+    } else if (e < e2) {
+      e3 = e2; e2 = e; j2 = j;
+    } else if (e < e3) {
+      e3 = e;
+    }
+  };
+  auto next = [&]() {  // the next member (one is left)
+    while (mk == 0u) mk = bw[++wi];
+    const int j = wi * 32 + __ffs(mk) - 1;
+    mk &= mk - 1;
+    return j;
+  };
+  int end = nm;  // this point's pairs end here
+#pragma unroll
+  for (int o = LPP; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, end, o);
+    if (lane >= o) end += y;
+  }
+  const int total = __shfl_sync(0xffffffffu, end, 31);
+  const int mmax = (int)__reduce_max_sync(0xffffffffu, (unsigned)nm);
+  // (staged centroid rows: a round saved pays the list from two on)
+  if (total <= PAIRS && mmax > (total + PPW - 1) / PPW + (CSM ? 1 : 0)) {
+    float *dist = reinterpret_cast<float *>(pairs + PAIRS);
+    if (h == 0)
+      for (int t = end - nm; t < end; t++) pairs[t] = p << 8 | next();
+    __syncwarp();
+    for (int t0 = 0; t0 < total; t0 += PPW) {
+      const int t = t0 + p;
+      float e = 0.f;
+      if (t < total) {
+        const int pr = pairs[t];
+        e = part(reinterpret_cast<const float4 *>(X + (long)(r0 + (pr >> 8)) * d), pr & 255);
       }
+      e = group_sum(e);
+      if (h == 0 && t < total) dist[t] = e;
+    }
+    __syncwarp();
+    for (int t = end - nm; t < end; t++) take(dist[t], pairs[t] & 255);
+    __syncwarp();  // the list is the next tile's
+  } else {
+    for (int m = 0; m < mmax; m++) {
+      const int j = m < nm ? next() : 0;
+      const float e = group_sum(m < nm ? part(xr, j) : 0.f);
+      if (m < nm) take(e, j);
     }
   }
   int oj = -1;
@@ -239,7 +291,7 @@ __device__ __forceinline__ void phase_b_decide(const Params &P, const unsigned *
       for (int t = 0; t < nh; t++) {
         int i = i0 + t;
         if (i >= nh) i -= nh;
-        const int q = 2 * i + h;
+        const int q = LPP * i + h;
         const float4 xv = xr[q];
         const float4 av = CSM ? ca[q] : __ldg(ca + q);
         const float4 bv = CSM ? cb[q] : __ldg(cb + q);
@@ -255,9 +307,12 @@ __device__ __forceinline__ void phase_b_decide(const Params &P, const unsigned *
         }
       }
     }
-    dl += __shfl_xor_sync(0xffffffffu, dl, 1);
-    sa += __shfl_xor_sync(0xffffffffu, sa, 1);
-    sb += __shfl_xor_sync(0xffffffffu, sb, 1);
+#pragma unroll
+    for (int o = 1; o < LPP; o <<= 1) {
+      dl += __shfl_xor_sync(0xffffffffu, dl, o);
+      sa += __shfl_xor_sync(0xffffffffu, sa, o);
+      sb += __shfl_xor_sync(0xffffffffu, sb, o);
+    }
     if (pair) {
       // per coordinate p = fl(a - b), s = fl(a + b), t = fl(p fl(s - 2x)):
       // |t - exact| <= u |p| (|a + b| + 3 |s - 2x|) to first order, and the
@@ -272,8 +327,8 @@ __device__ __forceinline__ void phase_b_decide(const Params &P, const unsigned *
     }
   }
   if (__any_sync(0xffffffffu, need64)) {
-    // near tie: FP64 over the members, sequential over coordinates, the two
-    // lanes of the point taking alternate members
+    // near tie: FP64 over the members, sequential over coordinates, the lanes
+    // of the point taking every LPP-th member
     double best = INFINITY;
     int bj = INT_MAX;
     if (need64) {
@@ -284,7 +339,7 @@ __device__ __forceinline__ void phase_b_decide(const Params &P, const unsigned *
         while (tk == 0u) tk = bw[++tw];
         const int j = tw * 32 + __ffs(tk) - 1;
         tk &= tk - 1;
-        if ((m & 1) != h) continue;
+        if (m % LPP != h) continue;
         const float *cr = Ci + (long)j * d;
         double sd = 0;
         for (int c = 0; c < d; c++) {
@@ -294,9 +349,12 @@ __device__ __forceinline__ void phase_b_decide(const Params &P, const unsigned *
         if (sd < best || (sd == best && j < bj)) { best = sd; bj = j; }
       }
     }
-    const double ob = __shfl_xor_sync(0xffffffffu, best, 1);
-    const int oj2 = __shfl_xor_sync(0xffffffffu, bj, 1);
-    if (ob < best || (ob == best && oj2 < bj)) { best = ob; bj = oj2; }
+#pragma unroll
+    for (int o = 1; o < LPP; o <<= 1) {
+      const double ob = __shfl_xor_sync(0xffffffffu, best, o);
+      const int oj2 = __shfl_xor_sync(0xffffffffu, bj, o);
+      if (ob < best || (ob == best && oj2 < bj)) { best = ob; bj = oj2; }
+    }
     if (need64) {
       if (bj != INT_MAX && best < 1e30) { oj = bj; od = (float)best; }
       else { oj = -1; od = 1e30f; }
@@ -315,7 +373,7 @@ __device__ __forceinline__ void phase_b_decide(const Params &P, const unsigned *
   }
 }
 
-// The fused sums of the warp's sixteen points (r0 .. r0 + 15): their moves
+// The fused sums of the warp's points (r0 .. r0 + PPW - 1): their moves
 // (joins toj[r], leaves toj[128 + r], written by the warp's own decision),
 // one after another, lanes over coordinates (lane + 32 i), as 64-bit integer
 // atomics into the sums (rows: k x d, in shared memory for an instance whose
@@ -326,10 +384,10 @@ template <int N32>
 __device__ __forceinline__ void phase_b_sums(unsigned long long *rows, int *cnts, const int *toj,
                                              int r0, int np, const float *X, int lane, int d,
                                              int sh) {
-  // lanes 0-15 hold the sixteen points' (join, leave); a moving point's row
-  // is read and converted once for both
-  const int r = r0 + (lane & 15);
-  const bool pv = lane < 16 && r < np;
+  // lanes 0 .. PPW - 1 hold the points' (join, leave); a moving point's row is
+  // read and converted once for both
+  const int r = r0 + (lane & (PPW - 1));
+  const bool pv = lane < PPW && r < np;
   const int oj = pv ? toj[r] : -1, oa = pv ? toj[128 + r] : -1;
   unsigned m = __ballot_sync(0xffffffffu, oj >= 0 || oa >= 0);
   while (m) {
@@ -379,15 +437,16 @@ __global__ void __launch_bounds__(NT, 1)
   uint8_t *Bs = base + lay.b_off;
   uint8_t *Bside = base + lay.bside_off;
   float *Cf = reinterpret_cast<float *>(base + lay.cf_off);
-  unsigned *band = reinterpret_cast<unsigned *>(base + lay.band_off);  // [2][128][BW]
+  unsigned *band = reinterpret_cast<unsigned *>(base + lay.band_off);  // [2][128][words]
   int *toj = reinterpret_cast<int *>(base + lay.lst_off);    // the tile's chosen centroids
   unsigned long long *sacc = reinterpret_cast<unsigned long long *>(base + lay.acc_off);
   int *scnt = reinterpret_cast<int *>(base + lay.cnt_off);
   uint64_t *bars = reinterpret_cast<uint64_t *>(base + lay.bar_off);
   uint64_t *full = bars, *empty = bars + S, *tfull = bars + 2 * S, *tempty = bars + 2 * S + 2;
   uint64_t *bfull = bars + 2 * S + 4, *bempty = bars + 2 * S + 5, *mdone = bars + 2 * S + 6;
-  uint64_t *cempty = bars + 2 * S + 7;  // the staged FP32 centroids read by the epilogue
-  uint32_t *tmem_holder = reinterpret_cast<uint32_t *>(bars + 2 * S + 8);
+  uint64_t *cempty = bars + 2 * S + 7;  // the staged FP32 centroids read by the decision
+  uint64_t *lfull = bars + 2 * S + 8, *lempty = bars + 2 * S + 10;  // the two band lists
+  uint32_t *tmem_holder = reinterpret_cast<uint32_t *>(bars + 2 * S + 12);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_holder + 1);
   const uint64_t wl = P.wait_ns ? (uint64_t)P.wait_ns : kWaitLimitNs;
   const uint32_t tcols = N * 2 <= 32 ? 32u : N * 2 <= 64 ? 64u : N * 2 <= 128 ? 128u
@@ -401,18 +460,20 @@ __global__ void __launch_bounds__(NT, 1)
   if (threadIdx.x == 0) {
     for (int s = 0; s < S; s++) {
       mbar_init(&full[s], 1);
-      // the MMAs' commit and the eight epilogue warps (the stage's side data,
-      // and its FP32 rows when staged)
-      mbar_init(&empty[s], 9);
+      // the MMAs' commit, the band warps (the stage's side data) and the
+      // decision warps (its FP32 rows when staged)
+      mbar_init(&empty[s], 1 + 4 + NDEC);
     }
     for (int a = 0; a < 2; a++) {
       mbar_init(&tfull[a], 1);
-      mbar_init(&tempty[a], 4);  // the four lane-quadrant warps of the epilogue
+      mbar_init(&tempty[a], 4);  // the four lane-quadrant warps of the band
+      mbar_init(&lfull[a], 4);
+      mbar_init(&lempty[a], NDEC);
     }
     mbar_init(bfull, 1);
     mbar_init(bempty, 1);
     mbar_init(mdone, 1);
-    mbar_init(cempty, 8);  // the eight epilogue warps
+    mbar_init(cempty, NDEC);
     *abort_flag = 0;
     fence_mbar_init();
   }
@@ -420,9 +481,9 @@ __global__ void __launch_bounds__(NT, 1)
     tmem_alloc(tmem_holder, tcols);
     tmem_relinquish();
   }
-  if (sfuse && warp >= 2) {
-    for (int i = threadIdx.x - 64; i < k * d; i += 256) sacc[i] = 0ull;
-    for (int i = threadIdx.x - 64; i < k; i += 256) scnt[i] = 0;
+  if (sfuse) {
+    for (int i = threadIdx.x; i < k * d; i += NT) sacc[i] = 0ull;
+    for (int i = threadIdx.x; i < k; i += NT) scnt[i] = 0;
   }
   tc_fence_before();
   __syncthreads();
@@ -530,36 +591,120 @@ __global__ void __launch_bounds__(NT, 1)
         mbar_wait_drain(mdone, 0);
       }
     }
-  } else {
-    // ---------------- epilogue
-    const int ew = warp - 2;       // 0..7
-    const int grp = warp & 3;      // TMEM lane quadrant (warps 2-5 read TMEM)
+  } else if (warp < 6) {
+    // ---------------- band
+    const int grp = warp & 3;      // TMEM lane quadrant
     const int row = grp * 32 + lane;
     const uint32_t lane_base = (uint32_t)(grp * 32) << 16;
     const float u24 = 5.9604645e-08f;
-    const float rho = (float)(d + 4) * u24;
     const float Kt = (float)(P.Kp + 16);
     const float un = (float)((d + 31) / 32 + 6) * u24;
-    int it = 0, cur = -1;
-    bool ok = true;
+    int it = 0, sn = 0;
+    uint32_t phn = 0;  // the ring's stage and phase, followed as the producer does
+    for (int w = w0; w < w1; w++) {
+      const KmTcUnit u = P.units[w];
+      if (!P.active[u.inst]) continue;
+      const int a = it & 1, s = sn;
+      const uint32_t uu = (uint32_t)(it >> 1), ph = phn;
+      if (++sn == S) { sn = 0; phn ^= 1; }
+      unsigned *bl = band + a * 128 * band_words(N);
+      const bool rv = row < u.np;
+      // this list read by the decision two tiles ago, the tile's copies landed
+      // (the MMAs waited for them too: here only for visibility), its products
+      bool ok = mbar_wait(&lempty[a], (uu & 1) ^ 1, abort_flag, wl) &&
+                mbar_wait(&full[s], ph, abort_flag, wl) &&
+                mbar_wait(&tfull[a], uu & 1, abort_flag, wl);
+      __syncwarp();
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) break;
+      tc_fence_after();
+      float eps = 0.f;
+      if (rv) {
+        const float2 nd = reinterpret_cast<const float2 *>(Stg + (size_t)s * lay.stage_bytes +
+                                                           lay.ts_off)[row];
+        const float qn = nd.x, dq = nd.y;
+        const float2 bd = P.ib[u.inst];  // the instance's centroids
+        const float B = bd.x, dB = bd.y;
+        const float dot = dq * (B + dB) + qn * dB;
+        const float accb = Kt * 2.f * u24 * (2.f * (qn + dq) * (B + dB) + 1.001f * B * B);
+        // the translation: x' = fl(x - mu), c' = fl(c - mu) are off by
+        // at most u ||x'||, u ||c'||, which moves ||x - c||^2 - ||x'||^2
+        // away from ||x' - c'||^2 - ||x'||^2 by at most 2 u (qn + B)^2 (1 + tiny)
+        const float tr = P.centered ? 2.01f * u24 * (qn + B) * (qn + B) : 0.f;
+        // (fp16 norm parts: their sum is within 2^-25 of ||c'||^2)
+        eps = (2.f * dot + u24 * B * B + accb + un * (qn * qn + B * B) + tr +
+               (P.f16 ? u24 : 0.f)) * 1.1f + 1e-30f;
+        // an infinite residual (a row fp16 cannot hold) times a zero one
+        // is NaN: such a point re-checks every centroid
+        if (!(eps <= 3.0e38f)) eps = INFINITY;
+      }
+      const uint32_t tc = tmem + lane_base + (uint32_t)(a * N);
+      uint32_t r[32], m;
+      float vmin = INFINITY;
+      for (int c0 = 0; c0 < N; c0 += 32) {
+        tmem_ld32_min(tc + (uint32_t)c0, r, m);
+        tmem_ld_wait(r, m);
+        if (c0 + 32 <= k) {
+          vmin = fminf(vmin, __uint_as_float(m));
+        } else {
+#pragma unroll
+          for (int i = 0; i < 31; i++)
+            if (c0 + i < k) vmin = fminf(vmin, __uint_as_float(r[i]));
+        }
+      }
+      const float lim = vmin + 2.f * eps;
+      // the members: a bit per centroid within 2 eps of the smallest; all
+      // of them without a usable bound, none for no point (or no finite
+      // distance)
+      const bool all = rv && eps == INFINITY, none = !rv || (!all && !(vmin < INFINITY));
+      for (int c0 = 0; c0 < N; c0 += 32) {
+        if (N > 32) {  // with one chunk r still holds it
+          tmem_ld32(tc + (uint32_t)c0, r);
+          tmem_ld_wait(r);
+        }
+        unsigned mk = 0u;
+#pragma unroll
+        for (int i = 0; i < 32; i++)
+          mk |= (all || __uint_as_float(r[i]) <= lim) ? 1u << i : 0u;
+        if (c0 + 32 > k) mk &= (1u << (k - c0)) - 1u;
+        bl[row * band_words(N) + (c0 >> 5)] = none ? 0u : mk;
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) {
+        mbar_arrive(&tempty[a]);
+        mbar_arrive(&lfull[a]);
+        mbar_arrive(&empty[s]);
+      }
+      it++;
+    }
+  } else {
+    // ---------------- decision
+    const int ew = warp - 6, dt = threadIdx.x - 192;
+    int *pairs = reinterpret_cast<int *>(base + lay.pair_off) + ew * 2 * PAIRS;
+    const float rho = (float)(d + 4) * 5.9604645e-08f;
+    // the shared sums of an instance to the global ones.  All decision warps
+    // come here for each of their instances, also after a wait that gave up
+    // (their loop has no early exit), so the barriers always complete.
     auto flush = [&](int inst) {
-      asm volatile("bar.sync 1, 256;" ::: "memory");
+      asm volatile("bar.sync 1, %0;" ::"n"(NDEC * 32) : "memory");
       const long g0 = (long)inst * k;
-      for (int i = threadIdx.x - 64; i < k * d; i += 256) {
+      for (int i = dt; i < k * d; i += NDEC * 32) {
         const unsigned long long x = sacc[i];
         if (x) atomicAdd((unsigned long long *)(P.acc + g0 * d + i), x);
         sacc[i] = 0ull;
       }
-      for (int i = threadIdx.x - 64; i < k; i += 256) {
+      for (int i = dt; i < k; i += NDEC * 32) {
         if (scnt[i]) atomicAdd(P.counts + g0 + i, scnt[i]);
         scnt[i] = 0;
       }
-      asm volatile("bar.sync 1, 256;" ::: "memory");
+      asm volatile("bar.sync 1, %0;" ::"n"(NDEC * 32) : "memory");
     };
-    int nbl = 0;  // centroid tiles seen (the staged FP32 rows' bfull phases)
-    int esn = 0;  // the ring's stage and phase, followed as the producer does
-    uint32_t ephn = 0;
-    for (int w = w0; w < w1 && ok; w++) {
+    int it = 0, cur = -1, nbl = 0;  // nbl: centroid tiles seen (the staged rows' bfull phases)
+    int sn = 0;
+    uint32_t phn = 0;
+    bool ok = true;
+    for (int w = w0; w < w1; w++) {
       const KmTcUnit u = P.units[w];
       if (!P.active[u.inst]) continue;
       if (u.inst != cur) {
@@ -569,120 +714,47 @@ __global__ void __launch_bounds__(NT, 1)
         if (P.csm) {
           // the new instance's rows have landed (the MMA warp waits on the same
           // phase of bfull before its first MMA of the instance)
-          ok = mbar_wait(bfull, (uint32_t)(nbl & 1), abort_flag, wl);
+          ok = ok && mbar_wait(bfull, (uint32_t)(nbl & 1), abort_flag, wl);
           __syncwarp();
           ok = __all_sync(0xffffffffu, ok);
         }
         nbl++;
         cur = u.inst;
       }
-      const int a = it & 1;
-      unsigned *bl = band + a * 128 * BW;
-      const int xs_s = esn;  // the stage this tile came in
-      const uint32_t xs_ph = ephn;
-      if (++esn == S) { esn = 0; ephn ^= 1; }
-      // the tile's copies have landed (the MMAs waited for them too: this
-      // wait only makes them visible here)
-      ok = ok && mbar_wait(&full[xs_s], xs_ph, abort_flag, wl);
+      const int a = it & 1, s = sn;
+      const uint32_t uu = (uint32_t)(it >> 1), ph = phn;
+      if (++sn == S) { sn = 0; phn ^= 1; }
+      it++;
+      ok = ok && mbar_wait(&full[s], ph, abort_flag, wl) &&
+           mbar_wait(&lfull[a], uu & 1, abort_flag, wl);
       __syncwarp();
       ok = __all_sync(0xffffffffu, ok);
-      const float2 *ts = reinterpret_cast<const float2 *>(Stg + (size_t)xs_s * lay.stage_bytes +
-                                                          lay.ts_off);
-      if (ew < 4) {
-        const uint32_t uu = (uint32_t)(it >> 1);
-        const bool rv = row < u.np;
-        ok = ok && mbar_wait(&tfull[a], uu & 1, abort_flag, wl);
-        __syncwarp();
-        ok = __all_sync(0xffffffffu, ok);
-        if (ok) {
-          tc_fence_after();
-          float eps = 0.f;
-          if (rv) {
-            const float2 nd = ts[row];
-            const float qn = nd.x, dq = nd.y;
-            const float2 bd = P.ib[u.inst];  // the instance's centroids
-            const float B = bd.x, dB = bd.y;
-            const float dot = dq * (B + dB) + qn * dB;
-            const float accb = Kt * 2.f * u24 * (2.f * (qn + dq) * (B + dB) + 1.001f * B * B);
-            // the translation: x' = fl(x - mu), c' = fl(c - mu) are off by
-            // at most u ||x'||, u ||c'||, which moves ||x - c||^2 - ||x'||^2
-            // away from ||x' - c'||^2 - ||x'||^2 by at most 2 u (qn + B)^2 (1 + tiny)
-            const float tr = P.centered ? 2.01f * u24 * (qn + B) * (qn + B) : 0.f;
-            // (fp16 norm parts: their sum is within 2^-25 of ||c'||^2)
-            eps = (2.f * dot + u24 * B * B + accb + un * (qn * qn + B * B) + tr +
-                   (P.f16 ? u24 : 0.f)) * 1.1f + 1e-30f;
-            // an infinite residual (a row fp16 cannot hold) times a zero one
-            // is NaN: such a point re-checks every centroid
-            if (!(eps <= 3.0e38f)) eps = INFINITY;
-          }
-          const uint32_t tc = tmem + lane_base + (uint32_t)(a * N);
-          uint32_t r[32];
-          float vmin = INFINITY;
-          for (int c0 = 0; c0 < N; c0 += 32) {
-            tmem_ld32(tc + (uint32_t)c0, r);
-            tmem_ld_wait(r);
-            // a tree of minima (fminf: any order gives the same minimum)
-            float m16[16];
-#pragma unroll
-            for (int i = 0; i < 16; i++)
-              m16[i] = fminf(c0 + i < k ? __uint_as_float(r[i]) : INFINITY,
-                             c0 + i + 16 < k ? __uint_as_float(r[i + 16]) : INFINITY);
-#pragma unroll
-            for (int w = 8; w > 0; w >>= 1)
-#pragma unroll
-              for (int i = 0; i < w; i++) m16[i] = fminf(m16[i], m16[i + w]);
-            vmin = fminf(vmin, m16[0]);
-          }
-          const float lim = vmin + 2.f * eps;
-          // the members: a bit per centroid within 2 eps of the smallest; all
-          // of them without a usable bound, none for no point (or no finite
-          // distance)
-          const bool all = rv && eps == INFINITY, none = !rv || (!all && !(vmin < INFINITY));
-          for (int c0 = 0; c0 < N; c0 += 32) {
-            if (N > 32) {  // with one chunk r still holds it
-              tmem_ld32(tc + (uint32_t)c0, r);
-              tmem_ld_wait(r);
-            }
-            unsigned mk = 0u;
-#pragma unroll
-            for (int i = 0; i < 32; i++)
-              mk |= (c0 + i < k && (all || __uint_as_float(r[i]) <= lim)) ? 1u << i : 0u;
-            bl[row * BW + (c0 >> 5)] = none ? 0u : mk;
-          }
-          tc_fence_before();
-        }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&tempty[a]);
-      }
-      // the band lists of this tile are written (and the other buffer's were
-      // read by every warp before it): one barrier per tile, all warps agree
-      ok = bar_red_and_256(ok);
-      if (!ok) break;
-      // phase B: the exact decision, sixteen points per warp, then the sums
+      if (!ok) continue;
+      const unsigned *bl = band + a * 128 * band_words(N);
       const int sh = fuse ? P.shift[u.inst] : 0;
       const float *Ci = P.csm ? Cf : P.C + (long)u.inst * k * d;
-      const float *Xs = reinterpret_cast<const float *>(Stg + (size_t)xs_s * lay.stage_bytes +
+      const float *Xs = reinterpret_cast<const float *>(Stg + (size_t)s * lay.stage_bytes +
                                                         lay.x_off);
       const float *X = P.xs ? Xs : P.v + u.p0 * d;
       if (P.csm)
-        phase_b_decide<true>(P, bl, ew * 16, u.np, u.p0, X, Ci, lane, d, k, rho,
-                             fuse ? toj : nullptr);
+        phase_b_decide<true>(P, bl, ew * PPW, u.np, u.p0, X, Ci, lane, d, k, rho,
+                             fuse ? toj : nullptr, pairs);
       else
-        phase_b_decide<false>(P, bl, ew * 16, u.np, u.p0, X, Ci, lane, d, k, rho,
-                              fuse ? toj : nullptr);
+        phase_b_decide<false>(P, bl, ew * PPW, u.np, u.p0, X, Ci, lane, d, k, rho,
+                              fuse ? toj : nullptr, pairs);
+      __syncwarp();  // the warp's own moves are in toj, its band read
+      if (lane == 0) mbar_arrive(&lempty[a]);
       if (fuse) {
-        __syncwarp();  // the warp's own moves are in toj
         if (sfuse)
-          phase_b_sums<ND>(sacc, scnt, toj, ew * 16, u.np, X, lane, d, sh);
+          phase_b_sums<ND>(sacc, scnt, toj, ew * PPW, u.np, X, lane, d, sh);
         else
           phase_b_sums<ND>(reinterpret_cast<unsigned long long *>(P.acc) + (long)u.inst * k * d,
-                           P.counts + (long)u.inst * k, toj, ew * 16, u.np, X, lane, d, sh);
+                           P.counts + (long)u.inst * k, toj, ew * PPW, u.np, X, lane, d, sh);
+        __syncwarp();
       }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&empty[xs_s]);  // this warp is done with the tile's stage
-      it++;
+      if (lane == 0) mbar_arrive(&empty[s]);  // this warp is done with the tile's stage
     }
-    if (sfuse && ok && cur >= 0) flush(cur);
+    if (sfuse && cur >= 0) flush(cur);
   }
 
   tc_fence_before();

@@ -19,6 +19,11 @@ __device__ __forceinline__ bool lex_less(unsigned long long ka, int ia,
   return ka < kb || (ka == kb && (unsigned)ia < (unsigned)ib);
 }
 
+__device__ __forceinline__ double ord2d(unsigned long long k) {
+  const unsigned long long u = (k & 0x8000000000000000ull) ? (k & 0x7fffffffffffffffull) : ~k;
+  return __longlong_as_double((long long)u);
+}
+
 // ascending bitonic sort of n (power of two) (key, id) pairs in shared memory
 // Ascending bitonic sort of n (a power of two) keys with ids, by the whole
 // block.  In a stage of stride s <= 32, thread i handles pairs inside elements
@@ -112,13 +117,149 @@ __device__ __forceinline__ float warp_sample_rank(int nq, int nchunk, int C, int
   return v;
 }
 
+// The need-th smallest (from 1) of a block's keys, RK per thread (0xffffffff where
+// valid has no bit), by counting digits of 8 bits below the keys' common range:
+// distances of one query share their leading bits, so two or three rounds of
+// mostly distinct bins do.  A few hundred keys: a fifth of a bitonic sort's time.
+constexpr int RK = 4;
+struct KthScratch {
+  int hist[256];
+  unsigned mn[RT / 32], mx[RT / 32];
+  int wsum[RT / 32];
+  unsigned lo;
+  int need;
+};
+__device__ unsigned block_kth(const unsigned (&key)[RK], unsigned valid, int need, KthScratch &S) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  unsigned mn = 0xffffffffu, mx = 0u;
+#pragma unroll
+  for (int r = 0; r < RK; r++)
+    if (valid >> r & 1u) {
+      mn = min(mn, key[r]);
+      mx = max(mx, key[r]);
+    }
+  mn = __reduce_min_sync(0xffffffffu, mn);
+  mx = __reduce_max_sync(0xffffffffu, mx);
+  __syncthreads();  // (the scratch may still be read from an earlier call)
+  if (lane == 0) {
+    S.mn[warp] = mn;
+    S.mx[warp] = mx;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int w = 0; w < RT / 32; w++) {
+    mn = min(mn, S.mn[w]);
+    mx = max(mx, S.mx[w]);
+  }
+  unsigned lo = mn;
+  int width = 32 - __clz(mx - mn);  // the answer is in [lo, lo + 2^width)
+  while (width > 0) {
+    const int shift = max(0, width - 8), bins = 1 << (width - shift);
+    S.hist[tid] = 0;
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < RK; r++) {
+      const unsigned b = (key[r] - lo) >> shift;
+      if ((valid >> r & 1u) && key[r] >= lo && b < (unsigned)bins) atomicAdd(&S.hist[b], 1);
+    }
+    __syncthreads();
+    const int h = S.hist[tid];
+    int x = h;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
+    }
+    if (lane == 31) S.wsum[warp] = x;
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < RT / 32; w++)
+      if (w < warp) x += S.wsum[w];
+    if (x - h < need && need <= x) {
+      S.lo = lo + ((unsigned)tid << shift);
+      S.need = need - (x - h);
+    }
+    __syncthreads();
+    lo = S.lo;
+    need = S.need;
+    width = shift;
+  }
+  return lo;
+}
+
+// FP32 distance of the query row to base row j by LPR lanes (sl: this one's
+// index; LPR = 8 with rows of whole aligned float4, else 32): 32 partial sums
+// over the coordinates c = 0 .. 31 (mod 32) and one tree over them, in the same
+// order for both, so the result does not depend on LPR.
+template <int LPR>
+__device__ __forceinline__ float lanes_dist32(const float *qv, const float *brow, int d,
+                                              int metric, int sl, unsigned gm) {
+  if constexpr (LPR == 32) {
+    return warp_dist32(qv, brow, d, metric);
+  } else {
+    float s[4] = {0.f, 0.f, 0.f, 0.f};
+    const bool L2 = metric == METRIC_L2;
+#pragma unroll 4
+    for (int c = 4 * sl; c < d; c += 32) {
+      const float4 b = __ldg(reinterpret_cast<const float4 *>(brow + c));
+      const float4 q = *reinterpret_cast<const float4 *>(qv + c);
+      const float bb[4] = {b.x, b.y, b.z, b.w}, qq[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+      for (int t = 0; t < 4; t++) {
+        const float u = qq[t] - bb[t];
+        s[t] = L2 ? fmaf(u, u, s[t]) : fmaf(qq[t], bb[t], s[t]);
+      }
+    }
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1)
+#pragma unroll
+      for (int t = 0; t < 4; t++) s[t] += __shfl_xor_sync(gm, s[t], o);
+    return (s[0] + s[2]) + (s[1] + s[3]);
+  }
+}
+
+// The same distance in pairs of floats (exact differences and products, two-sum
+// additions): within (d + 16) 2^-45 of its value (L2; of |q||b| for the inner
+// product).  This GPU's FP64 pipe runs at 1/64 of the FP32 rate; this takes about
+// 20 FP32 operations a coordinate.  The result is lane sl = 0's.
+template <int LPR>
+__device__ __forceinline__ double lanes_dist_pair(const float *qv, const float *brow, int d,
+                                                  int metric, int sl, unsigned gm) {
+  float hi = 0.f, lo = 0.f;
+  auto two_add = [&](float y, float ye) {
+    const float t = __fadd_rn(hi, y), z = __fsub_rn(t, hi);
+    const float e = __fadd_rn(__fsub_rn(hi, __fsub_rn(t, z)), __fsub_rn(y, z));
+    lo = __fadd_rn(lo, __fadd_rn(e, ye));
+    hi = t;
+  };
+  for (int c = sl; c < d; c += LPR) {
+    const float q = qv[c], b = __ldg(brow + c);
+    if (metric == METRIC_L2) {
+      const float t = __fsub_rn(q, b), z = __fsub_rn(t, q);
+      const float te = __fsub_rn(__fsub_rn(q, __fsub_rn(t, z)), __fadd_rn(b, z));
+      const float p = __fmul_rn(t, t);
+      two_add(p, __fmaf_rn(__fadd_rn(t, t), te, __fmaf_rn(t, t, -p)));
+    } else {
+      const float p = __fmul_rn(q, b);
+      two_add(p, __fmaf_rn(q, b, -p));
+    }
+  }
+#pragma unroll
+  for (int o = LPR / 2; o > 0; o >>= 1) {
+    const float h2 = __shfl_xor_sync(gm, hi, o), l2 = __shfl_xor_sync(gm, lo, o);
+    two_add(h2, l2);
+  }
+  return (double)hi + (double)lo;
+}
+
 __global__ void __launch_bounds__(RT) rerank_kernel(RerankArgs a, int Mp_alloc) {
   extern __shared__ __align__(16) unsigned char sm_raw[];
   unsigned long long *K = reinterpret_cast<unsigned long long *>(sm_raw);
   int *I = reinterpret_cast<int *>(K + Mp_alloc);
   float *E = reinterpret_cast<float *>(I + Mp_alloc);
   float *qv = E + Mp_alloc;  // the query row, d floats
-  __shared__ int sM, sfail, snband, sneed64;
+  __shared__ int sM, sfail, snband, sneed64, scount;
+  __shared__ KthScratch skth;
   __shared__ unsigned long long sT;  // TOPC boundary key (lexicographic (v, id))
 
   const int q = blockIdx.x;
@@ -227,10 +368,52 @@ __global__ void __launch_bounds__(RT) rerank_kernel(RerankArgs a, int Mp_alloc) 
   float kth_hi = INFINITY;  // upper bound of the k-th exact distance, when found
   if (sfail || M < k || M > Mp_alloc) goto failed;
   {
-    const int Mp = next_pow2(M);
-    for (int i = M + tid; i < Mp; i += RT) { K[i] = ~0ull; I[i] = 0x7fffffff; }
-    __syncthreads();
-    bitonic_sort(K, I, Mp);
+    // Up to RK candidates per thread stay in registers: the k-th approximate value
+    // is counted out, and only what can be an answer is sorted.  More than that
+    // (rare) are sorted as they are.
+    const bool few = M <= RK * RT;
+    unsigned ckey[RK], cvalid = 0;
+    int cid[RK];
+    unsigned akey;
+    // the elements whose bit of sel is set to the front of K and I, in any
+    // order; returns their number
+    auto compact = [&](unsigned sel) {
+      __syncthreads();
+      if (tid == 0) scount = 0;
+      __syncthreads();
+#pragma unroll
+      for (int r = 0; r < RK; r++)
+        if (sel >> r & 1u) {
+          const int pos = atomicAdd(&scount, 1);
+          K[pos] = ckey[r];
+          I[pos] = cid[r];
+        }
+      __syncthreads();
+      return scount;
+    };
+    auto sort_n = [&](int n) {
+      const int np2 = next_pow2(n);
+      for (int i = n + tid; i < np2; i += RT) { K[i] = ~0ull; I[i] = 0x7fffffff; }
+      __syncthreads();
+      bitonic_sort(K, I, np2);
+    };
+    if (few) {
+#pragma unroll
+      for (int r = 0; r < RK; r++) {
+        const int i = tid + r * RT;
+        ckey[r] = 0xffffffffu;
+        cid[r] = 0x7fffffff;
+        if (i < M) {
+          ckey[r] = (unsigned)K[i];
+          cid[r] = I[i];
+          cvalid |= 1u << r;
+        }
+      }
+      akey = block_kth(ckey, cvalid, k, skth);
+    } else {
+      sort_n(M);
+      akey = (unsigned)K[k - 1];
+    }
     if (a.n_cand && tid == 0) atomicAdd(a.n_cand, (unsigned long long)M);
 
     // boundary of the non-candidates, dist space
@@ -246,6 +429,13 @@ __global__ void __launch_bounds__(RT) rerank_kernel(RerankArgs a, int Mp_alloc) 
     }
 
     if (ex) {
+      if (few) {
+        unsigned sel = 0;
+#pragma unroll
+        for (int r = 0; r < RK; r++)
+          if ((cvalid >> r & 1u) && ckey[r] <= akey) sel |= 1u << r;
+        sort_n(compact(sel));
+      }
       // approx values are exact: the sorted prefix is the answer.  TOPC:
       // certified when (a_k, id_k) <= the lexicographic boundary.
       if (s.mode == SCAN_TOPC && sT != ~0ull) {
@@ -265,34 +455,45 @@ __global__ void __launch_bounds__(RT) rerank_kernel(RerankArgs a, int Mp_alloc) 
     }
 
     // ---- 2. band of candidates that can still be in the top k
-    const float ak = ord2f((unsigned)K[k - 1]);
+    const float ak = ord2f(akey);
     const double slack = 4e-7 * fabs((double)ak) + 1e-30;
     const double lim = (double)ak + 2.0 * (double)eps + slack;
-    if (tid == 0) snband = 0;
-    __syncthreads();
-    {
+    int nband;  // >= k: the candidates up to a_k are inside
+    if (few) {
+      unsigned sel = 0;
+#pragma unroll
+      for (int r = 0; r < RK; r++)
+        if ((cvalid >> r & 1u) && (double)ord2f(ckey[r]) <= lim) sel |= 1u << r;
+      nband = compact(sel);
+    } else {
+      if (tid == 0) snband = 0;
+      __syncthreads();
       int local = 0;
       for (int i = tid; i < M; i += RT)
         if ((double)ord2f((unsigned)K[i]) <= lim) local++;
       atomicAdd(&snband, local);
+      __syncthreads();
+      nband = snband;
     }
-    __syncthreads();
-    const int nband = snband;  // >= k: the sorted prefix up to a_k is inside
 
-    // ---- 3. FP32 re-rank of the band
-    const int warp = tid >> 5, nw = RT / 32;
-    for (int i = warp; i < nband; i += nw) {
-      const float e = warp_dist32(qv, B + (long)I[i] * ldb, d, a.metric);
-      if ((tid & 31) == 0) E[i] = e;
+    // ---- 3. FP32 re-rank of the band: 8 lanes per row where its float4 are
+    // aligned (four rows per warp in flight), else a warp per row
+    const bool vec = (d & 3) == 0 && (ldb & 3) == 0 && ((uintptr_t)B & 15) == 0;
+    const int sl8 = tid & 7;
+    const unsigned gm8 = 0xffu << (tid & 24);
+    if (vec) {
+      for (int i = tid >> 3; i < nband; i += RT / 8) {
+        const float e = lanes_dist32<8>(qv, B + (long)I[i] * ldb, d, a.metric, sl8, gm8);
+        if (sl8 == 0) E[i] = e;
+      }
+    } else {
+      for (int i = tid >> 5; i < nband; i += RT / 32) {
+        const float e =
+            lanes_dist32<32>(qv, B + (long)I[i] * ldb, d, a.metric, tid & 31, 0xffffffffu);
+        if ((tid & 31) == 0) E[i] = e;
+      }
     }
     __syncthreads();
-    const int nbp = next_pow2(nband);
-    for (int i = tid; i < nbp; i += RT) {
-      if (i < nband) K[i] = f2ord(E[i]);
-      else { K[i] = ~0ull; I[i] = 0x7fffffff; }
-    }
-    __syncthreads();
-    bitonic_sort(K, I, nbp);
 
     // error model of the FP32 re-rank
     const float rho = (float)(d + 4) * kU;
@@ -301,8 +502,36 @@ __global__ void __launch_bounds__(RT) rerank_kernel(RerankArgs a, int Mp_alloc) 
       const float B = __uint_as_float(bst->max_norm_bits);
       eta = (float)(d + 4) * kU * (float)sqrt(fmax(a.qn64 ? a.qn64[q] : 0.0, 0.0)) * B;
     }
-    // near ties anywhere up to position k -> FP64 for the whole band
-    const int lastpair = imin(k, nband - 1);
+    // the k + 1 smallest, and what lies within their error bounds of the last
+    // of them (a row further out cannot be among the k nearest), sorted
+    int n2 = nband;
+    if (few && nband > k + 1) {
+      cvalid = 0;
+#pragma unroll
+      for (int r = 0; r < RK; r++) {
+        const int i = tid + r * RT;
+        if (i < nband) {
+          ckey[r] = f2ord(E[i]);
+          cid[r] = I[i];
+          cvalid |= 1u << r;
+        }
+      }
+      const float t = ord2f(block_kth(ckey, cvalid, k + 1, skth));
+      const float lim2 = t + 6.f * (rho * fabsf(t) + eta);
+      unsigned sel = cvalid;
+      if (lim2 < INFINITY) {
+#pragma unroll
+        for (int r = 0; r < RK; r++)
+          if (!(ord2f(ckey[r]) <= lim2)) sel &= ~(1u << r);
+      }
+      n2 = compact(sel);
+    } else {
+      for (int i = tid; i < nband; i += RT) K[i] = f2ord(E[i]);
+    }
+    sort_n(n2);
+    // near ties anywhere up to position k: all of them again in pairs of floats,
+    // and in FP64 (the order that decides) where those still nearly tie
+    const int lastpair = imin(k, n2 - 1);
     for (int i = tid; i < lastpair; i += RT) {
       const float e0 = ord2f((unsigned)K[i]), e1 = ord2f((unsigned)K[i + 1]);
       const float tol = rho * (fabsf(e0) + fabsf(e1)) + 2.f * eta;
@@ -311,17 +540,43 @@ __global__ void __launch_bounds__(RT) rerank_kernel(RerankArgs a, int Mp_alloc) 
     __syncthreads();
     double ek_hi;
     if (sneed64) {
-      // one thread per candidate, sequential FP64 sum
-      for (int i = tid; i < nband; i += RT) {
-        const double e = dist64_seq(qv, B + (long)I[i] * ldb, d, a.metric);
-        K[i] = d2ord(e);
-      }
+      const bool finite = (unsigned)K[n2 - 1] <= f2ord(FLT_MAX) && (unsigned)K[0] >= f2ord(-FLT_MAX);
       __syncthreads();
-      bitonic_sort(K, I, nbp);
+      if (finite) {
+        if (vec) {
+          for (int i = tid >> 3; i < n2; i += RT / 8) {
+            const double e = lanes_dist_pair<8>(qv, B + (long)I[i] * ldb, d, a.metric, sl8, gm8);
+            if (sl8 == 0) K[i] = d2ord(e);
+          }
+        } else {
+          for (int i = tid >> 5; i < n2; i += RT / 32) {
+            const double e = lanes_dist_pair<32>(qv, B + (long)I[i] * ldb, d, a.metric, tid & 31,
+                                                 0xffffffffu);
+            if ((tid & 31) == 0) K[i] = d2ord(e);
+          }
+        }
+        if (tid == 0) sneed64 = 0;
+        sort_n(n2);
+        __syncthreads();
+        for (int i = tid; i < lastpair; i += RT) {
+          const double e0 = ord2d(K[i]), e1 = ord2d(K[i + 1]);
+          const double tol = (double)(d + 16) * 2.9e-14 * (fabs(e0) + fabs(e1)) +
+                             (double)eta * 1e-6 + 1e-36;
+          if (!(e1 - e0 > tol)) sneed64 = 1;
+        }
+        __syncthreads();
+      }
+      if (sneed64) {
+        // one thread per candidate, sequential FP64 sum
+        for (int i = tid; i < n2; i += RT)
+          K[i] = d2ord(dist64_seq(qv, B + (long)I[i] * ldb, d, a.metric));
+        sort_n(n2);
+      }
       const unsigned long long kk = K[k - 1];
       const unsigned long long u = (kk & 0x8000000000000000ull) ? (kk & 0x7fffffffffffffffull) : ~kk;
       const double ek = __longlong_as_double((long long)u);
-      ek_hi = ek + 1e-12 * fabs(ek);
+      // (pairs of floats: within (d + 16) 2.9e-14 of the value and 1e-6 eta)
+      ek_hi = ek + (1e-12 + (double)(d + 16) * 2.9e-14) * fabs(ek) + 1e-6 * (double)eta + 1e-36;
       for (int r = tid; r < k; r += RT) {
         const unsigned long long kr = K[r];
         const unsigned long long ur = (kr & 0x8000000000000000ull) ? (kr & 0x7fffffffffffffffull) : ~kr;
@@ -458,11 +713,6 @@ __device__ __forceinline__ void group_pair_diff(const float *qv, const float *ra
   dl = t0;
   st = t1;
   sps = t2;
-}
-
-__device__ __forceinline__ double ord2d(unsigned long long k) {
-  const unsigned long long u = (k & 0x8000000000000000ull) ? (k & 0x7fffffffffffffffull) : ~k;
-  return __longlong_as_double((long long)u);
 }
 
 // One query q by its group of G lanes; returns the number of candidates the

@@ -218,7 +218,17 @@ int wave_prepare(const yael_gpu_knn_pair *pairs, const Wave &w, int d, int k, in
   YG_LAUNCH_CHECK();
   YG_CUDA(cudaMemsetAsync(S.status, 0, sizeof(GroupStatus), sp));
   const float qscale = L2 ? -2.f : 1.f;
-  for (int i = 0; i < np; i++) {
+  YG_CHECK(gs_get(ws, o + GS_PAIRS, np, &S.dpairs));
+  const bool grouped_prep = prep_group_ok(hp.data(), np, d, Kp);
+  if (grouped_prep) {
+    // (the table as far as it is known; the whole of it follows below)
+    YG_CUDA(cudaMemcpyAsync(S.dpairs, hp.data(), sizeof(GroupPair) * np, cudaMemcpyHostToDevice,
+                            sp));
+    YG_CHECK(prep_group(S.dpairs, np, brows, nq_all, d, Kp, qscale, S.bpack,
+                        L2 ? S.bnorm : nullptr, S.stats,
+                        S.qpack, L2 ? S.qnorm : nullptr, S.qn64, S.qflag, S.qres, S.qpair, sp));
+  }
+  for (int i = 0; i < np && !grouped_prep; i++) {
     const GroupPair &g = hp[i];
     YG_CHECK(prep_rows(g.b, d, g.nb, d, 1.f, nullptr, nullptr, nullptr, nullptr,
                        S.bpack + (size_t)g.boff * Kp, Kp,
@@ -296,7 +306,6 @@ int wave_prepare(const yael_gpu_knn_pair *pairs, const Wave &w, int d, int k, in
   }
   S.n_mu = mu.size();
   S.n_su = su.size();
-  YG_CHECK(gs_get(ws, o + GS_PAIRS, np, &S.dpairs));
   YG_CHECK(gs_get(ws, o + GS_MUNITS, mu.size(), &S.dmu));
   if (!su.empty()) {
     YG_CHECK(gs_get(ws, o + GS_SUNITS, su.size(), &S.dsu));

@@ -64,6 +64,17 @@ int prep_rows_split(const float *x, long ld, int n, int d, float scale, int layo
                     float *resid, __nv_bfloat16 *packed, int Kp1, __nv_bfloat16 *normpart,
                     int normpart_mode, SetStats *stats, cudaStream_t st);
 
+// The packing of many pairs of a grouped pass in two launches: every base (and
+// its statistics) and every query (and its pair's index).  prep_group_ok
+// tells whether all rows have the form it reads (whole aligned float4, at most
+// 128 packed columns, bases at multiples of 256 rows); pairs: the device table.
+struct GroupPair;
+bool prep_group_ok(const GroupPair *host_pairs, int np, int d, int Kp);
+int prep_group(const GroupPair *pairs, int np, long brows, int nq, int d, int Kp, float qscale,
+               __nv_bfloat16 *bpack, __nv_bfloat16 *bnorm, SetStats *stats, __nv_bfloat16 *qpack,
+               __nv_bfloat16 *qnorm, double *qn64, unsigned char *qflag, float *qres, int *qpair,
+               cudaStream_t st);
+
 int stats_reset(SetStats *stats, cudaStream_t st);
 
 }  // namespace yg

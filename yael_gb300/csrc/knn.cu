@@ -501,9 +501,16 @@ int knn_batch(KnnJob &job, Ctx *ctx, cudaStream_t st, Small *dsmall, BaseOps *bo
       sel.cap = L.cap;
       YG_CHECK(band_thresholds(nq, job.metric, job.band_kth, qn64, eps, thr, st));
     } else if (prior) {
-      // every row whose exact distance can be <= the known bound
-      sel.cap = prior_cap(sel.nchunk);
-      sel.queue = nb >= 8192;  // a few rows in the band of the bound
+      // every row whose exact distance can be <= the known bound; the thresholds
+      // run on from there (fewer candidates, so fewer regions that overflow:
+      // 2M x 16,384, second iteration: 28,720 points rejected -> none, re-rank
+      // 1.53 -> 0.98 ms)
+      if (sel.nchunk <= 4) {
+        sel.run_eps = eps;
+        sel.cap = running_cap(sel.nchunk);
+      } else {
+        sel.cap = prior_cap(sel.nchunk);
+      }
       YG_CHECK(band_thresholds(nq, job.metric, job.prior_kth, qn64, eps, thr, st));
     } else if (up ? sns < 4 * c : !plan.usable(nb)) {
       // The sample is too short for a threshold: every base row is a candidate,

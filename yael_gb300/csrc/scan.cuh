@@ -72,7 +72,9 @@ struct ScanSel {
   float *topv = nullptr;
   int *topi = nullptr;
   const float *thr = nullptr;
-  const float *run_eps = nullptr;  // THRESH: eps per query, thresholds run (thr unused)
+  // THRESH: eps per query, thresholds run; they start from thr where it is given
+  // (tc_scan)
+  const float *run_eps = nullptr;
   int *cnt = nullptr;
   float *candv = nullptr;
   int *candi = nullptr;

@@ -1111,10 +1111,11 @@ __device__ __forceinline__ unsigned rerank_small_k1(const RerankArgs &a, int q) 
       // settled; the few it may reject at the edge go to the band pass.
       if (thresh) {
         // every non-candidate has approx > thr, so exact > thr + ||q||^2 - eps
-        // (a running threshold ends at or above the least value plus its slack)
-        const float t = s.run_eps ? __fadd_rd(ord2f(__reduce_min_sync(gm, f2ord(vraw))),
-                                              run_slack(eps))
-                                  : s.thr[q];
+        // (a running threshold ends at or above the least value plus its slack,
+        // or the threshold it started from)
+        float t = s.thr ? s.thr[q] : INFINITY;
+        if (s.run_eps)
+          t = fminf(t, __fadd_rd(ord2f(__reduce_min_sync(gm, f2ord(vraw))), run_slack(eps)));
         float blo = t, babs = fabsf(t);
         if (L2) {
           const double bd = (double)t + qn;
@@ -1211,31 +1212,34 @@ __global__ void eps_kernel(int nq, int d, int prec, int metric, const double *qn
   const bool ex = qflag[q] && bs->all_exact;
   qexact[q] = ex;
   if (ex) { eps[q] = 0.f; return; }
-  const double u = 5.9604644775390625e-08;  // 2^-24
+  // In FP32: every term is non-negative, so some twenty roundings lose at most
+  // 2e-6 of the sum (terms that underflow are far below its 1e-30), which the
+  // last factor gives back.  (In FP64, at 1/64 of the rate, 2M queries took 87 us.)
+  const float u = kU;  // 2^-24
   // norms are FP32 sums: relative error <= (d/32 + 6) u, on both sides
-  const double un = ((d + 31) / 32 + 6) * u;
-  const double qn = sqrt(fmax(qn64[q], 0.0)) * (1 + 1e-5);
-  const double B = (double)__uint_as_float(bs->max_norm_bits);
-  double e;
+  const float un = (float)((d + 31) / 32 + 6) * u;
+  const float qn = sqrtf(fmaxf((float)qn64[q], 0.f)) * (1.f + 1.1e-5f);
+  const float B = __uint_as_float(bs->max_norm_bits);
+  float e;
   if (prec == PREC_FP32) {
-    const double g = (d + 2) * u * 1.01;
-    e = metric == METRIC_L2 ? 2 * g * qn * B + u * (B * B + 2 * qn * B) + u * B * B
+    const float g = (float)(d + 2) * u * 1.01f;
+    e = metric == METRIC_L2 ? 2.f * g * qn * B + u * (B * B + 2.f * qn * B) + u * B * B
                             : g * qn * B;
   } else {
-    const double dq = qres ? (double)qres[q] : 0.0;
-    const double dB = (double)__uint_as_float(bs->max_resid_bits);
-    const double dot = dq * (B + dB) + qn * dB;
-    const double Kt = (double)(((d + 63) / 64) * 64 + 16);
-    const double acc = Kt * 2 * u * ((metric == METRIC_L2 ? 2 : 1) * (qn + dq) * (B + dB) +
-                                     (metric == METRIC_L2 ? 1.001 * B * B : 0.0));
-    e = metric == METRIC_L2 ? 2 * dot + u * B * B + acc : dot + acc;
+    const float dq = qres ? qres[q] : 0.f;
+    const float dB = __uint_as_float(bs->max_resid_bits);
+    const float dot = dq * (B + dB) + qn * dB;
+    const float Kt = (float)(((d + 63) / 64) * 64 + 16);
+    const float acc = Kt * 2.f * u * ((metric == METRIC_L2 ? 2.f : 1.f) * (qn + dq) * (B + dB) +
+                                      (metric == METRIC_L2 ? 1.001f * B * B : 0.f));
+    e = metric == METRIC_L2 ? 2.f * dot + u * B * B + acc : dot + acc;
   }
   // ||q||^2 (added in the re-rank) and ||b||^2 (inside v) each off by un relative
   e += un * (qn * qn + B * B);
   // fp16 norm parts: their sum is within 2^-25 of ||b||^2
   if (prec == PREC_FP16) e += u;
-  e = e * 1.1 + 1e-30;
-  eps[q] = isfinite(e) ? (float)e : INFINITY;
+  e = e * (1.1f * 1.000005f) + 1.001e-30f;
+  eps[q] = isfinite(e) ? e : INFINITY;
 }
 
 __global__ void eps_split_kernel(int nq, int d, int metric, const double *qn64, const float *qlo,

@@ -229,7 +229,10 @@ __global__ void __launch_bounds__(NT_TC, 1)
     return u;
   };
   // tiles of a unit of n that are scanned twice
-  auto lead_tiles = [](int n) { return RUN && n >= kRunLeadMin ? kRunLead : 0; };
+  const bool seeded = RUN && sel.thr != nullptr;
+  auto lead_tiles = [seeded](int n) {
+    return RUN && !seeded && n >= kRunLeadMin ? kRunLead : 0;
+  };
   const uint32_t crank = PAIR ? cluster_ctarank() : 0;
   const bool leader = crank == 0;
 
@@ -496,7 +499,8 @@ __global__ void __launch_bounds__(NT_TC, 1)
     volatile float *lv_own = Lv + half * 128 + row, *lv_other = Lv + (half ^ 1) * 128 + row;
     if (RUN) {
       if (rvalid) {
-        thr = rmin = INFINITY;
+        rmin = INFINITY;
+        thr = seeded ? sel.thr[qrow] : INFINITY;
         slack = run_slack(sel.run_eps[qrow]);
       }
     } else if (MODE == SCAN_THRESH && rvalid) {
@@ -753,7 +757,7 @@ __global__ void __launch_bounds__(NT_TC, 1)
             m = fminf(m, *lv_other);
           }
           if (m < rmin) {
-            thr = __fadd_ru(m, slack);
+            thr = fminf(thr, __fadd_ru(m, slack));
             // every candidate so far is above the new threshold: start over
             if (thr < rmin) rcount = 0;
             rmin = m;

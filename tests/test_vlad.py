@@ -147,3 +147,29 @@ def test_oracle_port_bit_identical_to_reference(nt):
     got = np.zeros((k, d), np.float32)
     o.orc_vlad_compute(k, d, ptr(C), v.shape[0], ptr(v), ptr(got), nt)
     np.testing.assert_array_equal(got, exp)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,d,k", [(1, 3, 1), (127, 130, 5), (1030, 4, 300), (8192, 36, 7),
+                                   (8193, 9, 64)])
+def test_gpu_vlad_sums(n, d, k):
+    """Both forms of the ordered sums (few points: a block per cluster; many:
+    sorted) at their edges, with empty clusters; then points without a nearest
+    centroid, whose assignment is settled after the sums were queued."""
+    rng = np.random.default_rng(n)
+    C = (rng.standard_normal((k, d)) * 4).astype(np.float32)
+    v = (C[rng.integers(0, max(1, k // 2), n)] + 0.1 * rng.standard_normal((n, d))).astype(np.float32)
+    w = rng.uniform(0.5, 2.0, n).astype(np.float32)
+    a = knn_exact(C, v, 1)[0][:, 0]
+    L = yg.lib()
+    out = np.empty((k, d), np.float32)
+    L.vlad_compute(k, d, ptr(C), n, ptr(v), ptr(out))
+    np.testing.assert_array_equal(out, vlad_np(C, v, a)[0])
+    L.vlad_compute_weighted(k, d, ptr(C), n, ptr(v), ptr(w), ptr(out))
+    np.testing.assert_array_equal(out, vlad_np(C, v, a, w)[0])
+    bad = np.unique(np.array([0, n // 2, n - 1]))
+    v2 = v.copy()
+    v2[bad] = np.nan
+    keep = np.setdiff1d(np.arange(n), bad).astype(np.int32)
+    L.vlad_compute(k, d, ptr(C), n, ptr(v2), ptr(out))
+    np.testing.assert_array_equal(out, vlad_np(C, v, a, None, keep, np.array([len(keep)]))[0])

@@ -102,6 +102,13 @@ constexpr int kPinnedStageSlot = 3;
 // driver's own staging of a pageable destination.
 int copy_to_host(Ctx *c, cudaStream_t st, void *dst, const void *src, size_t bytes);
 
+// Host -> device copy on st.  Up to 64 KB goes through the context's pinned
+// slot and is queued like a kernel (the slot may be used again only after st has
+// been synchronised); more than that is the driver's copy of the caller's
+// memory, which this host's GPU reads in place: 1 MB 17 us, through pinned
+// memory 47.
+int copy_to_device(Ctx *c, cudaStream_t st, int slot, void *dst, const void *src, size_t bytes);
+
 // returns the calling thread's context (created on first use)
 int ctx_get(Ctx **out);
 

@@ -692,12 +692,8 @@ struct GmmDev {
   }
   void upload_v(const float *hv) {
     const size_t bytes = sizeof(float) * (size_t)(n * d);
-    v.get(ctx, where, n * d);
-    const void *src = hv;
-    // (a small pageable copy goes through pinned memory here rather than by
-    // the driver's own staging, which waits for it)
-    if (bytes <= (size_t)1 << 20) src = memcpy(pinned(GP_V, bytes), hv, bytes);
-    ok(where, cudaMemcpyAsync(v.p, src, bytes, cudaMemcpyHostToDevice, ctx->stream));
+    if (copy_to_device(ctx, ctx->stream, GP_V, v.get(ctx, where, n * d), hv, bytes) != OK)
+      die(where);
   }
   void upload_P(const float *hp) {
     ok(where, cudaMemcpyAsync(P.get(ctx, where, n * k), hp, sizeof(float) * (size_t)(n * k),

@@ -332,15 +332,14 @@ int knn_batch(KnnJob &job, Ctx *ctx, cudaStream_t st, Small *dsmall, BaseOps *bo
   }
   if (split)
     YG_CHECK(compute_eps_split(nq, d, job.metric, qn64, qlo, qres, qflag, &dsmall->bs3, eps,
-                               qexact, st));
+                               qexact, st, &dsmall->fail_cnt));
   else
     YG_CHECK(compute_eps(nq, d, job.prec, job.metric, qn64, qres, qflag, &dsmall->bs, eps,
-                         qexact, st));
+                         qexact, st, nullptr, nullptr, &dsmall->fail_cnt));
 
   nv.reset(new NvtxRange(job.band_kth ? "knn.band_pass" : "knn.distance_pass"));
   int *fail_list;
   YG_CHECK(ws_get(ws, WS_FAIL, nq, &fail_list));
-  YG_CUDA(cudaMemsetAsync(&dsmall->fail_cnt, 0, sizeof(int), st));
 
   RerankArgs ra;
   ra.nq = nq; ra.nb = nb; ra.d = d; ra.k = k; ra.metric = job.metric;
@@ -875,11 +874,12 @@ int knn_device(KnnJob &job, Ctx *ctx, cudaStream_t st) {
     YG_CHECK(prep_rows(job.b, job.ldb, nb, d, 1.f, nullptr, bn32, nullptr, bres, nullptr, 0,
                        nullptr, 0, &dsmall->bs, st));
   }
-  // the list length of k > 1 depends on whether the base is exact class (k = 1
-  // does not: no host round trip then); every later read of the small state
-  // also checks the tensor-core passes' error flag
+  // the lists of 2 to 16 neighbours depend on whether the base is exact class
+  // (only the tensor-core passes keep lists, and k = 1 and longer k do without: no
+  // host round trip then); every later read of the small state also checks the
+  // tensor-core passes' error flag
   int bexact = 0;
-  if (k > 1) {
+  if (k > 1 && k <= 16 && job.prec != PREC_FP32) {
     Small hs;
     YG_CHECK(read_small(ctx, dsmall, st, &hs));
     bexact = hs.bs.all_exact;

@@ -133,6 +133,17 @@ int ctx_pinned_status(Ctx *c, void **out) {
   return OK;
 }
 
+int copy_to_device(Ctx *c, cudaStream_t st, int slot, void *dst, const void *src, size_t bytes) {
+  if (bytes == 0) return OK;
+  if (bytes <= (size_t)64 << 10) {
+    void *h;
+    YG_CHECK(c->pinned.get(slot, bytes, &h));
+    src = memcpy(h, src, bytes);
+  }
+  YG_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st));
+  return OK;
+}
+
 int copy_to_host(Ctx *c, cudaStream_t st, void *dst, const void *src, size_t bytes) {
   if (!dst || bytes == 0) return OK;
   cudaPointerAttributes at;

@@ -1205,8 +1205,9 @@ __global__ void __launch_bounds__(256) rerank_small_kernel(RerankArgs a) {
 __global__ void eps_kernel(int nq, int d, int prec, int metric, const double *qn64,
                            const float *qres, const unsigned char *qflag,
                            const SetStats *bs, float *eps, unsigned char *qexact,
-                           const int *qpair, const GroupPair *gpairs) {
+                           const int *qpair, const GroupPair *gpairs, int *zero) {
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
+  if (q == 0 && zero) *zero = 0;
   if (q >= nq) return;
   if (qpair) bs = gpairs[qpair[q]].bs;  // grouped: the query's own pair
   const bool ex = qflag[q] && bs->all_exact;
@@ -1244,8 +1245,10 @@ __global__ void eps_kernel(int nq, int d, int prec, int metric, const double *qn
 
 __global__ void eps_split_kernel(int nq, int d, int metric, const double *qn64, const float *qlo,
                                  const float *qres2, const unsigned char *qflag,
-                                 const SetStats *bs, float *eps, unsigned char *qexact) {
+                                 const SetStats *bs, float *eps, unsigned char *qexact,
+                                 int *zero) {
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
+  if (q == 0 && zero) *zero = 0;
   if (q >= nq) return;
   const bool ex = qflag[q] && bs->all_exact;
   qexact[q] = ex;
@@ -1514,21 +1517,21 @@ int rerank(const RerankArgs &a, cudaStream_t st) {
 int compute_eps(int nq, int d, int prec, int metric, const double *qn64,
                 const float *qres, const unsigned char *qflag, const SetStats *bstats,
                 float *eps, unsigned char *qexact, cudaStream_t st, const int *qpair,
-                const GroupPair *gpairs) {
+                const GroupPair *gpairs, int *zero) {
   if (nq <= 0) return OK;
   eps_kernel<<<(unsigned)ceil_div(nq, 256), 256, 0, st>>>(nq, d, prec, metric, qn64, qres,
                                                           qflag, bstats, eps, qexact, qpair,
-                                                          gpairs);
+                                                          gpairs, zero);
   YG_LAUNCH_CHECK();
   return OK;
 }
 
 int compute_eps_split(int nq, int d, int metric, const double *qn64, const float *qlo,
                       const float *qres2, const unsigned char *qflag, const SetStats *bstats,
-                      float *eps, unsigned char *qexact, cudaStream_t st) {
+                      float *eps, unsigned char *qexact, cudaStream_t st, int *zero) {
   if (nq <= 0) return OK;
   eps_split_kernel<<<(unsigned)ceil_div(nq, 256), 256, 0, st>>>(nq, d, metric, qn64, qlo, qres2,
-                                                                qflag, bstats, eps, qexact);
+                                                                qflag, bstats, eps, qexact, zero);
   YG_LAUNCH_CHECK();
   return OK;
 }

@@ -61,17 +61,20 @@ int rerank(const RerankArgs &a, cudaStream_t st);
 // eps[q] in dist space for the FP32 path (prec 0) or the BF16 path (prec 1),
 // computed from the query's norm / residual and the base set statistics
 // (grouped: those of the query's pair, gpairs[qpair[q]].bs).
-// qexact[q] = query exact class and every base row exact class.
+// qexact[q] = query exact class and every base row exact class.  zero (may be
+// null): an integer set to 0 on the way (the pass's counter of rejected
+// queries, which would take a launch of its own).
 int compute_eps(int nq, int d, int prec, int metric, const double *qn64,
                 const float *qres, const unsigned char *qflag, const SetStats *bstats,
                 float *eps, unsigned char *qexact, cudaStream_t st,
-                const int *qpair = nullptr, const GroupPair *gpairs = nullptr);
+                const int *qpair = nullptr, const GroupPair *gpairs = nullptr,
+                int *zero = nullptr);
 
 // eps[q] for the 3xBF16 split pass: the left-out q_lo.b_lo and residual
 // terms plus the FP32 accumulation of 3*Kp1 + 16 products.
 int compute_eps_split(int nq, int d, int metric, const double *qn64, const float *qlo,
                       const float *qres2, const unsigned char *qflag, const SetStats *bstats,
-                      float *eps, unsigned char *qexact, cudaStream_t st);
+                      float *eps, unsigned char *qexact, cudaStream_t st, int *zero = nullptr);
 
 // THRESH thresholds from a TOPC pass over a sample: thr[q] (v space) = the
 // c-th smallest sampled value + 2 eps[q], rounded up.

@@ -58,6 +58,33 @@ __global__ void offsets_kernel(const int *sorted, long n, int nseg, int *offs) {
   offs[g] = (int)lo;
 }
 
+// The sum of (v_i - cj) (* w_i) over the m points idx[0..m), one after the other;
+// v: the coordinate's column (stride d).  Eight loads in flight: the sum's
+// order is fixed, the loads' is not.
+__device__ __forceinline__ float ordered_sum(const int *idx, int m, const float *__restrict__ v,
+                                             int d, float cj, const float *__restrict__ w) {
+  float s = 0.f;
+  int e = 0;
+  for (; e + 8 <= m; e += 8) {
+    float r[8];
+#pragma unroll
+    for (int u = 0; u < 8; u++) {
+      const int i = idx[e + u];
+      r[u] = __fsub_rn(v[(long)i * d], cj);
+      if (w) r[u] = __fmul_rn(r[u], w[i]);
+    }
+#pragma unroll
+    for (int u = 0; u < 8; u++) s = __fadd_rn(s, r[u]);
+  }
+  for (; e < m; e++) {
+    const int i = idx[e];
+    float r = __fsub_rn(v[(long)i * d], cj);
+    if (w) r = __fmul_rn(r, w[i]);
+    s = __fadd_rn(s, r);
+  }
+  return s;
+}
+
 // desc[g][j], g = subset * k + c: the ordered sum of (v_i[j] - C[c][j]) (* w_i)
 __global__ void vlad_sum_kernel(const int *perm, const int *offs, const float *v, int d,
                                 const float *C, const float *w, int k, long nseg, float *desc) {
@@ -66,14 +93,47 @@ __global__ void vlad_sum_kernel(const int *perm, const int *offs, const float *v
   const long g = t / d;
   const int j = (int)(t - g * d), c = (int)(g % k);
   const float cj = C[(long)c * d + j];
-  float s = 0.f;
-  for (int e = offs[g]; e < offs[g + 1]; e++) {
-    const int i = perm[e];
-    float r = __fsub_rn(v[(long)i * d + j], cj);
-    if (w) r = __fmul_rn(r, w[i]);
-    s = __fadd_rn(s, r);
+  const int e0 = offs[g];
+  desc[t] = ordered_sum(perm + e0, offs[g + 1] - e0, v + j, d, cj, w);
+}
+
+// The same for few points without subsets (kScanMax): a block per cluster (and
+// 128 coordinates) picks its cluster's points out of the assignment itself, in
+// order, instead of a sort of all of them and its three launches.
+// 2,000 points, k = 64, d = 128: 35 us for keys, sort, offsets and sums, 10 here.
+constexpr int kScanMax = 8192, kScanT = 128;
+__global__ void __launch_bounds__(kScanT)
+    vlad_scan_kernel(const int *__restrict__ assign, int n, const float *__restrict__ v, int d,
+                     const float *__restrict__ C, const float *__restrict__ w,
+                     float *__restrict__ desc) {
+  __shared__ int list[kScanMax];
+  __shared__ int wcount[kScanT / 32];
+  const int c = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  // each thread looks at consecutive points: counts, offsets, then indices
+  const int per = (n + kScanT - 1) / kScanT, i0 = tid * per, i1 = min(n, i0 + per);
+  int cnt = 0;
+  for (int i = i0; i < i1; i++) cnt += assign[i] == c;
+  int x = cnt;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
   }
-  desc[t] = s;
+  if (lane == 31) wcount[warp] = x;
+  __syncthreads();
+  int total = 0;
+  for (int q = 0; q < kScanT / 32; q++) {
+    if (q < warp) x += wcount[q];
+    total += wcount[q];
+  }
+  int pos = x - cnt;
+  if (cnt)
+    for (int i = i0; i < i1; i++)
+      if (assign[i] == c) list[pos++] = i;
+  __syncthreads();
+  const int j = blockIdx.y * kScanT + tid;
+  if (j >= d) return;
+  desc[(long)c * d + j] = ordered_sum(list, total, v + j, d, C[(long)c * d + j], w);
 }
 
 __global__ void hist_int_kernel(const int *assign, long n, int k, int *desc) {
@@ -104,16 +164,21 @@ __global__ void subset_of_kernel(const int *ends, int nsub, long n, int *sub_of)
   sub_of[e] = lo;
 }
 
+// pinned slots of the small uploads and of a small descriptor on its way back
+enum VladPinned : int { VP_V = 11, VP_C, VP_DESC };
+
 struct Assigned {
   Ctx *ctx = nullptr;
   cudaStream_t st = nullptr;
   float *dv = nullptr, *dc = nullptr;
   int *assign = nullptr;
+  KnnJob job;  // pending when its certificate check was deferred (defer)
 };
 
-// the ma nearest centroids of every point (yael's nn / knn_thread semantics)
+// the ma nearest centroids of every point (yael's nn / knn_thread semantics);
+// defer: the check of ma = 1 may be left to the caller's knn_resolve
 int assign_points(int k, int d, const float *centroids, int n, const float *v, int ma,
-                  Assigned *A) {
+                  Assigned *A, bool defer = false) {
   YG_CHECK(ctx_get(&A->ctx));
   A->st = A->ctx->stream;
   Workspace &ws = A->ctx->ws;
@@ -122,14 +187,14 @@ int assign_points(int k, int d, const float *centroids, int n, const float *v, i
   YG_CHECK(vs_get(ws, VS_C, (size_t)k * d, &A->dc));
   YG_CHECK(vs_get(ws, VS_ASSIGN, (size_t)n * ma, &A->assign));
   YG_CHECK(vs_get(ws, VS_DIS, (size_t)n * ma, &dis));
-  YG_CUDA(cudaMemcpyAsync(A->dv, v, sizeof(float) * n * (size_t)d, cudaMemcpyHostToDevice, A->st));
-  YG_CUDA(cudaMemcpyAsync(A->dc, centroids, sizeof(float) * k * (size_t)d, cudaMemcpyHostToDevice,
-                          A->st));
-  KnnJob job;
+  YG_CHECK(copy_to_device(A->ctx, A->st, VP_V, A->dv, v, sizeof(float) * n * (size_t)d));
+  YG_CHECK(copy_to_device(A->ctx, A->st, VP_C, A->dc, centroids, sizeof(float) * k * (size_t)d));
+  KnnJob &job = A->job;
   job.nq = n; job.nb = k; job.d = d; job.k = ma; job.metric = METRIC_L2;
   job.prec = default_precision();
   job.q = A->dv; job.ldq = d; job.b = A->dc; job.ldb = d;
   job.out_idx = A->assign; job.out_dis = dis;
+  job.defer = defer && ma == 1;
   return knn_device(job, A->ctx, A->st);
 }
 
@@ -179,7 +244,7 @@ int vlad_run(int k, int d, const float *centroids, int n, const float *v, const 
     return OK;
   }
   Assigned A;
-  YG_CHECK(assign_points(k, d, centroids, n, v, 1, &A));
+  YG_CHECK(assign_points(k, d, centroids, n, v, 1, &A, true));
   Workspace &ws = A.ctx->ws;
   const float *dw = nullptr;
   if (weights) {
@@ -203,15 +268,34 @@ int vlad_run(int k, int d, const float *centroids, int n, const float *v, const 
     didx = ix;
     dsub = so;
   }
-  int *perm, *offs;
-  YG_CHECK(sort_segments(A, didx, dsub, ne, k, (int)nseg, &perm, &offs));
   float *ddesc;
+  const size_t bytes = sizeof(float) * (size_t)nseg * d;
   YG_CHECK(vs_get(ws, VS_DESC, (size_t)nseg * d, &ddesc));
-  vlad_sum_kernel<<<(unsigned)ceil_div(nseg * d, 256), 256, 0, A.st>>>(perm, offs, A.dv, d, A.dc,
-                                                                       dw, k, nseg, ddesc);
-  YG_LAUNCH_CHECK();
-  YG_CUDA(cudaMemcpyAsync(desc, ddesc, sizeof(float) * nseg * d, cudaMemcpyDeviceToHost, A.st));
-  YG_CUDA(cudaStreamSynchronize(A.st));
+  void *host = desc;  // a small descriptor comes back through pinned memory
+  if (bytes <= (size_t)1 << 20) YG_CHECK(A.ctx->pinned.get(VP_DESC, bytes, &host));
+  auto sums = [&]() -> int {
+    if (!subsets && n <= kScanMax && ceil_div(d, kScanT) <= 65535) {
+      vlad_scan_kernel<<<dim3((unsigned)k, (unsigned)ceil_div(d, kScanT)), kScanT, 0, A.st>>>(
+          A.assign, n, A.dv, d, A.dc, dw, ddesc);
+    } else {
+      int *perm, *offs;
+      YG_CHECK(sort_segments(A, didx, dsub, ne, k, (int)nseg, &perm, &offs));
+      vlad_sum_kernel<<<(unsigned)ceil_div(nseg * d, 256), 256, 0, A.st>>>(
+          perm, offs, A.dv, d, A.dc, dw, k, nseg, ddesc);
+    }
+    YG_LAUNCH_CHECK();
+    YG_CUDA(cudaMemcpyAsync(host, ddesc, bytes, cudaMemcpyDeviceToHost, A.st));
+    YG_CUDA(cudaStreamSynchronize(A.st));
+    return OK;
+  };
+  YG_CHECK(sums());
+  if (A.job.pending) {
+    // (the assignment's certificate, checked behind the sums: where it rejected
+    // points, they are settled and the sums run again)
+    YG_CHECK(knn_resolve(A.job, A.ctx, A.st));
+    if (A.job.n_band + A.job.n_fallback > 0) YG_CHECK(sums());
+  }
+  if (host != desc) memcpy(desc, host, bytes);
   return OK;
 }
 

@@ -40,7 +40,7 @@ enum KmSlot : int {
   KS_TCU = 160, KS_TCPK, KS_TCSIDE, KS_TCXN, KS_TCXRES, KS_TCCPK, KS_TCCSIDE, KS_TCSTATS,
   KS_TCERR, KS_PRIOR, KS_TCMU, KS_TCMUPART, KS_TCSLF, KS_TCNPT, KS_TCHMAX,
   KS_HSTART, KS_HPINST, KS_GCNT, KS_GTOT, KS_TCTSIDE, KS_TCCSCR, KS_TCIB, KS_SPLITROWS,
-  KS_SPLITBUF,
+  KS_SPLITBUF, KS_CUR, KS_MOVED,
 };
 
 // the split centroid rows put back: row r of src to row rows[r] of dst
@@ -109,16 +109,28 @@ struct Engine {
   float ms_assign = 0, ms_update = 0;
   long point_iters = 0, engine_iters = 0;  // sum of active points per iteration; iterations
 
-  // CUDA graphs of one Lloyd iteration's device work: the update always, the
-  // assignment on the grouped small-k path (the k-NN path reads its
-  // certificate results on the host).  Both are captured on the second
-  // iteration (the first runs eagerly and sets every kernel attribute) and
-  // replayed after.
+  // CUDA graphs of one Lloyd iteration's device work: the whole of it on the
+  // grouped small-k path, the update alone on the k-NN path (which reads its
+  // certificate results on the host); [1]: with the update from the points
+  // that moved.  They are captured from the second iteration on (the first
+  // runs eagerly and sets every kernel attribute) and replayed after.
   // Their arguments never change within a run: the per-iteration state (active
   // instances, split centroids) lives in device buffers written between
   // replays.  YAEL_GPU_GRAPHS=0 runs every iteration eagerly.
-  cudaGraphExec_t g_assign = nullptr, g_update = nullptr;
+  cudaGraphExec_t g_all[2] = {}, g_update[2] = {};
   bool eager_done = false;
+  // the iteration's timing events (ev[1] between assignment and update), and
+  // the side stream of a capture with its fork and join
+  cudaEvent_t ev[3] = {}, ev_fork = nullptr, ev_join = nullptr;
+  cudaStream_t side = nullptr;
+  bool capturing = false;
+  // One instance whose sums are not fused with its assignment: acc and counts
+  // are those of the assignment in cur.  Where the last iteration moved few
+  // points, the next update adds and subtracts the moved rows alone (integer
+  // sums: the same bits as the full update's).
+  int *cur = nullptr, *moved = nullptr, *ph_moved = nullptr;
+  bool sums_live = false;   // cur and the sums hold an assignment of this run
+  long last_moved = -1;     // points that changed centroid in the last iteration
   // The chosen form's assignment for k <= 256 (km_tc.cu): the 16-bit tensor
   // cores with an exact band re-check, and, when k * d fits shared memory, the
   // centroid sums fused into it (no second pass over the points).
@@ -132,14 +144,35 @@ struct Engine {
   int *tc_err = nullptr;
   int *ph_err = nullptr;  // pinned copy of tc_err the update graph writes
   bool assign_settled = false;  // the grouped assignment's variant is tuned
-  long g_assign_n = 0, g_update_n = 0;  // kernels per replay
+  long g_all_n[2] = {}, g_update_n[2] = {};  // kernels per replay
   bool graphs_failed = false;
   int *ph_counts = nullptr;     // pinned copies the update graph writes
   double *ph_part = nullptr;
 
   ~Engine() {
-    if (g_assign) cudaGraphExecDestroy(g_assign);
-    if (g_update) cudaGraphExecDestroy(g_update);
+    for (int i = 0; i < 2; i++) {
+      if (g_all[i]) cudaGraphExecDestroy(g_all[i]);
+      if (g_update[i]) cudaGraphExecDestroy(g_update[i]);
+    }
+    for (cudaEvent_t e : {ev[0], ev[1], ev[2], ev_fork, ev_join})
+      if (e) cudaEventDestroy(e);
+    if (side) cudaStreamDestroy(side);
+  }
+
+  // body(stream) beside what follows on st until join(): on the side stream
+  // of a capture, in line otherwise
+  template <typename F>
+  int fork(F body) {
+    if (!capturing) return body(st);
+    YG_CUDA(cudaEventRecord(ev_fork, st));
+    YG_CUDA(cudaStreamWaitEvent(side, ev_fork, 0));
+    YG_CHECK(body(side));
+    YG_CUDA(cudaEventRecord(ev_join, side));
+    return OK;
+  }
+  int join() {
+    if (capturing) YG_CUDA(cudaStreamWaitEvent(st, ev_join, 0));
+    return OK;
   }
 
   // L1 / chi2 k-means (one instance): per-coordinate distances searched
@@ -161,11 +194,19 @@ struct Engine {
   template <typename F>
   bool capture(F body, cudaGraphExec_t *exec, long *nlaunch) {
     const long l0 = launch_count();
+    if (!side && (cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking) != cudaSuccess ||
+                  cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming) != cudaSuccess ||
+                  cudaEventCreateWithFlags(&ev_join, cudaEventDisableTiming) != cudaSuccess)) {
+      (void)cudaGetLastError();
+      return false;
+    }
     if (cudaStreamBeginCapture(st, cudaStreamCaptureModeRelaxed) != cudaSuccess) {
       (void)cudaGetLastError();
       return false;
     }
+    capturing = true;
     const int rc = body();
+    capturing = false;
     cudaGraph_t g = nullptr;
     const cudaError_t e = cudaStreamEndCapture(st, &g);
     // uploaded here, so that the first replay does not carry the upload
@@ -499,20 +540,38 @@ struct Engine {
         point_iters += x.n;
       }
     engine_iters++;
-    cudaEvent_t e0, e1, e2;
-    cudaEventCreate(&e0);
-    cudaEventCreate(&e1);
-    cudaEventCreate(&e2);
+    for (cudaEvent_t &e : ev)
+      if (!e) YG_CUDA(cudaEventCreate(&e));
+    const cudaEvent_t e0 = ev[0], e1 = ev[1], e2 = ev[2];
+    const bool track = ni == 1 && !tc_fuse && !tc && !alt_mode();
+    if (track && !cur) {
+      YG_CHECK(ws_get(ctx->ws, KS_CUR, (size_t)ntot, &cur));
+      YG_CHECK(ws_get(ctx->ws, KS_MOVED, 1, &moved));
+      YG_CHECK(ctx->pinned.get(5, sizeof(int), reinterpret_cast<void **>(&ph_moved)));
+    }
+    // A moved row costs two rows of 64-bit atomics where the full update reads
+    // every row once: 50k x 64, k = 100: full update 34 us, XXD with few moves.
+    const int delta = track && sums_live && last_moved >= 0 && 16 * last_moved < ntot ? 1 : 0;
+    // the counts, the slice sums and a flag go straight to the pinned host
+    // buffers (no copies in the step); the slice sums run beside the centroids
+    auto slice_sums = [&](cudaStream_t s) { return km_slice_sums(slices, nsl, dis, ph_part, s); };
     auto update_body = [&]() -> int {
       if (tc_fuse) {
-        // the sums and counts came with the assignment; the counts, the error
-        // flag and the objective's slice sums are written straight to the
-        // pinned host buffers (no copies in the step)
+        // the sums and counts came with the assignment
+        YG_CHECK(fork(slice_sums));
         YG_CHECK(km_finalize(acc, counts, ncl, d, k, shift, active, C, st, ph_counts, tc_err,
                              ph_err));
         if (flags & YAEL_KMEANS_NORMALIZE_CENTS) YG_CHECK(km_normalize(C, ncl, d, k, active, st));
-        YG_CHECK(km_slice_sums(slices, nsl, dis, ph_part, st));
-        return OK;
+        return join();
+      }
+      if (delta) {
+        YG_CHECK(fork(slice_sums));
+        YG_CUDA(cudaMemsetAsync(moved, 0, sizeof(int), st));
+        YG_CHECK(km_moves(assign, cur, v, d, ntot, shift, acc, counts, moved, st));
+        YG_CHECK(km_finalize(acc, counts, ncl, d, k, shift, active, C, st, ph_counts, moved,
+                             ph_moved));
+        if (flags & YAEL_KMEANS_NORMALIZE_CENTS) YG_CHECK(km_normalize(C, ncl, d, k, active, st));
+        return join();
       }
       if (tc) YG_CUDA(cudaMemcpyAsync(ph_err, tc_err, sizeof(int), cudaMemcpyDeviceToHost, st));
       YG_CUDA(cudaMemsetAsync(counts, 0, sizeof(int) * ncl, st));
@@ -541,14 +600,23 @@ struct Engine {
         YG_CUDA(cudaMemcpyAsync(ph_part, part, sizeof(double) * nsl, cudaMemcpyDeviceToHost, st));
         return OK;
       }
+      YG_CHECK(fork(slice_sums));
       YG_CHECK(km_scan(counts, ncl, offs, cursor, st));
       YG_CHECK(km_scatter(assign, pinst, ntot, k, active, cursor, perm, st));
+      if (track) {
+        YG_CUDA(cudaMemsetAsync(moved, 0, sizeof(int), st));
+        YG_CHECK(km_track(assign, cur, ntot, moved, st));
+      }
       YG_CHECK(km_update(perm, offs + ncl, ntot, assign, pinst, counts, v, d, ncl, k, shift,
-                         active, acc, C, st));
+                         active, acc, C, st, ph_counts, track ? moved : nullptr,
+                         track ? ph_moved : nullptr));
       if (flags & YAEL_KMEANS_NORMALIZE_CENTS) YG_CHECK(km_normalize(C, ncl, d, k, active, st));
-      YG_CHECK(km_slice_sums(slices, nsl, dis, part, st));
-      YG_CUDA(cudaMemcpyAsync(ph_counts, counts, sizeof(int) * ncl, cudaMemcpyDeviceToHost, st));
-      YG_CUDA(cudaMemcpyAsync(ph_part, part, sizeof(double) * nsl, cudaMemcpyDeviceToHost, st));
+      return join();
+    };
+    auto run_update = [&](bool graph) -> int {
+      if (!graph) return update_body();
+      YG_CUDA(cudaGraphLaunch(g_update[delta], st));
+      count_launches(g_update_n[delta]);
       return OK;
     };
     const bool probing = probe && probe->n_probe > 0 && ni == 1 && probe_t < probe->probe_iters;
@@ -563,44 +631,46 @@ struct Engine {
     // (a run's first fused assignment starts its sums: eager, as it differs)
     const bool graph_assign =
         use_graphs && assign_graph_wanted() && assign_settled && !(tc_fuse && !tc_live);
-    if (use_graphs && !g_update && !capture(update_body, &g_update, &g_update_n))
+    if (graph_assign) {
+      // (one graph, one launch: the event between the two is a node of it)
+      auto all = [&]() -> int {
+        YG_CHECK(assign_step());
+        YG_CUDA(cudaEventRecordWithFlags(e1, st, cudaEventRecordExternal));
+        return update_body();
+      };
+      if (!g_all[delta] && !capture(all, &g_all[delta], &g_all_n[delta])) graphs_failed = true;
+    } else if (use_graphs && !g_update[delta] &&
+               !capture(update_body, &g_update[delta], &g_update_n[delta])) {
       graphs_failed = true;
-    if (graph_assign && !g_assign && !graphs_failed &&
-        !capture([&] { return assign_step(); }, &g_assign, &g_assign_n))
-      graphs_failed = true;
+    }
+    const bool graph_update = use_graphs && !graph_assign && !graphs_failed;
     cudaEventRecord(e0, st);
     std::unique_ptr<NvtxRange> nv(new NvtxRange("kmeans.assign"));
     if (graph_assign && !graphs_failed) {
-      YG_CUDA(cudaGraphLaunch(g_assign, st));
-      count_launches(g_assign_n);
+      YG_CUDA(cudaGraphLaunch(g_all[delta], st));
+      count_launches(g_all_n[delta]);
     } else {
       YG_CHECK(assign_step());
-    }
-    cudaEventRecord(e1, st);
-    nv.reset(new NvtxRange("kmeans.update"));
-    if (use_graphs && !graphs_failed) {
-      YG_CUDA(cudaGraphLaunch(g_update, st));
-      count_launches(g_update_n);
-    } else {
-      YG_CHECK(update_body());
+      cudaEventRecord(e1, st);
+      nv.reset(new NvtxRange("kmeans.update"));
+      YG_CHECK(run_update(graph_update));
     }
     eager_done = true;
     cudaEventRecord(e2, st);
     YG_CUDA(cudaStreamSynchronize(st));
-    if (!g_assign) assign_settled = km_assign_tune_collect();
+    long nmoved = track ? *ph_moved : -1;
+    if (!g_all[0] && !g_all[1]) assign_settled = km_assign_tune_collect();
     if (pend.pending) {
       YG_CHECK(knn_resolve(pend, ctx, st));
       count_assign(pend);
       if (pend.n_band > 0) {  // some points were re-run: their clusters changed
-        if (use_graphs && !graphs_failed) {
-          YG_CUDA(cudaGraphLaunch(g_update, st));
-          count_launches(g_update_n);
-        } else {
-          YG_CHECK(update_body());
-        }
+        YG_CHECK(run_update(graph_update));
         YG_CUDA(cudaStreamSynchronize(st));
+        if (track) nmoved += *ph_moved;
       }
     }
+    last_moved = sums_live ? nmoved : -1;  // (against an assignment of this run)
+    sums_live = track;
     if (tc && *ph_err) {
       set_error(E_TIMEOUT, "k-means tensor-core assignment gave up waiting (bounded wait expired)");
       return E_TIMEOUT;
@@ -615,9 +685,6 @@ struct Engine {
     if (trace_enabled())
       fprintf(stderr, "[yael_gpu] kmeans iteration %ld: assign %.3f ms, update %.3f ms (events), "
               "%.3f ms on the host clock\n", engine_iters, a, b, wall_ms() - t_host0);
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
-    cudaEventDestroy(e2);
 
     // objective per instance: slice sums in point order
     std::vector<double> q(ni, 0.0);
@@ -854,6 +921,7 @@ int kmeans_run(int d, int n, int k, int niter, const float *v_in, int flags, lon
     x.tot_re = 0; x.iters = 0; x.ret = 0; x.done = false;
     E.have_prev = false;
     E.tc_live = false;
+    E.sums_live = false;
     x.qerr = HUGE_VAL; x.qerr_old = HUGE_VAL;
     YG_CHECK(E.set_active());
     if (tr) YG_CUDA(cudaStreamSynchronize(st));
@@ -889,8 +957,8 @@ int kmeans_run(int d, int n, int k, int niter, const float *v_in, int flags, lon
     fprintf(stderr,
             "[yael_gpu] kmeans n=%d k=%d d=%d iterations=%ld assign=%.3fms update=%.3fms "
             "graphs(assign=%d update=%d failed=%d) tc=%d fused=%d prec=%d\n",
-            n, k, d, iter_tot, E.ms_assign, E.ms_update, E.g_assign != nullptr,
-            E.g_update != nullptr, (int)E.graphs_failed, (int)E.tc, (int)E.tc_fuse, E.prec_used);
+            n, k, d, iter_tot, E.ms_assign, E.ms_update, E.g_all[0] || E.g_all[1],
+            E.g_update[0] || E.g_update[1], (int)E.graphs_failed, (int)E.tc, (int)E.tc_fuse, E.prec_used);
   if (verbose && core_ret >= 0) {
     printf("Total number of iterations: %ld\n", iter_tot);
     // unbalanced factor of the last iteration's counts (yael/vector.c:2301-2314)

@@ -160,7 +160,8 @@ int km_scatter(const int *assign, const int *pinst, long n, int k,
 int km_update(const long *perm, const long *total, long nmax, const int *assign,
               const int *pinst, const int *counts, const float *v, int d, long ncl, int k,
               const int *shift, const unsigned char *active, long long *acc, float *C,
-              cudaStream_t st);
+              cudaStream_t st, int *counts_out = nullptr,
+              const int *flag = nullptr, int *flag_out = nullptr);
 
 // kth[p] >= the exact squared distance from point p to centroid assign[p]
 // (FP32 direct differences widened by their rounding bound; +inf for -1): an
@@ -168,6 +169,11 @@ int km_update(const long *perm, const long *total, long nmax, const int *assign,
 int km_prior_bound(const float *v, int d, long n, const int *assign, const float *C, float *kth,
                    cudaStream_t st);
 
+// cur = assign, *moved += the points that differed; km_moves also brings the
+// sums and counts of cur to those of assign (one instance: shift[0])
+int km_track(const int *assign, int *cur, long n, int *moved, cudaStream_t st);
+int km_moves(const int *assign, int *cur, const float *v, int d, long n, const int *shift,
+             long long *acc, int *counts, int *moved, cudaStream_t st);
 // the readout of km_update alone, for sums accumulated elsewhere (km_tc_assign);
 // with counts_out / err_out (host-mapped memory, say) it also copies the
 // counts and *err there

@@ -495,6 +495,57 @@ __global__ void __launch_bounds__(256)
   }
 }
 
+// cur = assign; *moved += the points where they differed
+__global__ void track_kernel(const int *__restrict__ assign, int *__restrict__ cur, long n,
+                             int *moved) {
+  const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  bool m = false;
+  if (i < n) {
+    const int a = assign[i];
+    m = a != cur[i];
+    if (m) cur[i] = a;
+  }
+  const unsigned b = __ballot_sync(0xffffffffu, m);
+  if (b && (threadIdx.x & 31) == 0) atomicAdd(moved, __popc(b));
+}
+
+// The sums and counts of cur made those of assign: a warp looks at 32 points and
+// adds each moved one's row to its new cluster and takes it from its old one
+// (lanes over coordinates, integer atomics: the order does not matter).
+__global__ void moves_kernel(const int *__restrict__ assign, int *__restrict__ cur,
+                             const float *__restrict__ v, int d, long n,
+                             const int *__restrict__ shift, long long *acc, int *counts,
+                             int *moved) {
+  const int lane = threadIdx.x & 31;
+  const long i0 = ((long)blockIdx.x * blockDim.x + threadIdx.x) - lane, i = i0 + lane;
+  int a = -1, b = -1;
+  if (i < n) {
+    a = assign[i];
+    b = cur[i];
+    if (a != b) cur[i] = a;
+  }
+  unsigned m = __ballot_sync(0xffffffffu, a != b);
+  if (!m) return;
+  if (lane == 0) atomicAdd(moved, __popc(m));
+  const int sh = shift[0];
+  while (m) {
+    const int s = __ffs(m) - 1;
+    m &= m - 1;
+    const int jn = __shfl_sync(0xffffffffu, a, s), jo = __shfl_sync(0xffffffffu, b, s);
+    const float *x = v + (i0 + s) * d;
+    for (int c = lane; c < d; c += 32) {
+      const long long f = fixed_of(x[c], sh);
+      if (jn >= 0) atomicAdd((unsigned long long *)(acc + (long)jn * d + c), (unsigned long long)f);
+      if (jo >= 0)
+        atomicAdd((unsigned long long *)(acc + (long)jo * d + c), (unsigned long long)(-f));
+    }
+    if (lane == 0) {
+      if (jn >= 0) atomicAdd(counts + jn, 1);
+      if (jo >= 0) atomicAdd(counts + jo, -1);
+    }
+  }
+}
+
 __global__ void finalize_kernel(const long long *acc, const int *counts, long ncl, int d,
                                 int k, const int *shift, const unsigned char *active,
                                 float *C, int *counts_out, const int *err, int *err_out) {
@@ -923,7 +974,7 @@ int km_scatter(const int *assign, const int *pinst, long n, int k,
 int km_update(const long *perm, const long *total, long nmax, const int *assign,
               const int *pinst, const int *counts, const float *v, int d, long ncl, int k,
               const int *shift, const unsigned char *active, long long *acc, float *C,
-              cudaStream_t st) {
+              cudaStream_t st, int *counts_out, const int *flag, int *flag_out) {
   YG_CUDA(cudaMemsetAsync(acc, 0, sizeof(long long) * ncl * d, st));
   if (nmax > 0) {
     const long warps = ceil_div(nmax, 32);
@@ -938,7 +989,7 @@ int km_update(const long *perm, const long *total, long nmax, const int *assign,
     YG_LAUNCH_CHECK();
   }
   finalize_kernel<<<(unsigned)ceil_div(ncl * d, 256), 256, 0, st>>>(
-      acc, counts, ncl, d, k, shift, active, C, nullptr, nullptr, nullptr);
+      acc, counts, ncl, d, k, shift, active, C, counts_out, flag, flag_out);
   YG_LAUNCH_CHECK();
   return OK;
 }
@@ -975,6 +1026,22 @@ int km_prior_bound(const float *v, int d, long n, const int *assign, const float
                    cudaStream_t st) {
   if (n <= 0) return OK;
   prior_bound_kernel<<<(unsigned)ceil_div(n * 32, 256), 256, 0, st>>>(v, d, n, assign, C, kth);
+  YG_LAUNCH_CHECK();
+  return OK;
+}
+
+int km_track(const int *assign, int *cur, long n, int *moved, cudaStream_t st) {
+  if (n <= 0) return OK;
+  track_kernel<<<(unsigned)ceil_div(n, 256), 256, 0, st>>>(assign, cur, n, moved);
+  YG_LAUNCH_CHECK();
+  return OK;
+}
+
+int km_moves(const int *assign, int *cur, const float *v, int d, long n, const int *shift,
+             long long *acc, int *counts, int *moved, cudaStream_t st) {
+  if (n <= 0) return OK;
+  moves_kernel<<<(unsigned)ceil_div(n, 256), 256, 0, st>>>(assign, cur, v, d, n, shift, acc,
+                                                           counts, moved);
   YG_LAUNCH_CHECK();
   return OK;
 }

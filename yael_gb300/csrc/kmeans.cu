@@ -550,8 +550,8 @@ struct Engine {
       YG_CHECK(ctx->pinned.get(5, sizeof(int), reinterpret_cast<void **>(&ph_moved)));
     }
     // A moved row costs two rows of 64-bit atomics where the full update reads
-    // every row once: 50k x 64, k = 100: full update 34 us, XXD with few moves.
-    const int delta = track && sums_live && last_moved >= 0 && 16 * last_moved < ntot ? 1 : 0;
+    // every row once: 50k x 64, k = 100: full update 34 us, 5 with few moves.
+    const int delta = track && sums_live && last_moved >= 0 && 3 * last_moved < ntot ? 1 : 0;
     // the counts, the slice sums and a flag go straight to the pinned host
     // buffers (no copies in the step); the slice sums run beside the centroids
     auto slice_sums = [&](cudaStream_t s) { return km_slice_sums(slices, nsl, dis, ph_part, s); };

@@ -743,7 +743,7 @@ int knn_batches(KnnJob &job, Ctx *ctx, cudaStream_t st, Small *dsmall, BaseOps *
                          : plan.usable(nb)
                              ? pow2_at_least((int)(2.0 * er + 6.0 * sqrt(er) + 16.0))
                              : 2 * (size_t)ceil_div(nb, nch) + 2 * tile_n;
-      per_query = (size_t)nch * (cap * 8 + 8) + 64 * 16 * 4 + 64;
+      per_query = (size_t)nch * (cap * 8 + 8) + (k == 1 ? 0 : 64 * 16 * 4) + 64;
     } else if (cn <= 16) {
       // the autotuner may try up to 3x the heuristic's chunk count
       const int nch = imin(imin(1024, kMaxCandidates / C),

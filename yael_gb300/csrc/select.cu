@@ -117,6 +117,46 @@ __device__ __forceinline__ float warp_sample_rank(int nq, int nchunk, int C, int
   return v;
 }
 
+// ||q||^2 of the distance pass: the packing's FP32 sum, kept as a double
+__device__ __forceinline__ float query_norm(const RerankArgs &a, int q) {
+  return a.metric == METRIC_L2 ? (float)a.qn64[q] : 0.f;
+}
+
+// error bound of an FP32 inner product (the squared distances' is relative)
+__device__ __forceinline__ float dot_error(const RerankArgs &a, int q, const SetStats *bs) {
+  if (a.metric == METRIC_L2) return 0.f;
+  const float qn = a.qn64 ? sqrtf(fmaxf((float)a.qn64[q], 0.f)) * 1.000001f : 0.f;
+  return (float)(a.d + 4) * kU * qn * __uint_as_float(bs->max_norm_bits);
+}
+
+// The limit of the band of candidates, ak + 2 eps + 4e-7 |ak| + 1e-30, in FP32
+// rounded up, with larger constants and a relative margin: at least its exact
+// value, so the band holds every row that can be an answer.  (This part's FP64
+// pipe runs at 1/64 of the FP32 rate: a few FP64 operations per thread of a
+// block were a tenth of the re-rank.)
+__device__ __forceinline__ float band_limit(float ak, float eps) {
+  const float l = __fadd_ru(__fadd_ru(ak, __fmul_ru(2.f, eps)),
+                            __fadd_ru(__fmul_ru(4.01e-7f, fabsf(ak)), 1.01e-30f));
+  return __fadd_ru(l, __fmul_ru(fabsf(l), 1.2e-7f));
+}
+
+// The certificate ekh <= bound - eps - 4e-7 |bound| (TOPC: <) in FP32 with outward
+// rounding (and 4.01e-7 for the roundings of the bound): it holds only where
+// the exact form holds.  ekh: the k-th exact distance rounded up; t: the
+// value below which (THRESH: up to which, without ||q||^2) every row is a
+// candidate.  Without one (t = +inf: every row is, or no list was full) nothing
+// lies outside; an infinite eps certifies nothing.
+__device__ __forceinline__ bool certified(float ekh, float t, float qn, float eps, bool thresh) {
+  if (t == INFINITY) return eps < INFINITY;
+  float blo = t, babs = fabsf(t);
+  if (thresh) {
+    blo = __fadd_rd(t, qn);
+    babs = fmaxf(fabsf(blo), fabsf(__fadd_ru(t, qn)));
+  }
+  const float low = __fsub_rd(__fsub_rd(blo, eps), __fmul_ru(4.01e-7f, babs));
+  return thresh ? ekh <= low : ekh < low;
+}
+
 // The need-th smallest (from 1) of a block's keys, RK per thread (0xffffffff where
 // valid has no bit), by counting digits of 8 bits below the keys' common range:
 // distances of one query share their leading bits, so two or three rounds of
@@ -265,8 +305,7 @@ __global__ void __launch_bounds__(RT) rerank_kernel(RerankArgs a, int Mp_alloc) 
   const int q = blockIdx.x;
   const int tid = threadIdx.x;
   const int k = a.k, d = a.d;
-  const bool L2 = a.metric == METRIC_L2;
-  const double qn = L2 ? a.qn64[q] : 0.0;
+  const float qn = query_norm(a, q);
   const float eps = a.eps ? a.eps[q] : 0.f;
   const bool ex = a.qexact ? a.qexact[q] != 0 : false;
   // a grouped row reads its pair's candidate regions, base, statistics and
@@ -300,7 +339,7 @@ __global__ void __launch_bounds__(RT) rerank_kernel(RerankArgs a, int Mp_alloc) 
       const int id = s.topi[o];
       if (id < 0) continue;
       const float v = s.topv[o];
-      const float av = L2 ? (float)((double)v + qn) : v;
+      const float av = __fadd_rn(v, qn);
       const int pos = atomicAdd(&sM, 1);
       K[pos] = f2ord(av);
       I[pos] = id;
@@ -357,7 +396,7 @@ __global__ void __launch_bounds__(RT) rerank_kernel(RerankArgs a, int Mp_alloc) 
         }
         const long o = cand_base + ((long)lo * nqv + qloc) * cap + (e - s_off[lo]);
         const float v = s.candv[o];
-        const float av = L2 ? (float)((double)v + qn) : v;
+        const float av = __fadd_rn(v, qn);
         K[e] = f2ord(av);
         I[e] = s.candi[o];
       }
@@ -416,18 +455,6 @@ __global__ void __launch_bounds__(RT) rerank_kernel(RerankArgs a, int Mp_alloc) 
     }
     if (a.n_cand && tid == 0) atomicAdd(a.n_cand, (unsigned long long)M);
 
-    // boundary of the non-candidates, dist space
-    double bound;        // every non-candidate has approx >= bound (TOPC) / > bound (THRESH)
-    bool bound_strict;   // true: non-candidates are strictly above bound
-    if (s.mode == SCAN_TOPC) {
-      bound = (sT == ~0ull) ? INFINITY : (double)ord2f((unsigned)(sT >> 32));
-      bound_strict = false;
-    } else {
-      const float t = s.thr[q];
-      bound = L2 ? (double)t + qn : (double)t;
-      bound_strict = true;
-    }
-
     if (ex) {
       if (few) {
         unsigned sel = 0;
@@ -455,22 +482,20 @@ __global__ void __launch_bounds__(RT) rerank_kernel(RerankArgs a, int Mp_alloc) 
     }
 
     // ---- 2. band of candidates that can still be in the top k
-    const float ak = ord2f(akey);
-    const double slack = 4e-7 * fabs((double)ak) + 1e-30;
-    const double lim = (double)ak + 2.0 * (double)eps + slack;
+    const float lim = band_limit(ord2f(akey), eps);
     int nband;  // >= k: the candidates up to a_k are inside
     if (few) {
       unsigned sel = 0;
 #pragma unroll
       for (int r = 0; r < RK; r++)
-        if ((cvalid >> r & 1u) && (double)ord2f(ckey[r]) <= lim) sel |= 1u << r;
+        if ((cvalid >> r & 1u) && ord2f(ckey[r]) <= lim) sel |= 1u << r;
       nband = compact(sel);
     } else {
       if (tid == 0) snband = 0;
       __syncthreads();
       int local = 0;
       for (int i = tid; i < M; i += RT)
-        if ((double)ord2f((unsigned)K[i]) <= lim) local++;
+        if (ord2f((unsigned)K[i]) <= lim) local++;
       atomicAdd(&snband, local);
       __syncthreads();
       nband = snband;
@@ -497,11 +522,7 @@ __global__ void __launch_bounds__(RT) rerank_kernel(RerankArgs a, int Mp_alloc) 
 
     // error model of the FP32 re-rank
     const float rho = (float)(d + 4) * kU;
-    float eta = 0.f;
-    if (!L2) {
-      const float B = __uint_as_float(bst->max_norm_bits);
-      eta = (float)(d + 4) * kU * (float)sqrt(fmax(a.qn64 ? a.qn64[q] : 0.0, 0.0)) * B;
-    }
+    const float eta = dot_error(a, q, bst);
     // the k + 1 smallest, and what lies within their error bounds of the last
     // of them (a row further out cannot be among the k nearest), sorted
     int n2 = nband;
@@ -538,7 +559,7 @@ __global__ void __launch_bounds__(RT) rerank_kernel(RerankArgs a, int Mp_alloc) 
       if (e1 - e0 <= tol) sneed64 = 1;
     }
     __syncthreads();
-    double ek_hi;
+    float ekh;  // the k-th exact distance, rounded up
     if (sneed64) {
       const bool finite = (unsigned)K[n2 - 1] <= f2ord(FLT_MAX) && (unsigned)K[0] >= f2ord(-FLT_MAX);
       __syncthreads();
@@ -576,7 +597,8 @@ __global__ void __launch_bounds__(RT) rerank_kernel(RerankArgs a, int Mp_alloc) 
       const unsigned long long u = (kk & 0x8000000000000000ull) ? (kk & 0x7fffffffffffffffull) : ~kk;
       const double ek = __longlong_as_double((long long)u);
       // (pairs of floats: within (d + 16) 2.9e-14 of the value and 1e-6 eta)
-      ek_hi = ek + (1e-12 + (double)(d + 16) * 2.9e-14) * fabs(ek) + 1e-6 * (double)eta + 1e-36;
+      ekh = __double2float_ru(ek + (1e-12 + (double)(d + 16) * 2.9e-14) * fabs(ek) +
+                              1e-6 * (double)eta + 1e-36);
       for (int r = tid; r < k; r += RT) {
         const unsigned long long kr = K[r];
         const unsigned long long ur = (kr & 0x8000000000000000ull) ? (kr & 0x7fffffffffffffffull) : ~kr;
@@ -585,19 +607,18 @@ __global__ void __launch_bounds__(RT) rerank_kernel(RerankArgs a, int Mp_alloc) 
       }
     } else {
       const float ek = ord2f((unsigned)K[k - 1]);
-      ek_hi = (double)ek + (double)rho * fabs((double)ek) + (double)eta;
+      ekh = __fadd_ru(__fadd_ru(ek, __fmul_ru(rho, fabsf(ek))), eta);
       for (int r = tid; r < k; r += RT) {
         oidx[qloc * k + r] = I[r];
         odis[qloc * k + r] = ord2f((unsigned)K[r]);
       }
     }
     // ---- 4. certificate: every non-candidate is provably worse than the k-th
-    const double bslack = 4e-7 * fabs(bound);
-    const double lowest_outside = bound - (double)eps - bslack;
-    const bool ok = bound_strict ? (ek_hi <= lowest_outside) : (ek_hi < lowest_outside);
-    if (ok) return;
+    const bool topc = s.mode == SCAN_TOPC;
+    const float t = topc ? (sT == ~0ull ? INFINITY : ord2f((unsigned)(sT >> 32))) : s.thr[q];
+    if (certified(ekh, t, qn, eps, !topc)) return;
     // widened so that it also bounds a later FP32 re-rank of the same k-th value
-    kth_hi = __double2float_ru(ek_hi + 2.0 * (double)rho * fabs(ek_hi) + 2.0 * (double)eta);
+    kth_hi = __fadd_ru(__fadd_ru(ekh, __fmul_ru(2.f * rho, fabsf(ekh))), 2.f * eta);
     __syncthreads();
   }
 failed:
@@ -731,7 +752,7 @@ __device__ __forceinline__ unsigned rerank_small_query(const RerankArgs &a, int 
   const bool thresh = s.mode == SCAN_THRESH;
   const int k = a.k, d = a.d;
   const bool L2 = a.metric == METRIC_L2;
-  const double qn = L2 ? a.qn64[q] : 0.0;
+  const float qn = query_norm(a, q);
   const float eps = a.eps ? a.eps[q] : 0.f;
   const bool ex = a.qexact ? a.qexact[q] != 0 : false;
   const float *qv = a.q + (long)q * a.ldq;
@@ -749,7 +770,7 @@ __device__ __forceinline__ unsigned rerank_small_query(const RerankArgs &a, int 
       if (sl < cnt && sl < s.cap) {
         const long o = ((long)r * a.nq + q) * s.cap + sl;
         const float v = s.candv[o];
-        key = f2ord(L2 ? (float)((double)v + qn) : v);
+        key = f2ord(__fadd_rn(v, qn));
         id = s.candi[o];
       }
     }
@@ -761,7 +782,7 @@ __device__ __forceinline__ unsigned rerank_small_query(const RerankArgs &a, int 
       const int j = s.topi[o];
       if (j >= 0) {
         const float v = s.topv[o];
-        const float av = L2 ? (float)((double)v + qn) : v;
+        const float av = __fadd_rn(v, qn);
         key = f2ord(av);
         id = j;
         if (sl == s.C - 1) tkey = ((unsigned long long)f2ord(av) << 32) | (unsigned)j;
@@ -796,8 +817,8 @@ __device__ __forceinline__ unsigned rerank_small_query(const RerankArgs &a, int 
       }
     } else {
       const float ak = ord2f((unsigned)__shfl_sync(gm, key, k - 1, G));
-      const double lim = (double)ak + 2.0 * (double)eps + 4e-7 * fabs((double)ak) + 1e-30;
-      const bool inband = id != 0x7fffffff && (double)ord2f((unsigned)key) <= lim;
+      const float lim = band_limit(ak, eps);
+      const bool inband = id != 0x7fffffff && ord2f((unsigned)key) <= lim;
       const int nband = __popc(gballot(inband));
       // FP32 re-rank of the band, two candidates at a time across the group
       float e = INFINITY;
@@ -814,9 +835,7 @@ __device__ __forceinline__ unsigned rerank_small_query(const RerankArgs &a, int 
       if (gl >= nband) id = 0x7fffffff;
       group_sort<G>(key, id, gm);
       const float rho = (float)(d + 4) * kU;
-      float eta = 0.f;
-      if (!L2) eta = (float)(d + 4) * kU * (float)sqrt(fmax(a.qn64[q], 0.0)) *
-                     __uint_as_float(a.bstats->max_norm_bits);
+      const float eta = dot_error(a, q, a.bstats);
       const float e0 = ord2f((unsigned)key);
       const float e1 = ord2f((unsigned)__shfl_down_sync(gm, key, 1, G));
       const bool tie = gl < imin(k, nband - 1) && (e1 - e0 <= rho * (fabsf(e0) + fabsf(e1)) + 2.f * eta);
@@ -852,7 +871,7 @@ __device__ __forceinline__ unsigned rerank_small_query(const RerankArgs &a, int 
           }
         }
       }
-      double ek_hi;
+      float ekh;  // the k-th exact distance, rounded up
       if (need64) {
         // FP64, sequential over coordinates, for the whole band
         unsigned long long k64 = ~0ull;
@@ -860,29 +879,23 @@ __device__ __forceinline__ unsigned rerank_small_query(const RerankArgs &a, int 
         key = k64;
         group_sort<G>(key, id, gm);
         const double ek = ord2d(__shfl_sync(gm, key, k - 1, G));
-        ek_hi = ek + 1e-12 * fabs(ek);
+        ekh = __double2float_ru(ek + 1e-12 * fabs(ek));
         if (gl < k) {
           a.out_idx[(long)q * k + gl] = id;
           a.out_dis[(long)q * k + gl] = (float)ord2d(key);
         }
       } else {
         const float ek = ord2f((unsigned)__shfl_sync(gm, key, k - 1, G));
-        ek_hi = (double)ek + (double)rho * fabs((double)ek) + (double)eta;
+        ekh = __fadd_ru(__fadd_ru(ek, __fmul_ru(rho, fabsf(ek))), eta);
         if (gl < k) {
           a.out_idx[(long)q * k + gl] = id;
           a.out_dis[(long)q * k + gl] = ord2f((unsigned)key);
         }
       }
-      if (thresh) {
-        // every non-candidate has approx > thr, so exact > thr + ||q||^2 - eps
-        const float t = s.thr[q];
-        const double bound = L2 ? (double)t + qn : (double)t;
-        ok = ek_hi <= bound - (double)eps - 4e-7 * fabs(bound);
-      } else {
-        const double bound = tkey == ~0ull ? INFINITY : (double)ord2f((unsigned)(tkey >> 32));
-        ok = ek_hi < bound - (double)eps - 4e-7 * fabs(bound);
-      }
-      kth_hi = __double2float_ru(ek_hi + 2.0 * (double)rho * fabs(ek_hi) + 2.0 * (double)eta);
+      const float t = thresh ? s.thr[q]
+                             : tkey == ~0ull ? INFINITY : ord2f((unsigned)(tkey >> 32));
+      ok = certified(ekh, t, qn, eps, thresh);
+      kth_hi = __fadd_ru(__fadd_ru(ekh, __fmul_ru(2.f * rho, fabsf(ekh))), 2.f * eta);
     }
   }
   if (!ok && thresh && nvalid >= k && kth_hi == INFINITY && a.kth_out) {
@@ -902,9 +915,7 @@ __device__ __forceinline__ unsigned rerank_small_query(const RerankArgs &a, int 
     group_sort<G>(ekey, eid, gm);
     const float ek = ord2f((unsigned)__shfl_sync(gm, ekey, k - 1, G));
     const float rho = (float)(d + 4) * kU;
-    float eta = 0.f;
-    if (!L2) eta = (float)(d + 4) * kU * (float)sqrt(fmax(a.qn64[q], 0.0)) *
-                   __uint_as_float(a.bstats->max_norm_bits);
+    const float eta = dot_error(a, q, a.bstats);
     const double hi = (double)ek + (double)rho * fabs((double)ek) + (double)eta;
     kth_hi = __double2float_ru(hi + 2.0 * (double)rho * fabs(hi) + 2.0 * (double)eta);
   }
@@ -943,7 +954,7 @@ __device__ __forceinline__ unsigned rerank_small_k1(const RerankArgs &a, int q) 
   const bool thresh = s.mode == SCAN_THRESH;
   const int d = a.d;
   const bool L2 = a.metric == METRIC_L2;
-  const double qn = L2 ? a.qn64[q] : 0.0;
+  const float qn = query_norm(a, q);
   const float eps = a.eps ? a.eps[q] : 0.f;
   const bool ex = a.qexact ? a.qexact[q] != 0 : false;
   const float *qv = a.q + (long)q * a.ldq;
@@ -963,7 +974,7 @@ __device__ __forceinline__ unsigned rerank_small_k1(const RerankArgs &a, int q) 
       if (sl < cnt && sl < s.cap) {
         const long o = ((long)r * a.nq + q) * s.cap + sl;
         vraw = s.candv[o];
-        key = f2ord(L2 ? (float)((double)vraw + qn) : vraw);
+        key = f2ord(__fadd_rn(vraw, qn));
         id = s.candi[o];
       }
     }
@@ -976,7 +987,7 @@ __device__ __forceinline__ unsigned rerank_small_k1(const RerankArgs &a, int q) 
       const int j = s.topi[o];
       if (j >= 0) {
         const float v = s.topv[o];
-        const float av = L2 ? (float)((double)v + qn) : v;
+        const float av = __fadd_rn(v, qn);
         key = f2ord(av);
         id = j;
         if (sl == s.C - 1) { tk = key; ti = (unsigned)j; }
@@ -1010,14 +1021,7 @@ __device__ __forceinline__ unsigned rerank_small_k1(const RerankArgs &a, int q) 
       }
     } else {
       const float ak = ord2f(k0);
-      // The band's limit ak + 2 eps + 4e-7 |ak| + 1e-30 in FP32, rounded up,
-      // with larger constants and a relative margin: at least its FP64 value,
-      // so the band holds every row whose exact distance can be the least.
-      // (This part's FP64 pipe runs at 1/64 of the FP32 rate: FP64 is kept
-      // for the keys and the THRESH bound.)
-      float limf = __fadd_ru(__fadd_ru(ak, __fmul_ru(2.f, eps)),
-                             __fadd_ru(__fmul_ru(4.01e-7f, fabsf(ak)), 1.01e-30f));
-      limf = __fadd_ru(limf, __fmul_ru(fabsf(limf), 1.2e-7f));
+      const float limf = band_limit(ak, eps);
       const bool inband = valid && ord2f(key) <= limf;
       const unsigned bmask = gballot(inband);
       const int nband = __popc(bmask);
@@ -1046,9 +1050,7 @@ __device__ __forceinline__ unsigned rerank_small_k1(const RerankArgs &a, int q) 
         group_argmin<G>(r1 ? ek32 : 0xffffffffu, r1 ? eid : 0x7fffffff, gm, e1k, j1);
       }
       const float rho = (float)(d + 4) * kU;
-      float eta = 0.f;
-      if (!L2) eta = (float)(d + 4) * kU * (float)sqrt(fmax(a.qn64[q], 0.0)) *
-                     __uint_as_float(a.bstats->max_norm_bits);
+      const float eta = dot_error(a, q, a.bstats);
       const float e0 = ord2f(e0k), e1 = ord2f(e1k);
       bool need64 = nband > 1 && (e1 - e0 <= rho * (fabsf(e0) + fabsf(e1)) + 2.f * eta);
       unsigned wk = e0k;
@@ -1105,28 +1107,17 @@ __device__ __forceinline__ unsigned rerank_small_k1(const RerankArgs &a, int q) 
           a.out_dis[q] = ekf;
         }
       }
-      // The certificate ek_hi <= bound - eps - 4e-7 |bound| in FP32 with
-      // outward rounding (and 4.01e-7 for the FP64 roundings of the bound): it
-      // holds only where the FP64 form holds, so every query it accepts is
-      // settled; the few it may reject at the edge go to the band pass.
+      // (a running threshold ends at or above the least value plus its slack,
+      // or the threshold it started from)
+      float t = INFINITY;
       if (thresh) {
-        // every non-candidate has approx > thr, so exact > thr + ||q||^2 - eps
-        // (a running threshold ends at or above the least value plus its slack,
-        // or the threshold it started from)
-        float t = s.thr ? s.thr[q] : INFINITY;
+        if (s.thr) t = s.thr[q];
         if (s.run_eps)
           t = fminf(t, __fadd_rd(ord2f(__reduce_min_sync(gm, f2ord(vraw))), run_slack(eps)));
-        float blo = t, babs = fabsf(t);
-        if (L2) {
-          const double bd = (double)t + qn;
-          blo = __double2float_rd(bd);
-          babs = fmaxf(fabsf(blo), fabsf(__double2float_ru(bd)));
-        }
-        ok = ekh <= __fsub_rd(__fsub_rd(blo, eps), __fmul_ru(4.01e-7f, babs));
-      } else {
-        const float b = tkey == ~0ull ? INFINITY : ord2f((unsigned)(tkey >> 32));
-        ok = ekh < __fsub_rd(__fsub_rd(b, eps), __fmul_ru(4.01e-7f, fabsf(b)));
+      } else if (tkey != ~0ull) {
+        t = ord2f((unsigned)(tkey >> 32));
       }
+      ok = certified(ekh, t, qn, eps, thresh);
       if (!ok) {
         // the bound the band pass starts from (as the general form gives it)
         const double ek_hi =
@@ -1156,9 +1147,7 @@ __device__ __forceinline__ unsigned rerank_small_k1(const RerankArgs &a, int q) 
     }
     const float ek = ord2f(__reduce_min_sync(gm, valid ? f2ord(e) : 0xffffffffu));
     const float rho = (float)(d + 4) * kU;
-    float eta = 0.f;
-    if (!L2) eta = (float)(d + 4) * kU * (float)sqrt(fmax(a.qn64[q], 0.0)) *
-                   __uint_as_float(a.bstats->max_norm_bits);
+    const float eta = dot_error(a, q, a.bstats);
     const double hi = (double)ek + (double)rho * fabs((double)ek) + (double)eta;
     kth_hi = __double2float_ru(hi + 2.0 * (double)rho * fabs(hi) + 2.0 * (double)eta);
   }

@@ -110,7 +110,9 @@ __device__ __forceinline__ void softmax_row(float *row, float *out, const float 
 // FUSED: P gets the posteriors, nnz (if not null) the counts of positive
 // ones per component; else P gets the squared distances (k too large for the
 // tile's rows in shared memory; softmax_kernel follows).
-template <int VR, bool FUSED>
+// PAD: a last slice of fewer than ML dimensions, whose padding is not worked
+// through (d = 100: 74 -> 69 us for 20k vectors, k = 100; the test costs others 2 to 8%).
+template <int VR, bool FUSED, bool PAD>
 __global__ void __launch_bounds__(MT, 1)
     posterior_kernel(const float *__restrict__ v, const float *__restrict__ mu,
                      const float *__restrict__ isig, const float *__restrict__ hi,
@@ -168,8 +170,10 @@ __global__ void __launch_bounds__(MT, 1)
     const float *xs = sm + (it & 1) * BUF + (wv * 4 * VR + lv) * MLD;
     const float *ms = sm + (it & 1) * BUF + (VT + wc * 32 + lc) * MLD;
     const float *is = ms + MC * MLD;
+    const int left = d - (it % nl) * ML;
 #pragma unroll
     for (int l = 0; l < ML; l += 4) {
+      if (PAD && l >= left) break;
       float4 x[VR];
 #pragma unroll
       for (int r = 0; r < VR; r++)
@@ -757,8 +761,9 @@ struct GmmDev {
   template <int VR, bool FUSED>
   void launch_posteriors(int *cnt) {
     const size_t smem = maha_floats(VR, FUSED ? k : 0) * sizeof(float);
-    if (ensure_smem((const void *)posterior_kernel<VR, FUSED>, smem) != OK) die(where);
-    posterior_kernel<VR, FUSED><<<(unsigned)((n + 16 * VR - 1) / (16 * VR)), MT, smem,
+    const auto kern = d % ML ? posterior_kernel<VR, FUSED, true> : posterior_kernel<VR, FUSED, false>;
+    if (ensure_smem((const void *)kern, smem) != OK) die(where);
+    kern<<<(unsigned)((n + 16 * VR - 1) / (16 * VR)), MT, smem,
                                   ctx->stream>>>(v.p, mu_dev(), isig.p, dhi.p, dlo.p, n, k, d, P.p,
                                                  cnt);
     launched(where);

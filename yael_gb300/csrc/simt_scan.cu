@@ -23,7 +23,7 @@ namespace {
 // use every bank twice) and arrive by cp.async three deep, which leaves the
 // registers for two CTAs per SM: one computes while the other selects or waits.
 // TM = 8: 1,000 x 100k, d = 100, thresholds: 0.70 ms for 128-row tiles staged in
-// shared memory, one CTA per SM -> 0.59 (39 TFLOP/s); TM = 2 where 128-row tiles would
+// shared memory, one CTA per SM -> 0.52 (39 TFLOP/s); TM = 2 where 128-row tiles would
 // leave SMs without one.
 namespace rows {
 
@@ -70,7 +70,7 @@ __device__ __forceinline__ float merge16(float a, float b, int tx) {
 
 enum Mode : int { FIXED, RUNNING, SAMPLE };
 
-template <int MODE, int TM>
+template <int MODE, int TM, bool PAD>
 __global__ void __launch_bounds__(NT, 2)
     rows_kernel(const float *__restrict__ Q, long ldq, int nq, const float *__restrict__ B,
                 long ldb, int nb, int d, const float *__restrict__ bn, long bn_stride, int metric,
@@ -158,8 +158,10 @@ __global__ void __launch_bounds__(NT, 2)
     const float *As = smem + buf * (BM + BN) * LD + ty * LD;
     const float *Bs = smem + buf * (BM + BN) * LD + (BM + tx) * LD;
     if (++buf == NST) buf = 0;
+    const int kleft = d - kb * BK;
 #pragma unroll
     for (int kk = 0; kk < BK; kk += 4) {
+      if (PAD && kk >= kleft) break;
       float4 a[TM];
 #pragma unroll
       for (int i = 0; i < TM; i++)
@@ -268,28 +270,31 @@ __global__ void __launch_bounds__(NT, 2)
   }
 }
 
-template <int MODE, int TM>
+template <int MODE, int TM, bool PAD>
 int launch(const float *q, long ldq, int nq, const float *b, long ldb, int nb, int d,
            const float *bn, long bn_stride, int metric, const ScanSel &sel, cudaStream_t st) {
   const size_t smem = sizeof(float) * smem_floats<TM>();
-  YG_CHECK(ensure_smem((const void *)rows_kernel<MODE, TM>, smem));
+  YG_CHECK(ensure_smem((const void *)rows_kernel<MODE, TM, PAD>, smem));
   const int vq = (ldq & 3) == 0 && ((uintptr_t)q & 15) == 0;
   const int vb = (ldb & 3) == 0 && ((uintptr_t)b & 15) == 0;
   const dim3 grid((unsigned)ceil_div(nq, 16 * TM), (unsigned)sel.nchunk);
-  rows_kernel<MODE, TM><<<grid, NT, smem, st>>>(q, ldq, nq, b, ldb, nb, d, bn, bn_stride, metric,
-                                                vq, vb, sel);
+  rows_kernel<MODE, TM, PAD><<<grid, NT, smem, st>>>(q, ldq, nq, b, ldb, nb, d, bn, bn_stride,
+                                                     metric, vq, vb, sel);
   YG_LAUNCH_CHECK();
   return OK;
 }
 
-template <int TM>
+// PAD: a last slice of fewer than 16 coordinates, whose padding is not worked
+// through (d = 100: 591 -> 517 us); a kernel of its own, as the test costs the
+// others 2%.
+template <int TM, bool PAD>
 int dispatch(const float *q, long ldq, int nq, const float *b, long ldb, int nb, int d,
              const float *bn, long bn_stride, int metric, const ScanSel &sel, cudaStream_t st) {
   if (sel.mode == SCAN_TOPV)
-    return launch<SAMPLE, TM>(q, ldq, nq, b, ldb, nb, d, bn, bn_stride, metric, sel, st);
+    return launch<SAMPLE, TM, PAD>(q, ldq, nq, b, ldb, nb, d, bn, bn_stride, metric, sel, st);
   if (sel.run_eps)
-    return launch<RUNNING, TM>(q, ldq, nq, b, ldb, nb, d, bn, bn_stride, metric, sel, st);
-  return launch<FIXED, TM>(q, ldq, nq, b, ldb, nb, d, bn, bn_stride, metric, sel, st);
+    return launch<RUNNING, TM, PAD>(q, ldq, nq, b, ldb, nb, d, bn, bn_stride, metric, sel, st);
+  return launch<FIXED, TM, PAD>(q, ldq, nq, b, ldb, nb, d, bn, bn_stride, metric, sel, st);
 }
 
 }  // namespace rows
@@ -412,9 +417,9 @@ int simt_scan(const float *q, long ldq, int nq, const float *b, long ldb, int nb
               cudaStream_t st) {
   if (nq <= 0 || nb <= 0) return OK;
   if (sel.mode != SCAN_TOPC) {
-    if (sel.tile_m == 32)
-      return rows::dispatch<2>(q, ldq, nq, b, ldb, nb, d, bn, bn_stride, metric, sel, st);
-    return rows::dispatch<8>(q, ldq, nq, b, ldb, nb, d, bn, bn_stride, metric, sel, st);
+    const auto f = d % rows::BK ? (sel.tile_m == 32 ? rows::dispatch<2, true> : rows::dispatch<8, true>)
+                                : (sel.tile_m == 32 ? rows::dispatch<2, false> : rows::dispatch<8, false>);
+    return f(q, ldq, nq, b, ldb, nb, d, bn, bn_stride, metric, sel, st);
   }
   switch (sel.C) {
     case 2: return launch<2>(q, ldq, nq, b, ldb, nb, d, bn, bn_stride, metric, sel, st);

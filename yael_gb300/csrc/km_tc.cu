@@ -96,7 +96,6 @@ struct Params {
   const float *v, *C;
   const float2 *tside;         // per unit, per point: (||x'|| rounded up, packing error)
   const float2 *ib;            // per instance: (max centroid norm, max centroid packing error)
-  const SetStats *cs;
   const unsigned char *active;
   int *assign;
   float *dis;
@@ -823,9 +822,10 @@ namespace {
 // a NaN value is never chosen: its distances are NaN) and keeps +inf (an
 // overflowing norm or a row fp16 cannot hold: no usable bound)
 __global__ void inst_bound_kernel(const float *cnorm, const float *cres, int k, float2 *ib) {
+  __shared__ float2 part[8];
   const long r0 = (long)blockIdx.x * k;
   float b = 0.f, e = 0.f;
-  for (int j = threadIdx.x; j < k; j += 32) {
+  for (int j = threadIdx.x; j < k; j += blockDim.x) {
     b = fmaxf(b, sqrtf(cnorm[r0 + j]) * (1.f + 1e-5f));
     e = fmaxf(e, cres[r0 + j]);
   }
@@ -833,7 +833,15 @@ __global__ void inst_bound_kernel(const float *cnorm, const float *cres, int k, 
     b = fmaxf(b, __shfl_xor_sync(0xffffffffu, b, o));
     e = fmaxf(e, __shfl_xor_sync(0xffffffffu, e, o));
   }
-  if (threadIdx.x == 0) ib[blockIdx.x] = make_float2(b, e);
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = make_float2(b, e);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < (int)(blockDim.x >> 5); w++) {
+      b = fmaxf(b, part[w].x);
+      e = fmaxf(e, part[w].y);
+    }
+    ib[blockIdx.x] = make_float2(b, e);
+  }
 }
 }  // namespace
 
@@ -851,7 +859,7 @@ bool km_tc_fuses(int d, int k) { return (size_t)k * d * 8 <= 48 * 1024; }
 
 int km_tc_assign(const KmTcUnit *units, int nunits, const KmTcPoints &P, const float *v, int d,
                  const float *C, int ninst, int k, void *cpk, void *cside, float *cscratch,
-                 float2 *ibound, SetStats *cstats, const unsigned char *active, int *assign,
+                 float2 *ibound, const unsigned char *active, int *assign,
                  float *dis, long long *acc, int *counts, const int *shift, int delta, int *err,
                  cudaStream_t st) {
   using namespace kmtc;
@@ -863,17 +871,16 @@ int km_tc_assign(const KmTcUnit *units, int nunits, const KmTcPoints &P, const f
   const int N = ((k + 31) / 32) * 32, nkb = P.Kp / 64;
   const long ncl = (long)ninst * k;
   // the centroids, packed as the points are (same 16-bit format)
-  YG_CHECK(stats_reset(cstats, st));
   RowShift rs;
   rs.mu = P.mu;
   rs.rows_per_inst = k;
   float *cnorm = cscratch, *cres = cscratch + ncl;
   YG_CHECK(prep_rows(C, d, (int)ncl, d, 1.f, nullptr, cnorm, nullptr, cres,
-                     (__nv_bfloat16 *)cpk, P.Kp, (__nv_bfloat16 *)cside, 1, cstats, st, 8, P.f16,
+                     (__nv_bfloat16 *)cpk, P.Kp, (__nv_bfloat16 *)cside, 1, nullptr, st, 8, P.f16,
                      rs));
   // each instance's own largest centroid norm and packing error: a point is
   // compared with its instance's centroids only, so these bound its errors
-  inst_bound_kernel<<<(unsigned)ninst, 32, 0, st>>>(cnorm, cres, k, ibound);
+  inst_bound_kernel<<<(unsigned)ninst, (unsigned)imin(256, N), 0, st>>>(cnorm, cres, k, ibound);
   YG_LAUNCH_CHECK();
   // the sums go through shared memory when an instance's k x d fit, else
   // straight to the global accumulators; the instance's FP32 centroid rows
@@ -919,7 +926,7 @@ int km_tc_assign(const KmTcUnit *units, int nunits, const KmTcPoints &P, const f
   YG_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
   Params p;
   p.units = units; p.nunits = nunits; p.d = d; p.k = k; p.N = N; p.Kp = P.Kp; p.f16 = P.f16;
-  p.v = v; p.C = C; p.tside = P.tside; p.ib = ibound; p.cs = cstats; p.active = active;
+  p.v = v; p.C = C; p.tside = P.tside; p.ib = ibound; p.active = active;
   p.assign = assign; p.dis = dis; p.acc = acc; p.counts = counts; p.shift = shift; p.err = err;
   p.acc_global = acc_global;
   p.csm = csm;

@@ -37,7 +37,7 @@ enum KmSlot : int {
   KS_BEST_C, KS_BEST_DIS, KS_BEST_ASSIGN, KS_NODE, KS_VSORT, KS_TMP, KS_CPREV,
   KS_AKEYS, KS_AKEYS2, KS_AVALS, KS_AVALS2, KS_AOFFS, KS_ATMP, KS_ASORT,
   // the small-k tensor-core assignment
-  KS_TCU = 160, KS_TCPK, KS_TCSIDE, KS_TCXN, KS_TCXRES, KS_TCCPK, KS_TCCSIDE, KS_TCSTATS,
+  KS_TCU = 160, KS_TCPK, KS_TCSIDE, KS_TCXN, KS_TCXRES, KS_TCCPK, KS_TCCSIDE,
   KS_TCERR, KS_PRIOR, KS_TCMU, KS_TCMUPART, KS_TCSLF, KS_TCNPT, KS_TCHMAX,
   KS_HSTART, KS_HPINST, KS_GCNT, KS_GTOT, KS_TCTSIDE, KS_TCCSCR, KS_TCIB, KS_SPLITROWS,
   KS_SPLITBUF, KS_CUR, KS_MOVED,
@@ -121,8 +121,8 @@ struct Engine {
   bool eager_done = false;
   // the iteration's timing events (ev[1] between assignment and update), and
   // the side stream of a capture with its fork and join
-  cudaEvent_t ev[3] = {}, ev_fork = nullptr, ev_join = nullptr;
-  cudaStream_t side = nullptr;
+  cudaEvent_t ev[3] = {}, ev_fork = nullptr, ev_join = nullptr, ev_timed = nullptr;
+  cudaStream_t side = nullptr, side_timed = nullptr;
   bool capturing = false;
   // One instance whose sums are not fused with its assignment: acc and counts
   // are those of the assignment in cur.  Where the last iteration moved few
@@ -140,7 +140,6 @@ struct Engine {
   int tc_nunits = 0;
   KmTcPoints tcP;
   void *tc_cpk = nullptr, *tc_cside = nullptr;
-  SetStats *tc_cstats = nullptr;
   int *tc_err = nullptr;
   int *ph_err = nullptr;  // pinned copy of tc_err the update graph writes
   bool assign_settled = false;  // the grouped assignment's variant is tuned
@@ -154,9 +153,10 @@ struct Engine {
       if (g_all[i]) cudaGraphExecDestroy(g_all[i]);
       if (g_update[i]) cudaGraphExecDestroy(g_update[i]);
     }
-    for (cudaEvent_t e : {ev[0], ev[1], ev[2], ev_fork, ev_join})
+    for (cudaEvent_t e : {ev[0], ev[1], ev[2], ev_fork, ev_join, ev_timed})
       if (e) cudaEventDestroy(e);
-    if (side) cudaStreamDestroy(side);
+    for (cudaStream_t s : {side, side_timed})
+      if (s) cudaStreamDestroy(s);
   }
 
   // body(stream) beside what follows on st until join(): on the side stream
@@ -195,6 +195,8 @@ struct Engine {
   bool capture(F body, cudaGraphExec_t *exec, long *nlaunch) {
     const long l0 = launch_count();
     if (!side && (cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking) != cudaSuccess ||
+                  cudaStreamCreateWithFlags(&side_timed, cudaStreamNonBlocking) != cudaSuccess ||
+                  cudaEventCreateWithFlags(&ev_timed, cudaEventDisableTiming) != cudaSuccess ||
                   cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming) != cudaSuccess ||
                   cudaEventCreateWithFlags(&ev_join, cudaEventDisableTiming) != cudaSuccess)) {
       (void)cudaGetLastError();
@@ -363,7 +365,6 @@ struct Engine {
     YG_CHECK(ws_get(ws, KS_TCXRES, (size_t)ntot, &tcP.xres));
     YG_CHECK(ws_get(ws, KS_TCCPK, (size_t)ncl * tcP.Kp, &cpk));
     YG_CHECK(ws_get(ws, KS_TCCSIDE, (size_t)ncl * 16, &cside));
-    YG_CHECK(ws_get(ws, KS_TCSTATS, 1, &tc_cstats));
     YG_CHECK(ws_get(ws, KS_TCERR, 1, &tc_err));
     YG_CUDA(cudaMemsetAsync(tc_err, 0, sizeof(int), st));
     tcP.pk = pk;
@@ -473,7 +474,7 @@ struct Engine {
       YG_CHECK(ws_get(ctx->ws, KS_TCCSCR, (size_t)ncl * 2, &cscr));
       YG_CHECK(ws_get(ctx->ws, KS_TCIB, in.size(), &ib));
       return km_tc_assign(tc_units, tc_nunits, tcP, v, d, C, (int)in.size(), k, tc_cpk,
-                          tc_cside, cscr, ib, tc_cstats, active, assign, dis,
+                          tc_cside, cscr, ib, active, assign, dis,
                           tc_fuse ? acc : nullptr, tc_fuse ? counts : nullptr, shift, delta,
                           tc_err, st);
     }
@@ -632,11 +633,17 @@ struct Engine {
     const bool graph_assign =
         use_graphs && assign_graph_wanted() && assign_settled && !(tc_fuse && !tc_live);
     if (graph_assign) {
-      // (one graph, one launch: the event between the two is a node of it)
+      // (one graph, one launch: the event between the two is a node of it, on a
+      // branch of its own, as what follows it in line starts 5 us later)
       auto all = [&]() -> int {
         YG_CHECK(assign_step());
-        YG_CUDA(cudaEventRecordWithFlags(e1, st, cudaEventRecordExternal));
-        return update_body();
+        YG_CUDA(cudaEventRecord(ev_fork, st));
+        YG_CUDA(cudaStreamWaitEvent(side_timed, ev_fork, 0));
+        YG_CUDA(cudaEventRecordWithFlags(e1, side_timed, cudaEventRecordExternal));
+        YG_CUDA(cudaEventRecord(ev_timed, side_timed));
+        YG_CHECK(update_body());
+        YG_CUDA(cudaStreamWaitEvent(st, ev_timed, 0));
+        return OK;
       };
       if (!g_all[delta] && !capture(all, &g_all[delta], &g_all_n[delta])) graphs_failed = true;
     } else if (use_graphs && !g_update[delta] &&

@@ -556,15 +556,6 @@ __global__ void __launch_bounds__(PW * 32)
 }
 }  // namespace
 
-__global__ void stats_reset_kernel(SetStats *stats) { *stats = SetStats{0u, 0u, 1, 0, 0u}; }
-
-// a kernel, not a copy from a host variable: it may be captured in a CUDA graph
-int stats_reset(SetStats *stats, cudaStream_t st) {
-  stats_reset_kernel<<<1, 1, 0, st>>>(stats);
-  YG_LAUNCH_CHECK();
-  return OK;
-}
-
 int prep_rows(const float *x, long ld, int n, int d, float scale, double *norm64,
               float *norm32, unsigned char *flags, float *resid,
               __nv_bfloat16 *packed_bf, int Kp, __nv_bfloat16 *normpart_bf,

@@ -75,6 +75,4 @@ int prep_group(const GroupPair *pairs, int np, long brows, int nq, int d, int Kp
                __nv_bfloat16 *qnorm, double *qn64, unsigned char *qflag, float *qres, int *qpair,
                cudaStream_t st);
 
-int stats_reset(SetStats *stats, cudaStream_t st);
-
 }  // namespace yg

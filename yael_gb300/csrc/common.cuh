@@ -93,14 +93,12 @@ constexpr size_t kPinnedStatusBytes = 4096;
 // the context's pinned status buffer: small device -> host reads stay async
 int ctx_pinned_status(Ctx *c, void **out);
 
-// pinned slots 3 and 4: the staging pieces of copy_to_host
-constexpr int kPinnedStageSlot = 3;
 // Device -> host copy into caller memory, complete on return (the stream is
-// synchronised): pinned or registered memory directly, pageable memory
-// through two 4 MB pinned pieces of the context (the copy of one piece runs
-// while the host copies the previous one out), several times faster than the
-// driver's own staging of a pageable destination.
-int copy_to_host(Ctx *c, cudaStream_t st, void *dst, const void *src, size_t bytes);
+// synchronised).  Pageable memory too is one copy of the driver's, which the GPU
+// writes in place on this host: gmm_compute_p with a result of 1 MB takes 95 us,
+// of 256 MB 3.8 ms (10.6 into pages not touched before), where two 4 MB pinned
+// pieces and a memcpy by the calling thread took 155 us and 20.6 ms (24.0).
+int copy_to_host(cudaStream_t st, void *dst, const void *src, size_t bytes);
 
 // Host -> device copy on st.  Up to 64 KB goes through the context's pinned
 // slot and is queued like a kernel (the slot may be used again only after st has

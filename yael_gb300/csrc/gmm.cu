@@ -704,7 +704,7 @@ struct GmmDev {
                               cudaMemcpyHostToDevice, ctx->stream));
   }
   void download_P(float *hp) {
-    if (copy_to_host(ctx, ctx->stream, hp, P.p, sizeof(float) * (size_t)(n * k)) != OK) die(where);
+    if (copy_to_host(ctx->stream, hp, P.p, sizeof(float) * (size_t)(n * k)) != OK) die(where);
   }
 
   // the mixture on the device (one copy from pinned memory; the caller
@@ -861,7 +861,7 @@ struct GmmDev {
     fisher_kernel<<<(unsigned)((t + 127) / 128), 128, 0, ctx->stream>>>(
         sum.p, w_dev(), mu_dev(), sigma_dev(), n, k, d, flags, fv.get(ctx, where, m));
     launched(where);
-    if (copy_to_host(ctx, ctx->stream, out, fv.p, sizeof(float) * (size_t)m) != OK) die(where);
+    if (copy_to_host(ctx->stream, out, fv.p, sizeof(float) * (size_t)m) != OK) die(where);
   }
   size_t gmm_len(int flags) const {
     const gmm_t g{d, k, nullptr, nullptr, nullptr};

@@ -786,9 +786,9 @@ struct Engine {
 };
 
 // D2H of whichever outputs are requested (device or host destinations)
-int copy_out(Ctx *ctx, cudaStream_t st, void *dst, const void *src, size_t bytes, bool dev) {
+int copy_out(cudaStream_t st, void *dst, const void *src, size_t bytes, bool dev) {
   if (!dst || bytes == 0) return OK;
-  if (!dev) return copy_to_host(ctx, st, dst, src, bytes);
+  if (!dev) return copy_to_host(st, dst, src, bytes);
   YG_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToDevice, st));
   return OK;
 }
@@ -977,9 +977,9 @@ int kmeans_run(int d, int n, int k, int niter, const float *v_in, int flags, lon
     printf("Unbalanced factor of last iteration: %g\n", uf * k / (tot * tot));
   }
   if (best < HUGE_VAL && bC) {
-    YG_CHECK(copy_out(ctx, st, C_out, bC, sizeof(float) * (size_t)k * d, dev));
-    YG_CHECK(copy_out(ctx, st, dis_out, bdis, sizeof(float) * (size_t)n, dev));
-    YG_CHECK(copy_out(ctx, st, assign_out, bassign, sizeof(int) * (size_t)n, dev));
+    YG_CHECK(copy_out(st, C_out, bC, sizeof(float) * (size_t)k * d, dev));
+    YG_CHECK(copy_out(st, dis_out, bdis, sizeof(float) * (size_t)n, dev));
+    YG_CHECK(copy_out(st, assign_out, bassign, sizeof(int) * (size_t)n, dev));
     if (nassign_out) {
       YG_CUDA(cudaMemcpyAsync(nassign_out, bnassign.data(), sizeof(int) * k,
                               dev ? cudaMemcpyHostToDevice : cudaMemcpyHostToHost, st));
@@ -1102,7 +1102,7 @@ int hkm_run(int n, int d, int nlevel, int bf, const float *points, int niter, bo
     // centroids of this level, then node = node * bf + child
     node_update_kernel<<<(unsigned)ceil_div(n, 256), 256, 0, st>>>(sorted, E.assign, n, bf, node);
     YG_LAUNCH_CHECK();
-    YG_CHECK(copy_to_host(ctx, st, levels_out[l], E.C, sizeof(float) * (size_t)k * bf * d));
+    YG_CHECK(copy_to_host(st, levels_out[l], E.C, sizeof(float) * (size_t)k * bf * d));
     if (trace_enabled())
       fprintf(stderr, "[yael_gpu] hkm level %d: %ld nodes, set-up %.3f ms (grouping %.3f, engine "
               "%.3f, init %.3f), iterations %.3f ms, wrap-up %.3f ms (host clock)\n", l, k,
@@ -1114,7 +1114,7 @@ int hkm_run(int n, int d, int nlevel, int bf, const float *points, int niter, bo
   if (ms_out) cudaEventElapsedTime(ms_out, t0, t1);
   cudaEventDestroy(t0);
   cudaEventDestroy(t1);
-  if (assign_out) YG_CHECK(copy_to_host(ctx, st, assign_out, node, sizeof(int) * (size_t)n));
+  if (assign_out) YG_CHECK(copy_to_host(st, assign_out, node, sizeof(int) * (size_t)n));
   if (iters_out) *iters_out = iters;
   stats.instance_iterations = iters;
   g_last_stats = stats;

@@ -324,6 +324,27 @@ def test_host_upload_in_parts(k):
     np.testing.assert_allclose(dis, rdis, rtol=2e-6, atol=1e-5)
 
 
+@pytest.mark.parametrize("nq,nb,d", [(1, 300, 16), (130, 20_000, 128), (20_000, 5000, 33)])
+def test_fp32_nearest_first_pass(nq, nb, d):
+    """k = 1 in FP32, settled by the first pass: rows whose exact distances tie
+    by the hundred (more than a region holds), and unit rows, whose distances
+    and dot products carry a rounding as large as the pass's."""
+    rng = np.random.default_rng(nb)
+    c = rng.integers(0, 9, (17, d)).astype(np.float32)
+    b, q = c[rng.integers(0, 17, nb)], c[rng.integers(0, 17, nq)]
+    st = assert_exact(b, q, 1, "fp32")
+    assert st["exact_class"] == 1 and st["n_band"] == 0 and st["n_fallback"] == 0
+    b = rng.standard_normal((nb, d)).astype(np.float32)
+    q = rng.standard_normal((nq, d)).astype(np.float32)
+    b /= np.linalg.norm(b, axis=1, keepdims=True)
+    q /= np.linalg.norm(q, axis=1, keepdims=True)
+    assert assert_exact(b, q, 1, "fp32")["n_band"] == 0
+    idx, _, st = gpu_knn(b, q, 1, "fp32", dt=16)
+    dots = q.astype(np.float64) @ b.astype(np.float64).T
+    np.testing.assert_array_equal(idx[:, 0], np.argmin(dots, axis=1))
+    assert st["n_band"] == 0 and st["n_fallback"] == 0
+
+
 @pytest.mark.parametrize("prec", ["bf16", "fp16", "bf16x3"])
 @pytest.mark.parametrize("nq,nb", [(19_500, 200), (20_001, 287), (40_000, 1031), (77_900, 2049),
                                    (20_000, 4099), (80_000, 3900)])

@@ -397,12 +397,13 @@ int knn_batch(KnnJob &job, Ctx *ctx, cudaStream_t st, Small *dsmall, BaseOps *bo
     sel.halves = bf16 ? 2 : 1;
     sel.tile_m = tile_m;
     sel.run_eps = eps;
+    sel.run_scale = bf16 ? 1.f : 2.f;
     const int nchunk = tune_chunks(TuneKey{4, job.prec, nqt, ntb, 0}, rc,
                                    bf16 ? imax(1, imin(4, ntb / 4)) : imin(1024, ntb),
                                    ctx->num_sms * ctas_per_sm, &scan_ticket);
     sel.tiles_per_chunk = (int)ceil_div(ntb, nchunk);
     sel.nchunk = (int)ceil_div(ntb, sel.tiles_per_chunk);
-    sel.cap = bf16 ? running_cap(sel.nchunk) : 8;
+    sel.cap = bf16 ? running_cap(sel.nchunk) : sel.nchunk <= 4 ? 8 : 16;
     const long nr = sel.nregion();
     YG_CHECK(ws_get(ws, WS_CNT, (size_t)nr * nq, &sel.cnt));
     YG_CHECK(ws_get(ws, WS_TOPV, (size_t)nr * nq * sel.cap, &sel.candv));
@@ -733,13 +734,13 @@ int knn_batches(KnnJob &job, Ctx *ctx, cudaStream_t st, Small *dsmall, BaseOps *
     const int C = pow2_at_least(cn);
     size_t per_query;
     if (!bf16) {
-      // running thresholds: 8 slots a region; else the regions' share of the
+      // running thresholds: up to 16 slots a region; else the regions' share of the
       // candidates, or the whole base where it is too short for a sample
       const int m = simt_tile_m(nq, nb, ctx->num_sms), nt = (int)ceil_div(nq, m);
       const int nch = imin(imin(1024, ntb), 3 * choose_chunks(nt, ntb, ctx->num_sms, 2, 1) + 2);
       const SamplePlan plan(k, nb, false);
       const double er = (double)plan.c * plan.stride / nch;
-      const size_t cap = k == 1 ? 8
+      const size_t cap = k == 1 ? 16
                          : plan.usable(nb)
                              ? pow2_at_least((int)(2.0 * er + 6.0 * sqrt(er) + 16.0))
                              : 2 * (size_t)ceil_div(nb, nch) + 2 * tile_n;

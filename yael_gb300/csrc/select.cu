@@ -1113,7 +1113,8 @@ __device__ __forceinline__ unsigned rerank_small_k1(const RerankArgs &a, int q) 
       if (thresh) {
         if (s.thr) t = s.thr[q];
         if (s.run_eps)
-          t = fminf(t, __fadd_rd(ord2f(__reduce_min_sync(gm, f2ord(vraw))), run_slack(eps)));
+          t = fminf(t, __fadd_rd(ord2f(__reduce_min_sync(gm, f2ord(vraw))),
+                                 s.run_scale * run_slack(eps)));
       } else if (tkey != ~0ull) {
         t = ord2f((unsigned)(tkey >> 32));
       }

@@ -94,7 +94,7 @@ __global__ void __launch_bounds__(NT, 2)
     if (MODE == FIXED) Thr[r] = ok ? sel.thr[q0 + r] : NAN;
     if (MODE == RUNNING) {
       Thr[r] = ok ? INFINITY : -INFINITY;
-      Slk[r] = ok ? run_slack(sel.run_eps[q0 + r]) : 0.f;
+      Slk[r] = ok ? sel.run_scale * run_slack(sel.run_eps[q0 + r]) : 0.f;
     }
     Cnt[r] = 0;
   }
@@ -264,7 +264,9 @@ __global__ void __launch_bounds__(NT, 2)
     if (MODE == SAMPLE) {
       sel.topv[o * 16 + tx] = lst[i];
     } else if (tx == 0) {
-      sel.cnt[o] = Cnt[row];
+      // (no slack: the candidates tie, and the first has the least id.  Rows
+      // that tie by the hundred, 20k x 5,000: 44.8 ms -> 0.8)
+      sel.cnt[o] = MODE == RUNNING && Slk[row] == 0.f ? min(Cnt[row], 1) : Cnt[row];
       if (MODE == RUNNING && sel.run_thr) sel.run_thr[o] = __fadd_ru(Thr[row], Slk[row]);
     }
   }

@@ -504,8 +504,10 @@ int knn_batch(KnnJob &job, Ctx *ctx, cudaStream_t st, Small *dsmall, BaseOps *bo
       // every row whose exact distance can be <= the known bound; the thresholds
       // run on from there (fewer candidates, so fewer regions that overflow:
       // 2M x 16,384, second iteration: 28,720 points rejected -> none, re-rank
-      // 1.53 -> 0.98 ms)
-      if (sel.nchunk <= 4) {
+      // 1.53 -> 0.98 ms).  Not over a few tiles, the first four of which would be
+      // read twice (60k x 1,000, crowded: 0.057 ms a pass as given, 0.098 running,
+      // whose regions are half the size and reject 5% of the points).
+      if (sel.nchunk <= 4 && sel.tiles_per_chunk > 16) {
         sel.run_eps = eps;
         sel.cap = running_cap(sel.nchunk);
       } else {

@@ -418,3 +418,31 @@ def test_fp32_row_tiles(nq, nb, d, k):
     idx, _, _ = gpu_knn(b, q, k, "fp32", dt=16)
     dots = q.astype(np.float64) @ b.astype(np.float64).T
     np.testing.assert_array_equal(idx, np.argsort(dots, axis=1, kind="stable")[:, :k])
+
+
+def fp64_order(q, b, k, dt=2):
+    """The k smallest (FP64 distance, id), NaN never selected: ids, -1 past the
+    rows that have a distance; k = 1: none that FP32 does not hold (yael/nn.c:404-407)."""
+    q64, b64 = q.astype(np.float64), b.astype(np.float64)
+    with np.errstate(all="ignore"):
+        full = q64 @ b64.T if dt == 16 else ((q64[:, None] - b64[None]) ** 2).sum(2)
+    key = np.where(np.isnan(full), np.inf, full)
+    ids = np.broadcast_to(np.arange(len(b)), full.shape)
+    order = np.lexsort((ids, key, np.isnan(full)), axis=1)[:, :k]
+    got = np.take_along_axis(full, order, 1)
+    bad = ~(got < 3.4e38) if k == 1 else np.isnan(got)
+    return np.where(bad, -1, order)
+
+
+@pytest.mark.parametrize("prec", ["fp16", "bf16x3"])
+@pytest.mark.parametrize("nb,k", [(24, 20), (6, 1), (3000, 8), (3000, 30)])
+def test_dot_product_infinite_rows(nb, k, prec):
+    """Inner products with infinite rows: -inf where the 16-bit operands give NaN
+    (a query value that is zero in fp16, the low part of an infinity)."""
+    rng = np.random.default_rng(nb + k)
+    b = rng.standard_normal((nb, 8)).astype(np.float32)
+    q = (1 + rng.random((40, 8))).astype(np.float32)
+    q[:, 5] = 1e-9
+    b[nb // 2, 5], b[nb // 3, 2], b[nb - 1, 5] = -np.inf, np.inf, -np.inf
+    idx, _, _ = gpu_knn(b, q, k, prec, dt=16)
+    np.testing.assert_array_equal(idx, fp64_order(q, b, k, 16))

@@ -1231,7 +1231,10 @@ __global__ void eps_kernel(int nq, int d, int prec, int metric, const double *qn
   // fp16 norm parts: their sum is within 2^-25 of ||b||^2
   if (prec == PREC_FP16) e += u;
   e = e * (1.1f * 1.000005f) + 1.001e-30f;
-  eps[q] = isfinite(e) ? e : INFINITY;
+  // (0 x inf: where a query's value is zero in fp16, an infinite row's inner
+  // product is NaN here and may be -inf)
+  const bool lost = prec == PREC_FP16 && metric == METRIC_DOT && bs->n_nan > 0;
+  eps[q] = isfinite(e) && !lost ? e : INFINITY;
 }
 
 __global__ void eps_split_kernel(int nq, int d, int metric, const double *qn64, const float *qlo,
@@ -1258,7 +1261,9 @@ __global__ void eps_split_kernel(int nq, int d, int metric, const double *qn64, 
   const double acc = Kt * 2 * u * ((L2 ? 2 : 1) * qn * B * 1.02 + (L2 ? 1.001 * B * B : 0.0));
   double e = (L2 ? 2 * dot + u * B * B : dot) + acc + un * (qn * qn + B * B);
   e = e * 1.1 + 1e-30;
-  eps[q] = isfinite(e) ? (float)e : INFINITY;
+  // (inf - inf: an infinite row's low part is NaN, its inner product may be -inf)
+  const bool lost = metric == METRIC_DOT && bs->n_nan > 0;
+  eps[q] = isfinite(e) && !lost ? (float)e : INFINITY;
 }
 
 // One warp per query (a serial merge by one thread spends a dependent load on

@@ -172,3 +172,25 @@ def test_grouped_batch_many_waves(pipeline):
     r = subprocess.run([sys.executable, "-c", code], cwd=root, env=env, capture_output=True,
                        text=True, timeout=300)
     assert r.returncode == 0 and "waves ok" in r.stdout, r.stdout + r.stderr
+
+
+def test_grouped_batch_not_finite():
+    """Pairs in which every row is a candidate, with infinite coordinates of either
+    sign, and with squared distances past FP32's range: FP64 order."""
+    torch = pytest.importorskip("torch")
+    k = 20
+    rng = np.random.default_rng(31)
+    pairs = unit_pairs(32, [(30, 24), (30, 24), (30, 24)], 16)
+    q0 = np.abs(pairs[0][0]) + np.float32(0.1)
+    b0 = pairs[0][1].copy()
+    rows = np.sort(rng.permutation(24)[:6])
+    b0[rows, np.arange(6)] = np.where(np.arange(6) % 2, -np.inf, np.inf)
+    pairs[0] = (q0, b0)
+    u = pairs[1][0][:1]
+    pairs[1] = ((1.6e19 * u * (1 + 1e-2 * rng.random((30, 1)))).astype(np.float32),
+                (-0.6e19 * u * rng.uniform(0.9, 1.1, (24, 1))).astype(np.float32))
+    out, o = _device_batch(pairs, k, 2, torch)
+    for (q, b), (idx, _) in zip(pairs, out):
+        full = ((q.astype(np.float64)[:, None] - b.astype(np.float64)[None]) ** 2).sum(2)
+        order = np.lexsort((np.broadcast_to(np.arange(24), full.shape), full), axis=1)[:, :k]
+        np.testing.assert_array_equal(idx, order)

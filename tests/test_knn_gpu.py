@@ -446,3 +446,39 @@ def test_dot_product_infinite_rows(nb, k, prec):
     b[nb // 2, 5], b[nb // 3, 2], b[nb - 1, 5] = -np.inf, np.inf, -np.inf
     idx, _, _ = gpu_knn(b, q, k, prec, dt=16)
     np.testing.assert_array_equal(idx, fp64_order(q, b, k, 16))
+
+
+@pytest.mark.parametrize("dt", [2, 16])
+@pytest.mark.parametrize("prec", ["fp32", "bf16", "fp16", "bf16x3"])
+@pytest.mark.parametrize("nb,inf,k", [(10, 2, 9), (10, 2, 10), (24, 6, 20), (24, 0, 20), (10, 0, 9),
+                                      (1, 1, 1), (6, 5, 1), (600, 595, 8), (300, 290, 20)])
+def test_short_bases_infinite_rows(nb, inf, k, prec, dt):
+    """Bases in which every row is a candidate, with rows that have infinite
+    coordinates of either sign: (distance, id) order up to and past the
+    finite rows; a finite base needs no later pass."""
+    rng = np.random.default_rng(nb + k)
+    b = rng.standard_normal((nb, 8)).astype(np.float32)
+    q = (1 + rng.random((40, 8))).astype(np.float32)
+    rows = np.sort(rng.permutation(nb)[:inf])
+    b[rows, rng.integers(0, 8, inf)] = np.where(np.arange(inf) % 2, -np.inf, np.inf)
+    q[:, 5] = 1e-9                # nothing in fp16, where it meets an infinity as 0 x inf
+    idx, _, st = gpu_knn(b, q, k, prec, dt=dt)
+    np.testing.assert_array_equal(idx, fp64_order(q, b, k, dt))
+    if inf == 0:
+        assert st["n_band"] == 0 and st["n_fallback"] == 0
+
+
+@pytest.mark.parametrize("prec", ["fp32", "bf16", "fp16", "bf16x3"])
+@pytest.mark.parametrize("nb,near,k", [(7, 0, 1), (7, 0, 5), (24, 0, 20), (600, 3, 8), (200, 7, 20)])
+def test_short_bases_overflowing_distances(nb, near, k, prec):
+    """Finite rows and queries whose norms are finite in FP32 and whose squared
+    distances are not (1.6e19 against 0.6e19 the other way): ids in FP64 order,
+    also where the list of a chunk is full of overflowed values."""
+    rng = np.random.default_rng(nb)
+    u = rng.standard_normal(8)
+    u /= np.linalg.norm(u)
+    q = (1.6e19 * u * (1 + 1e-2 * rng.random((20, 1)))).astype(np.float32)
+    b = (-0.6e19 * u * rng.uniform(0.9, 1.1, (nb, 1))).astype(np.float32)
+    b[rng.permutation(nb)[:near]] *= -1
+    idx, _, _ = gpu_knn(b, q, k, prec)
+    np.testing.assert_array_equal(idx, fp64_order(q, b, k))

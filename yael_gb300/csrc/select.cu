@@ -144,10 +144,17 @@ __device__ __forceinline__ float band_limit(float ak, float eps) {
 // rounding (and 4.01e-7 for the roundings of the bound): it holds only where
 // the exact form holds.  ekh: the k-th exact distance rounded up; t: the
 // value below which (THRESH: up to which, without ||q||^2) every row is a
-// candidate.  Without one (t = +inf: every row is, or no list was full) nothing
-// lies outside; an infinite eps certifies nothing.
-__device__ __forceinline__ bool certified(float ekh, float t, float qn, float eps, bool thresh) {
-  if (t == INFINITY) return eps < INFINITY;
+// candidate.  all: no list was full (TOPC) or the threshold is +inf (THRESH), so
+// that only rows whose value is NaN are no candidates.  With a finite eps those
+// have an infinite coordinate, and an exact squared distance of +inf or NaN, so
+// a finite ekh is below them all; an infinite one (FP32 overflow, an infinite
+// row) is settled in FP64 by the later passes.  (An inner product may be
+// -inf: no such short cut where a row is not finite.)  An infinite eps certifies
+// nothing.
+__device__ __forceinline__ bool certified(float ekh, float t, bool all, float qn, float eps,
+                                          const RerankArgs &a, const SetStats *bs) {
+  const bool thresh = a.sel.mode == SCAN_THRESH;
+  if (all && (a.metric == METRIC_L2 || bs->n_nan == 0)) return eps < INFINITY && ekh < INFINITY;
   float blo = t, babs = fabsf(t);
   if (thresh) {
     blo = __fadd_rd(t, qn);
@@ -557,7 +564,7 @@ __global__ void __launch_bounds__(RT) rerank_kernel(RerankArgs a, int Mp_alloc) 
     for (int i = tid; i < lastpair; i += RT) {
       const float e0 = ord2f((unsigned)K[i]), e1 = ord2f((unsigned)K[i + 1]);
       const float tol = rho * (fabsf(e0) + fabsf(e1)) + 2.f * eta;
-      if (e1 - e0 <= tol) sneed64 = 1;
+      if (!(e1 - e0 > tol)) sneed64 = 1;  // (also where both overflowed)
     }
     __syncthreads();
     float ekh;  // the k-th exact distance, rounded up
@@ -616,8 +623,8 @@ __global__ void __launch_bounds__(RT) rerank_kernel(RerankArgs a, int Mp_alloc) 
     }
     // ---- 4. certificate: every non-candidate is provably worse than the k-th
     const bool topc = s.mode == SCAN_TOPC;
-    const float t = topc ? (sT == ~0ull ? INFINITY : ord2f((unsigned)(sT >> 32))) : s.thr[q];
-    if (certified(ekh, t, qn, eps, !topc)) return;
+    const float t = topc ? ord2f((unsigned)(sT >> 32)) : s.thr[q];
+    if (certified(ekh, t, topc ? sT == ~0ull : t == INFINITY, qn, eps, a, bst)) return;
     // widened so that it also bounds a later FP32 re-rank of the same k-th value
     kth_hi = __fadd_ru(__fadd_ru(ekh, __fmul_ru(2.f * rho, fabsf(ekh))), 2.f * eta);
     __syncthreads();
@@ -839,7 +846,7 @@ __device__ __forceinline__ unsigned rerank_small_query(const RerankArgs &a, int 
       const float eta = dot_error(a, q, a.bstats);
       const float e0 = ord2f((unsigned)key);
       const float e1 = ord2f((unsigned)__shfl_down_sync(gm, key, 1, G));
-      const bool tie = gl < imin(k, nband - 1) && (e1 - e0 <= rho * (fabsf(e0) + fabsf(e1)) + 2.f * eta);
+      const bool tie = gl < imin(k, nband - 1) && !(e1 - e0 > rho * (fabsf(e0) + fabsf(e1)) + 2.f * eta);
       bool need64 = __any_sync(gm, tie);
       if (need64 && k == 1 && L2) {
         // A near tie of the best two alone (the third, if any, clearly worse
@@ -893,9 +900,8 @@ __device__ __forceinline__ unsigned rerank_small_query(const RerankArgs &a, int 
           a.out_dis[(long)q * k + gl] = ord2f((unsigned)key);
         }
       }
-      const float t = thresh ? s.thr[q]
-                             : tkey == ~0ull ? INFINITY : ord2f((unsigned)(tkey >> 32));
-      ok = certified(ekh, t, qn, eps, thresh);
+      const float t = thresh ? s.thr[q] : ord2f((unsigned)(tkey >> 32));
+      ok = certified(ekh, t, thresh ? t == INFINITY : tkey == ~0ull, qn, eps, a, a.bstats);
       kth_hi = __fadd_ru(__fadd_ru(ekh, __fmul_ru(2.f * rho, fabsf(ekh))), 2.f * eta);
     }
   }
@@ -1053,7 +1059,7 @@ __device__ __forceinline__ unsigned rerank_small_k1(const RerankArgs &a, int q) 
       const float rho = (float)(d + 4) * kU;
       const float eta = dot_error(a, q, a.bstats);
       const float e0 = ord2f(e0k), e1 = ord2f(e1k);
-      bool need64 = nband > 1 && (e1 - e0 <= rho * (fabsf(e0) + fabsf(e1)) + 2.f * eta);
+      bool need64 = nband > 1 && !(e1 - e0 > rho * (fabsf(e0) + fabsf(e1)) + 2.f * eta);
       unsigned wk = e0k;
       int wj = j0;
       if (need64 && L2) {
@@ -1116,10 +1122,10 @@ __device__ __forceinline__ unsigned rerank_small_k1(const RerankArgs &a, int q) 
         if (s.run_eps)
           t = fminf(t, __fadd_rd(ord2f(__reduce_min_sync(gm, f2ord(vraw))),
                                  s.run_scale * run_slack(eps)));
-      } else if (tkey != ~0ull) {
+      } else {
         t = ord2f((unsigned)(tkey >> 32));
       }
-      ok = certified(ekh, t, qn, eps, thresh);
+      ok = certified(ekh, t, thresh ? t == INFINITY : tkey == ~0ull, qn, eps, a, a.bstats);
       if (!ok) {
         // the bound the band pass starts from (as the general form gives it)
         const double ek_hi =

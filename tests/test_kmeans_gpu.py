@@ -318,6 +318,30 @@ def test_hkm_chosen_form_vs_oracle(prec, monkeypatch):
     assert st.point_iterations >= st.instance_iterations > 0
 
 
+@pytest.mark.parametrize("d,bf,scale", [(160, 256, 1.0), (160, 256, 300.0), (192, 225, 1.0),
+                                        (256, 128, 300.0)])
+def test_hkm_widest_shapes_vs_oracle(d, bf, scale, monkeypatch):
+    """Trees at the largest shapes that the tensor-core assignment takes, on fp16
+    and (values past fp16's range) on bf16 operands: the oracle's tree, bit for
+    bit."""
+    monkeypatch.setenv("YAEL_GPU_PRECISION", "bf16")
+    rng = np.random.default_rng(31)
+    n, nl = 40000, 2
+    v = rng.standard_normal((2000, d))[rng.integers(0, 2000, n)] + 0.5 * rng.standard_normal((n, d))
+    v = (v * scale).astype(np.float32)
+    cent = np.zeros(sum(bf ** (l + 1) for l in range(nl)) * d, np.float32)
+    oa = np.empty(n, np.int32)
+    srand48(5)
+    assert oracle().orc_hkm_learn(n, d, nl, bf, ptr(v), 2, ptr(cent), ptr(oa), 1 | 0x100) == 0
+    srand48(5)
+    levels, ga = yg.hkm(v, nl, bf, 2, small_nodes=True)
+    np.testing.assert_array_equal(ga, oa)
+    np.testing.assert_array_equal(np.concatenate([l.ravel() for l in levels]), cent)
+    st = yg.CallStats()
+    yg.lib().yael_gpu_last_stats(ctypes.byref(st))
+    assert st.prec_used == (3 if scale == 1.0 else 1)
+
+
 @pytest.mark.parametrize("prec", ["bf16", "fp32"])
 def test_hkm_small_nodes_vs_oracle(prec, monkeypatch):
     """Nodes with fewer points than bf (small_nodes = 1: one child per point,

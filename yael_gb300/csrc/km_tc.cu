@@ -47,47 +47,9 @@ namespace yg {
 namespace kmtc {
 using namespace ptx;
 
-constexpr int NDEC = 16;              // decision warps
 constexpr int PPW = 128 / NDEC;       // points per decision warp
 constexpr int LPP = 32 / PPW;         // lanes per point
 constexpr int NT = (6 + NDEC) * 32;
-constexpr int PAIRS = 64;             // (point, member) pairs listed per decision warp
-// band mask words per point (odd: no bank conflicts)
-__host__ __device__ constexpr int band_words(int N) { return (N >> 5) | 1; }
-constexpr int A_BLK = 128 * 128;  // 128 rows x 64 16-bit columns
-constexpr int A_SIDE = 128 * 32;  // 128 rows x 16 16-bit columns
-
-struct Lay {
-  int nkb, N, S, fuse, csm, xs;
-  size_t stage_bytes, x_off, ts_off, b_off, bside_off, cf_off, band_off, lst_off, pair_off, acc_off, cnt_off,
-      bar_off, total;
-};
-
-// xs: every stage also holds the tile's FP32 point rows (128 x d floats)
-__host__ __device__ inline Lay make_lay(int nkb, int N, int S, int fuse, int k, int d,
-                                       int csm, int xs) {
-  Lay L;
-  L.nkb = nkb; L.N = N; L.S = S; L.fuse = fuse; L.csm = csm; L.xs = xs;
-  size_t off = 0;
-  L.x_off = (size_t)nkb * A_BLK + A_SIDE;
-  // the tile's per-point norm and packing error (128 x float2) after its rows
-  L.ts_off = L.x_off + (xs ? (((size_t)128 * d * 4 + 1023) & ~(size_t)1023) : 0);
-  L.stage_bytes = L.ts_off + 1024;
-  off += (size_t)S * L.stage_bytes;
-  L.b_off = off;     off += (size_t)nkb * N * 128;  // N % 32 == 0: 1024-aligned blocks
-  L.bside_off = off; off += (size_t)N * 32;
-  L.cf_off = off;    off += csm ? (size_t)N * d * 4 : 0;  // FP32 centroid rows (d % 4 == 0)
-  L.band_off = off;  off += (size_t)2 * 128 * band_words(N) * 4;
-  L.lst_off = off;   off += (size_t)256 * 4;  // the tile's moves: new and old centroids
-  L.pair_off = off;  off += (size_t)NDEC * PAIRS * 8;  // pairs, then their distances
-  off = (off + 15) & ~(size_t)15;
-  L.acc_off = off;   off += fuse ? (size_t)k * d * 8 : 0;
-  L.cnt_off = off;   off += fuse ? (size_t)k * 4 : 0;
-  off = (off + 15) & ~(size_t)15;
-  L.bar_off = off;   off += (size_t)(2 * S + 12) * 8 + 16;
-  L.total = off + 1024;  // alignment slack of the 1024-byte aligned base
-  return L;
-}
 
 struct Params {
   const KmTcUnit *units;
@@ -107,6 +69,7 @@ struct Params {
                                // for shared memory)
   int csm;                     // the instance's FP32 centroid rows staged in shared memory
   int xs;                      // the tile's FP32 point rows staged with it
+  int pairs;                   // (point, member) pairs listed per decision warp
   int centered;                // the packed rows are translated by the instance's mean
   int delta;                   // the sums hold the previous assignment's: only moves are added
   unsigned long long wait_ns;  // bound of every wait (0: kWaitLimitNs)
@@ -245,8 +208,8 @@ __device__ __forceinline__ void phase_b_decide(const Params &P, const unsigned *
   const int total = __shfl_sync(0xffffffffu, end, 31);
   const int mmax = (int)__reduce_max_sync(0xffffffffu, (unsigned)nm);
   // (staged centroid rows: a round saved pays the list from two on)
-  if (total <= PAIRS && mmax > (total + PPW - 1) / PPW + (CSM ? 1 : 0)) {
-    float *dist = reinterpret_cast<float *>(pairs + PAIRS);
+  if (total <= P.pairs && mmax > (total + PPW - 1) / PPW + (CSM ? 1 : 0)) {
+    float *dist = reinterpret_cast<float *>(pairs + P.pairs);
     if (h == 0)
       for (int t = end - nm; t < end; t++) pairs[t] = p << 8 | next();
     __syncwarp();
@@ -431,7 +394,7 @@ __global__ void __launch_bounds__(NT, 1)
   const int nkb = P.Kp / 64, N = P.N, k = P.k, d = P.d;
   const bool fuse = P.acc != nullptr;
   const bool sfuse = fuse && !P.acc_global;  // shared-memory sums
-  const Lay lay = make_lay(nkb, N, S, sfuse ? 1 : 0, k, d, P.csm, P.xs);
+  const Lay lay = make_lay(nkb, N, S, sfuse ? 1 : 0, k, d, P.csm, P.xs, P.pairs);
   uint8_t *Stg = base;
   uint8_t *Bs = base + lay.b_off;
   uint8_t *Bside = base + lay.bside_off;
@@ -680,7 +643,7 @@ __global__ void __launch_bounds__(NT, 1)
   } else {
     // ---------------- decision
     const int ew = warp - 6, dt = threadIdx.x - 192;
-    int *pairs = reinterpret_cast<int *>(base + lay.pair_off) + ew * 2 * PAIRS;
+    int *pairs = reinterpret_cast<int *>(base + lay.pair_off) + ew * 2 * P.pairs;
     const float rho = (float)(d + 4) * 5.9604645e-08f;
     // the shared sums of an instance to the global ones.  All decision warps
     // come here for each of their instances, also after a wait that gave up
@@ -846,13 +809,8 @@ __global__ void inst_bound_kernel(const float *cnorm, const float *cres, int k, 
 }  // namespace
 
 bool km_tc_supported(int d, int k, const float *v, const float *C) {
-  if (!(d >= 4 && d % 4 == 0 && d <= 256 && k >= 1 && k <= kTcMaxK &&
-        (reinterpret_cast<uintptr_t>(v) & 15) == 0 && (reinterpret_cast<uintptr_t>(C) & 15) == 0))
-    return false;
-  // a ring of two stages beside the centroid tile, without staging or
-  // shared-memory sums, must fit (not so for d > 128 with k > 224)
-  const int Kp = ((d + 63) / 64) * 64, N = ((k + 31) / 32) * 32;
-  return kmtc::make_lay(Kp / 64, N, 2, 0, k, d, 0, 0).total <= 227 * 1024;
+  return kmtc::shape_ok(d, k) && (reinterpret_cast<uintptr_t>(v) & 15) == 0 &&
+         (reinterpret_cast<uintptr_t>(C) & 15) == 0;
 }
 
 bool km_tc_fuses(int d, int k) { return (size_t)k * d * 8 <= 48 * 1024; }
@@ -884,26 +842,9 @@ int km_tc_assign(const KmTcUnit *units, int nunits, const KmTcPoints &P, const f
   YG_LAUNCH_CHECK();
   // the sums go through shared memory when an instance's k x d fit, else
   // straight to the global accumulators; the instance's FP32 centroid rows
-  // are staged when they are few.  Both give way, staging first, when a ring
-  // of two stages would not fit beside them.
-  int acc_global = acc != nullptr && !km_tc_fuses(d, k);
-  int fuse = acc != nullptr && !acc_global;
-  int csm = (size_t)N * d * 4 <= 32 * 1024;
-  int xs = 1;
-  auto fits = [&](int S_) {
-    return make_lay(nkb, N, S_, fuse, k, d, csm, xs).total <= 227 * 1024;
-  };
-  // the tile's FP32 rows are staged when two stages still fit with them
-  if (!fits(2)) xs = 0;
-  if (!fits(2)) csm = 0;
-  if (!fits(2) && fuse) {
-    fuse = 0;
-    acc_global = 1;
-  }
-  int S = 6;
-  while (S > 2 && !fits(S)) S--;
-  const Lay lay = make_lay(nkb, N, S, fuse, k, d, csm, xs);
-  if (lay.total > 227 * 1024) {
+  // are staged when they are few
+  const Lay lay = choose_lay(d, k, acc != nullptr && km_tc_fuses(d, k));
+  if (lay.total > kSmemMax) {
     set_error(E_UNSUPPORTED, "km_tc_assign: shared memory %zu too large (d=%d k=%d)", lay.total,
               d, k);
     return E_UNSUPPORTED;
@@ -919,7 +860,7 @@ int km_tc_assign(const KmTcUnit *units, int nunits, const KmTcPoints &P, const f
   YG_CHECK(tck::make_map(&mB, cpk, P.Kp, ncl, (uint64_t)P.Kp * 2, 64, (uint32_t)N,
                          CU_TENSOR_MAP_SWIZZLE_128B));
   YG_CHECK(tck::make_map(&mBs, cside, 16, ncl, 32, 16, (uint32_t)N, CU_TENSOR_MAP_SWIZZLE_32B));
-  if (csm) YG_CHECK(make_map_f32(&mC, C, d, ncl, (uint32_t)d, (uint32_t)N));
+  if (lay.csm) YG_CHECK(make_map_f32(&mC, C, d, ncl, (uint32_t)d, (uint32_t)N));
   else mC = mBs;
   int dev = 0, nsm = 0;
   YG_CUDA(cudaGetDevice(&dev));
@@ -928,15 +869,16 @@ int km_tc_assign(const KmTcUnit *units, int nunits, const KmTcPoints &P, const f
   p.units = units; p.nunits = nunits; p.d = d; p.k = k; p.N = N; p.Kp = P.Kp; p.f16 = P.f16;
   p.v = v; p.C = C; p.tside = P.tside; p.ib = ibound; p.active = active;
   p.assign = assign; p.dis = dis; p.acc = acc; p.counts = counts; p.shift = shift; p.err = err;
-  p.acc_global = acc_global;
-  p.csm = csm;
-  p.xs = xs;
+  p.acc_global = acc != nullptr && !lay.fuse;
+  p.csm = lay.csm;
+  p.xs = lay.xs;
+  p.pairs = lay.pairs;
   p.centered = P.mu != nullptr;
   p.delta = acc != nullptr && delta ? 1 : 0;
   p.wait_ns = wait_limit_ns();
   p.withhold = test_withhold_loads() ? 1 : 0;
   const unsigned g = (unsigned)(nunits < nsm ? nunits : nsm);
-  kern<<<g, NT, lay.total, st>>>(mA, mAs, mB, mBs, mC, S, p);
+  kern<<<g, NT, lay.total, st>>>(mA, mAs, mB, mBs, mC, lay.S, p);
   YG_LAUNCH_CHECK();
   return OK;
 }

@@ -5,6 +5,7 @@
 // array; global cluster id = i*k + local id.
 #pragma once
 #include "common.cuh"
+#include "km_tc_lay.h"
 #include "prep.cuh"
 
 namespace yg {
@@ -71,7 +72,6 @@ struct KmTcUnit {
   int np;   // points in the tile
   long p0;  // first point (global index)
 };
-constexpr int kTcMaxK = 256;
 
 // The points of a run (or of an hkm level) packed once: 16-bit -2x in
 // [n][Kp] with a [n][16] side block of ones (the norm fold), ||x||^2 in FP64
@@ -96,7 +96,8 @@ struct KmTcPoints {
 int km_tc_tile_side(const KmTcUnit *units, int nunits, const double *xn64, const float *xres,
                     float2 *tside, cudaStream_t st);
 
-// shapes the kernel takes: d % 4 == 0, d <= 256, k <= 256, 16-byte aligned rows
+// shapes the kernel takes (kmtc::shape_ok: whole float4 rows, d <= 192 with k <= 256,
+// d <= 256 with k <= 128), 16-byte aligned rows
 bool km_tc_supported(int d, int k, const float *v, const float *C);
 
 // Nearest centroid of every point of the listed units, exact: the tensor

@@ -482,3 +482,19 @@ def test_short_bases_overflowing_distances(nb, near, k, prec):
     b[rng.permutation(nb)[:near]] *= -1
     idx, _, _ = gpu_knn(b, q, k, prec)
     np.testing.assert_array_equal(idx, fp64_order(q, b, k))
+
+
+@pytest.mark.parametrize("prec", ["fp32", "bf16", "fp16"])
+@pytest.mark.parametrize("k", [1, 5])
+@pytest.mark.parametrize("nq,nb,copies", [(1, 5000, 20), (3, 100_000, 17), (3, 100_000, 300),
+                                          (40, 30_000, 100), (200, 9000, 300)])
+def test_copies_of_a_row_need_no_exhaustive_pass(nq, nb, copies, k, prec):
+    """Real-valued rows, one of them repeated side by side more often than a
+    candidate region holds, next to every query: settled by the band passes."""
+    rng = np.random.default_rng(nb + copies)
+    b = rng.standard_normal((nb, 24)).astype(np.float32)
+    r = nb // 3
+    b[r:r + copies] = b[r]
+    q = (b[r] + 0.05 * rng.standard_normal((nq, 24))).astype(np.float32)
+    st = assert_exact(b, q, k, prec)
+    assert st["n_fallback"] == 0

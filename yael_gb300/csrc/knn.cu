@@ -218,9 +218,16 @@ int scan(const KnnJob &job, const float *q, int nq, const float *b, long ldb, in
 
 // Candidate layout of a band pass over nq queries: chunks of the base and the
 // per-region capacity.  A band holds every base row whose exact distance can
-// still be <= the query's k-th; ctot bounds its size (more fails the query).
+// still be <= the query's k-th; slots bounds its size (more fails the query).
+// Its rows may lie together (copies of a row, a base in some order), so a
+// region has room for all of them where that is within kRoomBytes.
+constexpr size_t kRoomBytes = (size_t)256 << 20;
+int room_cap(int cap, long want, int nq, int nregion) {
+  while (cap < want && (size_t)nq * nregion * 2 * cap * 8 <= kRoomBytes) cap *= 2;
+  return cap;
+}
 struct BandLayout {
-  int nchunk, tiles_per_chunk, cap, halves;
+  int nchunk, tiles_per_chunk, cap, halves, slots;
   size_t bytes_per_query() const {
     return (size_t)nchunk * halves * cap * 8 + (size_t)nchunk * halves * 4 + 64;
   }
@@ -234,7 +241,10 @@ BandLayout band_layout(int nq, int nb, int k, int tile_m, int tile_n, int halves
   L.tiles_per_chunk = (int)ceil_div(ntb, L.nchunk);
   L.nchunk = (int)ceil_div(ntb, L.tiles_per_chunk);
   const int ctot = imin(kMaxCandidates / 2, imax(512, 4 * k));
-  L.cap = pow2_at_least(imax(8, 2 * ctot / (halves * L.nchunk)));
+  const int nreg = halves * L.nchunk;
+  L.cap = pow2_at_least(imax(8, 2 * ctot / nreg));
+  L.slots = nreg * L.cap;
+  L.cap = room_cap(L.cap, imin(ctot, L.tiles_per_chunk * tile_n), nq, nreg);
   return L;
 }
 
@@ -499,6 +509,7 @@ int knn_batch(KnnJob &job, Ctx *ctx, cudaStream_t st, Small *dsmall, BaseOps *bo
       sel.nchunk = L.nchunk;
       sel.tiles_per_chunk = L.tiles_per_chunk;
       sel.cap = L.cap;
+      ra.m_max = L.slots;
       YG_CHECK(band_thresholds(nq, job.metric, job.band_kth, qn64, eps, thr, st));
     } else if (prior) {
       // every row whose exact distance can be <= the known bound; the thresholds

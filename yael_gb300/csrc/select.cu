@@ -630,6 +630,13 @@ __global__ void __launch_bounds__(RT) rerank_kernel(RerankArgs a, int Mp_alloc) 
     __syncthreads();
   }
 failed:
+  // a region, or all of them together, had more candidates than room: at least k
+  // rows lie at or below the threshold, so their k-th exact distance does within eps
+  // (4e-7: the roundings of the value)
+  if (s.mode == SCAN_THRESH && (sfail || M > Mp_alloc) && M >= k) {
+    const float b = __fadd_ru(s.thr[q], qn);
+    kth_hi = __fadd_ru(__fadd_ru(b, eps), __fmul_ru(4.01e-7f, fabsf(b)));
+  }
   // fewer than k rows below the sample's threshold: no bound of the k-th was
   // found, so the band pass starts from the sample's value of twice the rank
   if (a.sample_topv && M < k && !sfail && tid < 32) {
@@ -1503,6 +1510,7 @@ int rerank(const RerankArgs &a, cudaStream_t st) {
   int Mmax = a.sel.mode == SCAN_TOPC ? a.sel.nchunk * a.sel.C : a.sel.nregion() * a.sel.cap;
   if (a.sel.mode == SCAN_THRESH && a.m_expect > 0 && Mmax > 4 * a.m_expect + 64)
     Mmax = 4 * a.m_expect + 64;
+  if (a.m_max > 0) Mmax = imin(Mmax, a.m_max);
   if (a.gpairs) Mmax = a.max_candidates;  // grouped: sized by the caller over all pairs
   if (Mmax < a.k) Mmax = a.k;
   if (Mmax > kMaxCandidates) Mmax = kMaxCandidates;  // more candidates than this fail the query

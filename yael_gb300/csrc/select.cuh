@@ -43,6 +43,7 @@ struct RerankArgs {
   // sized for a few times this rather than for every region's capacity, and a
   // query with more candidates fails its certificate (the band pass follows)
   int m_expect = 0;
+  int m_max = 0;                 // THRESH: and for no more than this (0: no limit)
   // THRESH with thresholds from a sample: its lists and rank, from which a
   // query with fewer than k candidates gets the bound its band pass starts from
   const float *sample_topv = nullptr;

@@ -541,8 +541,12 @@ int knn_batch(KnnJob &job, Ctx *ctx, cudaStream_t st, Small *dsmall, BaseOps *bo
       ra.m_expect = (int)(c * per);
       // (under half a hit expected in 32 rows x 32 columns)
       sel.queue = 1024.0 * c * per < 0.5 * nb;
-      const double er = c * per / nreg;  // expected hits per region
-      sel.cap = pow2_at_least((int)(2.0 * er + 6.0 * sqrt(er) + 16.0));
+      // hits per region: the expected ones of rows in any order, or all of them in
+      // one (a base in the order of its norms)
+      auto room = [](double e) { return (int)(2.0 * e + 6.0 * sqrt(e) + 16.0); };
+      sel.cap = pow2_at_least(room(c * per / nreg));
+      ra.m_max = nreg * sel.cap;
+      sel.cap = room_cap(sel.cap, room(c * per), nq, nreg);
       ScanSel ss;
       ss.mode = SCAN_TOPV;  // only the c-th value is needed
       ss.C = 16;

@@ -520,3 +520,19 @@ def test_bases_in_norm_order(nq, nb, d, k, order, prec):
     # (a query whose sample has fewer than its share of the near rows may need a
     # band pass: 2e-5 of them)
     assert st["n_band"] <= 2 and st["n_second"] == 0 and st["n_fallback"] == 0
+
+
+@pytest.mark.parametrize("k", [2, 5, 10, 16, 17])
+@pytest.mark.parametrize("nq,nb", [(1, 60_000), (300, 60_000), (2000, 9000)])
+def test_fp32_copies_of_integer_rows(nq, nb, k):
+    """A base of copies of 17 integer rows: thousands of rows tie with the k-th,
+    and the least ids are the answer.  Up to 16 neighbours need no exhaustive
+    pass in FP32."""
+    rng = np.random.default_rng(nb)
+    c = rng.integers(0, 9, (17, 20)).astype(np.float32)
+    b, q = c[rng.integers(0, 17, nb)], c[rng.integers(0, 17, nq)]
+    st = assert_exact(b, q, k, "fp32")
+    assert st["exact_class"] == 1
+    assert k > 16 or st["n_fallback"] == 0
+    # queries that are not integers: no value is exact
+    assert_exact(b, (q[:8] + 0.25).astype(np.float32), k, "fp32")

@@ -365,10 +365,10 @@ int knn_batch(KnnJob &job, Ctx *ctx, cudaStream_t st, Small *dsmall, BaseOps *bo
 
   const bool timed = job.timing || trace_enabled();
   const int tile_n = bf16 ? TC_TILE_N : SIMT_TILE_N;
-  const int tile_m = bf16 ? TC_TILE_M : simt_tile_m(nq, nb, ctx->num_sms);
+  const int tile_m = bf16 ? TC_TILE_M : job.lists ? 128 : simt_tile_m(nq, nb, ctx->num_sms);
   const int nqt = (int)ceil_div(nq, tile_m);
   const int ntb = (int)ceil_div(nb, tile_n);
-  const int ctas_per_sm = bf16 ? 1 : 2;
+  const int ctas_per_sm = bf16 || job.lists ? 1 : 2;
   // (few CTAs in all: single tiles, so that every SM has some)
   const int min_tiles = bf16 || (long)nqt * ntb > 8L * ctx->num_sms ? 4 : 1;
   // oversampling for inexact distances: the certificate needs a margin between
@@ -437,7 +437,7 @@ int knn_batch(KnnJob &job, Ctx *ctx, cudaStream_t st, Small *dsmall, BaseOps *bo
       sel.run_eps = nullptr;
     }
     job.scan_launches++;
-  } else if (bf16 && !band && !prior && c_needed <= 16) {
+  } else if ((bf16 || job.lists) && !band && !prior && c_needed <= 16) {
     // ---- TOPC over the full base (register lists)
     sel.mode = SCAN_TOPC;
     sel.C = pow2_at_least(c_needed);
@@ -658,6 +658,11 @@ int knn_batch(KnnJob &job, Ctx *ctx, cudaStream_t st, Small *dsmall, BaseOps *bo
   // rejections (bands too wide for its candidate buffers) go to a band pass on
   // the 3xBF16 split operands, whose error bound and so whose band is ~2^-8 of
   // the BF16 one; everything else to the exhaustive FP64 path.
+  // A base of the exact class with up to 16 neighbours in FP32 takes lists of them
+  // first: 1,500 queries x 60k rows that are copies of 17, d = 128, k = 10: 152 ms by
+  // the band and the exhaustive pass, 1.9 with lists (1.1 with nothing before them).
+  const bool to_lists =
+      !bf16 && !band && !job.lists && k > 1 && k <= 16 && hs.bs.all_exact && job.w == nullptr;
   const bool to_band = !band && job.w == nullptr;
   const bool to_split =
       band && (job.prec == PREC_BF16 || job.prec == PREC_FP16) && job.w == nullptr;
@@ -689,7 +694,8 @@ int knn_batch(KnnJob &job, Ctx *ctx, cudaStream_t st, Small *dsmall, BaseOps *bo
     }
     KnnJob sub = job;
     sub.prec = to_split ? PREC_BF16X3 : job.prec;
-    sub.band_kth = ckth;
+    sub.band_kth = to_lists ? nullptr : ckth;
+    sub.lists = to_lists;
     sub.prior_kth = nullptr;
     sub.level = job.level + 1;
     sub.nq = nf;
@@ -698,7 +704,7 @@ int knn_batch(KnnJob &job, Ctx *ctx, cudaStream_t st, Small *dsmall, BaseOps *bo
     sub.out_idx = cidx;
     sub.out_dis = cdis;
     sub.timing = 0;
-    YG_CHECK(knn_batches(sub, ctx, st, dsmall, bops, bstats_exact));
+    YG_CHECK(knn_batches(sub, ctx, st, dsmall, bops, to_lists ? 1 : bstats_exact));
     scatter_rows_kernel<<<(unsigned)ceil_div((long)nf * k, 256), 256, 0, st>>>(cidx, cdis, map, nf,
                                                                              k, job.out_idx,
                                                                              job.out_dis);
@@ -750,7 +756,7 @@ int knn_batches(KnnJob &job, Ctx *ctx, cudaStream_t st, Small *dsmall, BaseOps *
     const int nqt = (int)ceil_div(nq, tile_m), ntb = (int)ceil_div(nb, tile_n);
     const int C = pow2_at_least(cn);
     size_t per_query;
-    if (!bf16) {
+    if (!bf16 && !job.lists) {
       // running thresholds: up to 16 slots a region; else the regions' share of the
       // candidates, or the whole base where it is too short for a sample
       const int m = simt_tile_m(nq, nb, ctx->num_sms), nt = (int)ceil_div(nq, m);

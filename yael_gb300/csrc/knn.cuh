@@ -39,6 +39,10 @@ struct KnnJob {
   // THRESH pass with thresholds from these bounds (no sample pass; short
   // candidate regions, whose overflow sends the query to the band pass).
   const float *prior_kth = nullptr;
+  // FP32 lists instead of thresholds (internal), for queries that thresholds
+  // rejected over a base of the exact class: rows whose distances tie by the
+  // hundred overflow the candidate regions, and lists keep the least ids of them
+  int lists = 0;
   int level = 0;  // nesting depth of the later-chance passes (workspace slots)
   BaseUpload *upload = nullptr;  // base arriving part by part (BF16 pass only)
   // CUDA-event timing of the passes (optional)

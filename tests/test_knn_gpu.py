@@ -536,3 +536,22 @@ def test_fp32_copies_of_integer_rows(nq, nb, k):
     assert k > 16 or st["n_fallback"] == 0
     # queries that are not integers: no value is exact
     assert_exact(b, (q[:8] + 0.25).astype(np.float32), k, "fp32")
+
+
+def test_tile_heights_are_tuned_apart():
+    """FP32 passes over 32-row and over 128-row query tiles with the same number of
+    tiles (256 and 1,024 queries: eight) choose their chunk counts by themselves (child
+    process: the trace is switched on by the environment)."""
+    import subprocess
+    import sys
+    code = (
+        "import numpy as np, yael_gb300 as yg;"
+        "rng = np.random.default_rng(7);"
+        "b = rng.standard_normal((5120, 16)).astype(np.float32);"
+        "q = rng.standard_normal((1024, 16)).astype(np.float32);"
+        "[yg.knn(q[:n], b, nnn=1, precision='fp32') for n in (256, 1024) for _ in range(6)]")
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True,
+                       env=dict(os.environ, YAEL_GPU_TRACE="1"), timeout=300)
+    assert r.returncode == 0, r.stderr
+    assert r.stderr.count("autotune kind=4 key=(8,40,") == 2, r.stderr[-2000:]

@@ -16,7 +16,8 @@ bool TuneKey::operator<(const TuneKey &o) const {
   if (prec != o.prec) return prec < o.prec;
   if (nqt != o.nqt) return nqt < o.nqt;
   if (ntb != o.ntb) return ntb < o.ntb;
-  return C < o.C;
+  if (C != o.C) return C < o.C;
+  return form < o.form;
 }
 
 namespace {
@@ -156,8 +157,8 @@ void tune_report(int ticket, float ms) {
   if (trace_enabled()) {
     for (const auto &kv : g_index) {
       if (kv.second != ticket / 4) continue;
-      fprintf(stderr, "[yael_gpu] autotune kind=%d key=(%d,%d,%d): candidate %d (", kv.first.kind,
-              kv.first.nqt, kv.first.ntb, kv.first.C, e.cand[b]);
+      fprintf(stderr, "[yael_gpu] autotune kind=%d key=(%d,%d,%d,%d): candidate %d (",
+              kv.first.kind, kv.first.nqt, kv.first.ntb, kv.first.C, kv.first.form, e.cand[b]);
       for (int i = 0; i < e.n; i++) fprintf(stderr, "%s%d: %.3f ms", i ? ", " : "", e.cand[i], e.ms[i]);
       fprintf(stderr, ")\n");
     }

@@ -20,8 +20,12 @@ struct TuneKey {
   int nqt;    // query tiles
   int ntb;    // base tiles
   int C;      // list length
+  int form = 0;  // what else sets a launch's cost: FP32 rows per query tile, 1 for a
+                 // sample of block minima (sample_form)
   bool operator<(const TuneKey &o) const;
 };
+
+inline int sample_form(int tile_m, bool blockmin) { return 2 * tile_m + (blockmin ? 1 : 0); }
 
 // The chunk count for this call, in [1, cmax].  *ticket >= 0 marks a trial
 // whose pass time must be reported with tune_report().

@@ -408,7 +408,7 @@ int knn_batch(KnnJob &job, Ctx *ctx, cudaStream_t st, Small *dsmall, BaseOps *bo
     sel.tile_m = tile_m;
     sel.run_eps = eps;
     sel.run_scale = bf16 ? 1.f : 2.f;
-    const int nchunk = tune_chunks(TuneKey{4, job.prec, nqt, ntb, 0}, rc,
+    const int nchunk = tune_chunks(TuneKey{4, job.prec, nqt, ntb, 0, tile_m}, rc,
                                    bf16 ? imax(1, imin(4, ntb / 4)) : imin(1024, ntb),
                                    ctx->num_sms * ctas_per_sm, &scan_ticket);
     sel.tiles_per_chunk = (int)ceil_div(ntb, nchunk);
@@ -481,7 +481,7 @@ int knn_batch(KnnJob &job, Ctx *ctx, cudaStream_t st, Small *dsmall, BaseOps *bo
     } else {
       sel.nchunk = band    ? 1
                    : prior ? choose_chunks(nqt, ntb, ctx->num_sms, ctas_per_sm, 4)
-                           : tune_chunks(TuneKey{1, job.prec, nqt, ntb, 0},
+                           : tune_chunks(TuneKey{1, job.prec, nqt, ntb, 0, tile_m},
                                          choose_chunks(nqt, ntb, ctx->num_sms, ctas_per_sm,
                                                        min_tiles),
                                          1024, ctx->num_sms * ctas_per_sm, &scan_ticket);
@@ -553,7 +553,7 @@ int knn_batch(KnnJob &job, Ctx *ctx, cudaStream_t st, Small *dsmall, BaseOps *bo
       ss.tile_m = tile_m;
       ss.blockmin = blockmin ? 1 : 0;
       const int nts = (int)ceil_div(sns, tile_n);
-      int nch = tune_chunks(TuneKey{2, job.prec, nqt, nts, ss.C},
+      int nch = tune_chunks(TuneKey{2, job.prec, nqt, nts, ss.C, sample_form(tile_m, blockmin)},
                                   choose_chunks(nqt, nts, ctx->num_sms, ctas_per_sm,
                                                 imin(2, min_tiles)), 64,
                                   ctx->num_sms * ctas_per_sm, &sample_ticket);

@@ -555,3 +555,15 @@ def test_tile_heights_are_tuned_apart():
                        env=dict(os.environ, YAEL_GPU_TRACE="1"), timeout=300)
     assert r.returncode == 0, r.stderr
     assert r.stderr.count("autotune kind=4 key=(8,40,") == 2, r.stderr[-2000:]
+
+
+@pytest.mark.parametrize("prec", PRECS)
+@pytest.mark.parametrize("nq,nb", [(300, 5000), (20_000, 5000), (40, 30_000), (7, 257)])
+def test_nearest_among_copies_of_integer_rows(nq, nb, prec):
+    """k = 1, exact values, hundreds of rows that tie with the nearest: the least
+    id, from short and from long candidate lists and from thresholds."""
+    rng = np.random.default_rng(nq)
+    c = rng.integers(0, 9, (17, 33)).astype(np.float32)
+    b, q = c[rng.integers(0, 17, nb)], c[rng.integers(0, 17, nq)]
+    st = assert_exact(b, q, 1, prec)
+    assert st["exact_class"] == 1 and st["n_band"] == 0 and st["n_fallback"] == 0

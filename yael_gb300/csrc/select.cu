@@ -464,7 +464,24 @@ __global__ void __launch_bounds__(RT) rerank_kernel(RerankArgs a, int Mp_alloc) 
     if (a.n_cand && tid == 0) atomicAdd(a.n_cand, (unsigned long long)M);
 
     if (ex) {
-      if (few) {
+      if (few && k == 1) {
+        // the least id of the least value: nothing to sort (40 candidates that
+        // tie, 20k x 5,000 copies of 17 rows: 160 us sorted, 82 reduced)
+        unsigned mi = 0x7fffffffu;
+#pragma unroll
+        for (int r = 0; r < RK; r++)
+          if ((cvalid >> r & 1u) && ckey[r] == akey) mi = min(mi, (unsigned)cid[r]);
+        mi = __reduce_min_sync(0xffffffffu, mi);
+        if (tid == 0) scount = 0x7fffffff;
+        __syncthreads();
+        if ((tid & 31) == 0) atomicMin(&scount, (int)mi);
+        __syncthreads();
+        if (tid == 0) {
+          K[0] = akey;
+          I[0] = scount;
+        }
+        __syncthreads();
+      } else if (few) {
         unsigned sel = 0;
 #pragma unroll
         for (int r = 0; r < RK; r++)

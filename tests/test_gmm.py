@@ -374,3 +374,74 @@ def test_gpu_moments_non_finite():
     np.testing.assert_array_equal(np.isinf(got), np.isinf(exp))
     fin = np.isfinite(exp)
     close(got[fin], exp[fin].astype(np.float64), FV_RTOL, FV_ATOL)
+
+
+def moments_32_64(p, v):
+    """sum p, sum p x and sum p x^2 as float sums over steps of 32 vectors and FP64
+    sums over the steps."""
+    n = len(p)
+    s0, s1, s2 = 0.0, 0.0, 0.0
+    with np.errstate(all="ignore"):
+        v2 = v * v
+        for i in range(0, n, 32):
+            a, x, x2 = p[i:i + 32], v[i:i + 32], v2[i:i + 32]
+            s0 = s0 + a.astype(np.float64).sum(0)
+            s1 = s1 + (a[:, :, None] * x[:, None]).sum(0, dtype=np.float32).astype(np.float64)
+            s2 = s2 + (a[:, :, None] * x2[:, None]).sum(0, dtype=np.float32).astype(np.float64)
+    return s0[:, None], s1, s2
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,d,k", [(3000, 70, 2), (20_000, 128, 40), (700, 33, 5)])
+@pytest.mark.parametrize("big", [2.0 ** 33, 2.0 ** 35, 1e17, 1e20])
+def test_gpu_moments_large_values(n, d, k, big):
+    """Values whose squares, or whose sums of squares, leave FP32's range, first met
+    part of the way through the vectors: the moments are those of FP64 sums over
+    steps of 32, finite, infinite or NaN entry by entry."""
+    L_ = bind(yg.lib())
+    rng = np.random.default_rng(n)
+    sigma = np.full((k, d), 1e30, np.float32)
+    mu, w = np.zeros((k, d), np.float32), np.full(k, 1 / k, np.float32)
+    v = rng.standard_normal((n, d)).astype(np.float32)
+    late = n // 2 + 7
+    v[late:, : d // 2] *= np.float32(big)       # all later vectors, half of the coordinates
+    p = np.zeros((n, k), np.float32)
+    p[np.arange(n), np.arange(n) % k] = 1
+    p[: n // 3] = 1 / k
+    g, keep = make_gmm(w, mu, sigma)
+    got = run_fisher(L_, v, g, go.FLAGS_MU | go.FLAGS_SIGMA, p).reshape(2, k, d)
+    s0, s1, s2 = moments_32_64(p, v)
+    with np.errstate(all="ignore"):
+        sg = sigma.astype(np.float64)
+        e1 = s1 / sg / np.sqrt(n * w[:, None] / sg)
+        e2 = (s2 - s0 * sg) / (sg * np.sqrt(2 * n * w[:, None]))
+        exp = np.stack([e1, e2]).astype(np.float32)
+    np.testing.assert_array_equal(np.isnan(got), np.isnan(exp))
+    np.testing.assert_array_equal(np.isinf(got), np.isinf(exp))
+    fin = np.isfinite(exp)
+    # 32 terms a step in float, in any order: 32 u of the sum of their magnitudes
+    with np.errstate(all="ignore"):
+        a1 = (np.abs(v).astype(np.float64)).max() * s0 / sg / np.sqrt(n * w[:, None] / sg)
+        a2 = (s2 + s0 * sg) / (sg * np.sqrt(2 * n * w[:, None]))
+        tol = 40 * 2.0 ** -24 * np.stack([a1 + 0 * e1, a2])
+    assert (np.abs(got - exp)[fin] <= tol[fin] + 1e-6 * np.abs(exp)[fin] + 1e-30).all()
+    assert np.isfinite(exp).all() == (big < 1e18)
+
+
+@pytest.mark.gpu
+def test_gpu_moments_sums_past_float():
+    """Finite squares whose FP64 sums over many vectors are past FP32's range."""
+    L_ = bind(yg.lib())
+    n, d, k = 200_000, 8, 2
+    rng = np.random.default_rng(3)
+    v = (1e18 * (1 + rng.random((n, d)))).astype(np.float32)
+    p = np.zeros((n, k), np.float32)
+    p[:, 1] = 1
+    w, mu = np.full(k, 0.5, np.float32), np.zeros((k, d), np.float32)
+    sigma = np.full((k, d), 1e36, np.float32)
+    g, keep = make_gmm(w, mu, sigma)
+    got = run_fisher(L_, v, g, go.FLAGS_SIGMA, p).reshape(k, d)
+    s0, s1, s2 = moments_32_64(p, v)
+    sg = sigma.astype(np.float64)
+    exp = (s2 - s0 * sg) / (sg * np.sqrt(2 * n * w[:, None]))
+    np.testing.assert_allclose(got, exp, rtol=1e-4)

@@ -20,6 +20,7 @@
 #include <string.h>
 
 #include <algorithm>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/yael_gpu.h"
@@ -283,28 +284,29 @@ __device__ __forceinline__ void acc2(f32x2 &s, f32x2 &c, f32x2 y) {
   c = add2(c, add2(sub2(s, sub2(t, b)), sub2(y, b)));
   s = t;
 }
-// the same for values that may be infinite or NaN: such a sum has no error term
-__device__ __forceinline__ void acc_any(float &s, float &c, float y) {
-  const float t = __fadd_rn(s, y), b = __fsub_rn(t, s);
-  const float e = __fadd_rn(__fsub_rn(s, __fsub_rn(t, b)), __fsub_rn(y, b));
-  c = fabsf(t) <= 3.4e38f ? __fadd_rn(c, e) : 0.f;
-  s = t;
+// A slice with a value that could overflow a float sum (an infinity or a NaN too)
+// is summed again with two FP64 sums in a pair's registers, so that its sums are
+// finite, infinite or NaN as FP64 sums are: of the low float in s, the high in c.
+__device__ __forceinline__ double as_d(f32x2 a) { return __longlong_as_double((long long)a); }
+__device__ __forceinline__ f32x2 d_as(double a) { return (f32x2)__double_as_longlong(a); }
+__device__ __forceinline__ void to64(f32x2 &s, f32x2 &c) {
+  const double a = (double)lo2(s) + (double)lo2(c), b = (double)hi2(s) + (double)hi2(c);
+  s = d_as(a);
+  c = d_as(b);
 }
-__device__ __forceinline__ void acc2_any(f32x2 &s, f32x2 &c, f32x2 y) {
-  float sa = lo2(s), sb = hi2(s), ca = lo2(c), cb = hi2(c);
-  acc_any(sa, ca, lo2(y));
-  acc_any(sb, cb, hi2(y));
-  s = (f32x2)__float_as_uint(sb) << 32 | __float_as_uint(sa);
-  c = (f32x2)__float_as_uint(cb) << 32 | __float_as_uint(ca);
+__device__ __forceinline__ void acc64(f32x2 &s, f32x2 &c, f32x2 y) {
+  s = d_as(as_d(s) + (double)lo2(y));
+  c = d_as(as_d(c) + (double)hi2(y));
 }
-// an infinity, a NaN, or a value whose square could overflow a float sum
-// (|x| >= 2^34) among the four
-__device__ __forceinline__ bool special4(float4 x) {
-  constexpr float h = 1073741824.f;
+// an infinity, a NaN or a value of 2^64 / h or more among the four.  2^34 for
+// coordinates and 2^20 for posteriors: below them 2^31 products p x^2 add up to
+// less than 2^119.
+__device__ __forceinline__ bool big4(float4 x, float h) {
   const float a = x.x * h, b = x.y * h, c = x.z * h, d = x.w * h;
   const float z = 0.f * (a * a) + 0.f * (b * b) + 0.f * (c * c) + 0.f * (d * d);
   return z != z;
 }
+constexpr float kBigX = 1073741824.f, kBigP = 17592186044416.f;  // 2^30, 2^44
 
 template <int NW, int DPL>
 __global__ void __launch_bounds__(NW * 32, 16 / NW)
@@ -359,7 +361,7 @@ __global__ void __launch_bounds__(NW * 32, 16 / NW)
     for (int q = 0; q < XQ; q++) {
       const int t = tid + q * NT, r = t / (XW / 4), c = (t % (XW / 4)) * 4;
       *reinterpret_cast<float4 *>(&xs[buf][r][c]) = rx[q];
-      if (special4(rx[q])) atomicOr(&bad[b3], 1u << r);
+      if (big4(rx[q], kBigX)) atomicOr(&bad[b3], 1u << r);
     }
 #pragma unroll
     for (int q = 0; q < PQ; q++) {
@@ -373,84 +375,93 @@ __global__ void __launch_bounds__(NW * 32, 16 / NW)
   };
 
   f32x2 s1[CPW][H], c1[CPW][H], s2[CPW][H], c2[CPW][H];
-  float s0[CPW], c0s[CPW];
+  f32x2 s0[CPW / 2], c0s[CPW / 2];  // two components each
+  // The sums of the slice; whether this warp met a value that is not for pairs
+  // of floats (big4).  wide: FP64 sums in the pairs' registers (acc64).
+  auto pass = [&](auto wide_) -> bool {
+    constexpr bool wide = decltype(wide_)::value;
 #pragma unroll
-  for (int c = 0; c < CPW; c++) {
-    s0[c] = c0s[c] = 0.f;
+    for (int c = 0; c < CPW; c++) {
+      s0[c / 2] = c0s[c / 2] = 0ull;
 #pragma unroll
-    for (int h = 0; h < H; h++) s1[c][h] = c1[c][h] = s2[c][h] = c2[c][h] = 0ull;
-  }
-  if (tid < 3) bad[tid] = 0u;
-  __syncthreads();
-  if (PRE) gload(ib);
-  int step = 0;
-  bool special = false;  // an infinity, a NaN or a huge value has been seen
-  for (long i = ib; i < ie; i += 32, step++) {
-    const int buf = step & 1, b3 = step % 3;
-    if (!PRE) gload(i);
-    sstore(buf, b3);
-    __syncthreads();
-    if (tid == 0) bad[(step + 2) % 3] = 0u;
-    if (PRE && i + 32 < ie) gload(i + 32);
-    // lane = vector: which vectors have a positive posterior here
-    const float *prow = &ps[buf][0][2 * warp * CPW];
-    bool any = false, spec = false;
-#pragma unroll
-    for (int c = 0; c < CPW; c += 2) {
-      const float4 p = *reinterpret_cast<const float4 *>(prow + lane * PLD + 2 * c);
-      any = any || p.x != 0.f || p.z != 0.f;
-      spec = spec || special4(p);
-      if (blockIdx.x == 0) {
-        acc_any(s0[c], c0s[c], p.x);
-        acc_any(s0[c + 1], c0s[c + 1], p.z);
-      }
+      for (int h = 0; h < H; h++) s1[c][h] = c1[c][h] = s2[c][h] = c2[c][h] = 0ull;
     }
-    unsigned m = __ballot_sync(0xffffffffu, any) | bad[b3];
-    special = special || bad[b3] || __any_sync(0xffffffffu, spec);
-    if (!m) continue;
-    f32x2 f1[CPW][H], f2[CPW][H];
-#pragma unroll
-    for (int c = 0; c < CPW; c++)
-#pragma unroll
-      for (int h = 0; h < H; h++) f1[c][h] = f2[c][h] = 0ull;
-    do {
-      const int ii = __ffs(m) - 1;
-      m &= m - 1;
-      f32x2 x[H];
-      if (H == 2) {
-        const ulonglong2 t = *reinterpret_cast<const ulonglong2 *>(&xs[buf][ii][lane * DPL]);
-        x[0] = t.x;
-        x[H - 1] = t.y;
-      } else {
-        x[0] = *reinterpret_cast<const f32x2 *>(&xs[buf][ii][lane * DPL]);
-      }
+    if (tid < 3) bad[tid] = 0u;
+    __syncthreads();
+    if (PRE) gload(ib);
+    int step = 0;
+    bool big = false;
+    for (long i = ib; i < ie; i += 32, step++) {
+      const int buf = step & 1, b3 = step % 3;
+      if (!PRE) gload(i);
+      sstore(buf, b3);
+      __syncthreads();
+      if (tid == 0) bad[(step + 2) % 3] = 0u;
+      if (PRE && i + 32 < ie) gload(i + 32);
+      // lane = vector: which vectors have a positive posterior here
+      const float *prow = &ps[buf][0][2 * warp * CPW];
+      bool any = false;
 #pragma unroll
       for (int c = 0; c < CPW; c += 2) {
-        const ulonglong2 p =
-            *reinterpret_cast<const ulonglong2 *>(prow + ii * PLD + 2 * c);
+        const float4 p = *reinterpret_cast<const float4 *>(prow + lane * PLD + 2 * c);
+        any = any || p.x != 0.f || p.z != 0.f;
+        big = big || big4(p, kBigP);
+        if (blockIdx.x == 0) {
+          const f32x2 y = (f32x2)__float_as_uint(p.z) << 32 | __float_as_uint(p.x);
+          if (wide) acc64(s0[c / 2], c0s[c / 2], y);
+          else acc2(s0[c / 2], c0s[c / 2], y);
+        }
+      }
+      unsigned m = __ballot_sync(0xffffffffu, any) | bad[b3];
+      big = big || bad[b3];
+      if (!m) continue;
+      f32x2 f1[CPW][H], f2[CPW][H];
+#pragma unroll
+      for (int c = 0; c < CPW; c++)
+#pragma unroll
+        for (int h = 0; h < H; h++) f1[c][h] = f2[c][h] = 0ull;
+      do {
+        const int ii = __ffs(m) - 1;
+        m &= m - 1;
+        f32x2 x[H];
+        if (H == 2) {
+          const ulonglong2 t = *reinterpret_cast<const ulonglong2 *>(&xs[buf][ii][lane * DPL]);
+          x[0] = t.x;
+          x[H - 1] = t.y;
+        } else {
+          x[0] = *reinterpret_cast<const f32x2 *>(&xs[buf][ii][lane * DPL]);
+        }
+#pragma unroll
+        for (int c = 0; c < CPW; c += 2) {
+          const ulonglong2 p =
+              *reinterpret_cast<const ulonglong2 *>(prow + ii * PLD + 2 * c);
+#pragma unroll
+          for (int h = 0; h < H; h++) {
+            f1[c][h] = fma2(p.x, x[h], f1[c][h]);
+            f1[c + 1][h] = fma2(p.y, x[h], f1[c + 1][h]);
+            const f32x2 xx = mul2(x[h], x[h]);
+            f2[c][h] = fma2(p.x, xx, f2[c][h]);
+            f2[c + 1][h] = fma2(p.y, xx, f2[c + 1][h]);
+          }
+        }
+      } while (m);
+#pragma unroll
+      for (int c = 0; c < CPW; c++)
 #pragma unroll
         for (int h = 0; h < H; h++) {
-          f1[c][h] = fma2(p.x, x[h], f1[c][h]);
-          f1[c + 1][h] = fma2(p.y, x[h], f1[c + 1][h]);
-          const f32x2 xx = mul2(x[h], x[h]);
-          f2[c][h] = fma2(p.x, xx, f2[c][h]);
-          f2[c + 1][h] = fma2(p.y, xx, f2[c + 1][h]);
+          if (wide) {
+            acc64(s1[c][h], c1[c][h], f1[c][h]);
+            acc64(s2[c][h], c2[c][h], f2[c][h]);
+          } else {
+            acc2(s1[c][h], c1[c][h], f1[c][h]);
+            acc2(s2[c][h], c2[c][h], f2[c][h]);
+          }
         }
-      }
-    } while (m);
-#pragma unroll
-    for (int c = 0; c < CPW; c++)
-#pragma unroll
-      for (int h = 0; h < H; h++) {
-        if (special) {
-          acc2_any(s1[c][h], c1[c][h], f1[c][h]);
-          acc2_any(s2[c][h], c2[c][h], f2[c][h]);
-        } else {
-          acc2(s1[c][h], c1[c][h], f1[c][h]);
-          acc2(s2[c][h], c2[c][h], f2[c][h]);
-        }
-      }
-  }
+    }
+    return big;
+  };
+  const bool wide = __syncthreads_or(pass(std::false_type()));
+  if (wide) (void)pass(std::true_type());  // rare: the slice again
 
   double *out = part + (long)blockIdx.z * k * (2L * d + 1);
 #pragma unroll
@@ -458,7 +469,8 @@ __global__ void __launch_bounds__(NW * 32, 16 / NW)
     const int j = j0 + warp * CPW + c;
     if (j >= k) break;
     if (blockIdx.x == 0) {
-      double t = (double)s0[c] + (double)c0s[c];
+      if (!wide && !(c & 1)) to64(s0[c / 2], c0s[c / 2]);
+      double t = as_d(c & 1 ? c0s[c / 2] : s0[c / 2]);
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
       if (lane == 0) out[2L * k * d + j] = t;
@@ -467,13 +479,17 @@ __global__ void __launch_bounds__(NW * 32, 16 / NW)
     for (int h = 0; h < H; h++) {
       const int l = l0 + lane * DPL + 2 * h;
       const long o = (long)j * d + l;
+      if (!wide) {
+        to64(s1[c][h], c1[c][h]);
+        to64(s2[c][h], c2[c][h]);
+      }
       if (l < d) {
-        out[o] = (double)lo2(s1[c][h]) + (double)lo2(c1[c][h]);
-        out[(long)k * d + o] = (double)lo2(s2[c][h]) + (double)lo2(c2[c][h]);
+        out[o] = as_d(s1[c][h]);
+        out[(long)k * d + o] = as_d(s2[c][h]);
       }
       if (l + 1 < d) {
-        out[o + 1] = (double)hi2(s1[c][h]) + (double)hi2(c1[c][h]);
-        out[(long)k * d + o + 1] = (double)hi2(s2[c][h]) + (double)hi2(c2[c][h]);
+        out[o + 1] = as_d(c1[c][h]);
+        out[(long)k * d + o + 1] = as_d(c2[c][h]);
       }
     }
   }

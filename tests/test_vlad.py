@@ -173,3 +173,26 @@ def test_gpu_vlad_sums(n, d, k):
     keep = np.setdiff1d(np.arange(n), bad).astype(np.int32)
     L.vlad_compute(k, d, ptr(C), n, ptr(v2), ptr(out))
     np.testing.assert_array_equal(out, vlad_np(C, v, a, None, keep, np.array([len(keep)]))[0])
+
+
+@pytest.mark.gpu
+def test_gpu_vlad_large_vocabularies_are_sorted():
+    """The form that reads the whole assignment once a cluster is for small
+    vocabularies: from 10M reads on, and from 32k blocks on, the points are sorted
+    (more launches, the same sums)."""
+    L = yg.lib()
+    rng = np.random.default_rng(4)
+    d = 8
+
+    def run(n, k):
+        C = (rng.standard_normal((k, d)) * 4).astype(np.float32)
+        v = (C[rng.integers(0, k, n)] + 0.1 * rng.standard_normal((n, d))).astype(np.float32)
+        out = np.empty((k, d), np.float32)
+        for _ in range(8):        # (the first calls of a shape tune its passes)
+            L0 = L.yael_gpu_launch_count()
+            L.vlad_compute(k, d, ptr(C), n, ptr(v), ptr(out))
+            launches = L.yael_gpu_launch_count() - L0
+        np.testing.assert_array_equal(out, vlad_np(C, v, knn_exact(C, v, 1)[0][:, 0])[0])
+        return launches
+    assert run(1100, 9200) - run(1000, 9200) == 2      # 10.1M and 9.2M reads
+    assert run(100, 33_000) - run(100, 32_000) == 2

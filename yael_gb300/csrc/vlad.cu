@@ -97,11 +97,20 @@ __global__ void vlad_sum_kernel(const int *perm, const int *offs, const float *v
   desc[t] = ordered_sum(perm + e0, offs[g + 1] - e0, v + j, d, cj, w);
 }
 
-// The same for few points without subsets (kScanMax): a block per cluster (and
-// 128 coordinates) picks its cluster's points out of the assignment itself, in
+// The same for few points without subsets: a block per cluster (and 128
+// coordinates) picks its cluster's points out of the assignment itself, in
 // order, instead of a sort of all of them and its three launches.
 // 2,000 points, k = 64, d = 128: 35 us for keys, sort, offsets and sums, 10 here.
+// The work is k n reads for each 128 coordinates, so the sort is left for large
+// vocabularies (a call with either form, us): 2,000 x 4,096, d = 128 (8M reads)
+// 205 and 214 sorted; 8,192 x 1,024, d = 300 (25M) 407 and 382; 2,000 x 16,384,
+// d = 128 (33M) 524 and 485; 8,192 x 16,384 (134M) 1,693 and 1,323; and by the
+// blocks alone, 100 x 65,536, d = 32, 264 and 236.
 constexpr int kScanMax = 8192, kScanT = 128;
+bool scan_form(long n, long k, long d) {
+  const long per = k * ceil_div(d, kScanT);  // blocks
+  return n <= kScanMax && per <= 32768 && per * n <= 10L * 1000 * 1000;
+}
 __global__ void __launch_bounds__(kScanT)
     vlad_scan_kernel(const int *__restrict__ assign, int n, const float *__restrict__ v, int d,
                      const float *__restrict__ C, const float *__restrict__ w,
@@ -274,7 +283,7 @@ int vlad_run(int k, int d, const float *centroids, int n, const float *v, const 
   void *host = desc;  // a small descriptor comes back through pinned memory
   if (bytes <= (size_t)1 << 20) YG_CHECK(A.ctx->pinned.get(VP_DESC, bytes, &host));
   auto sums = [&]() -> int {
-    if (!subsets && n <= kScanMax && ceil_div(d, kScanT) <= 65535) {
+    if (!subsets && scan_form(n, k, d)) {
       vlad_scan_kernel<<<dim3((unsigned)k, (unsigned)ceil_div(d, kScanT)), kScanT, 0, A.st>>>(
           A.assign, n, A.dv, d, A.dc, dw, ddesc);
     } else {

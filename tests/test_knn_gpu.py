@@ -567,3 +567,24 @@ def test_nearest_among_copies_of_integer_rows(nq, nb, prec):
     b, q = c[rng.integers(0, 17, nb)], c[rng.integers(0, 17, nq)]
     st = assert_exact(b, q, 1, prec)
     assert st["exact_class"] == 1 and st["n_band"] == 0 and st["n_fallback"] == 0
+
+
+@pytest.mark.parametrize("d", [900, 3000, 6002])
+@pytest.mark.parametrize("dt", [2, 16])
+def test_near_ties_in_long_rows(d, dt):
+    """Rows whose distances differ by 1e-12 to 1e-7 of their value, long enough that
+    the roundings of pairs of floats add up: ids in FP64 order."""
+    rng = np.random.default_rng(d)
+    q = rng.standard_normal((6, d)).astype(np.float32)
+    base = rng.standard_normal(d).astype(np.float32)
+    b = np.repeat(base[None], 400, 0)
+    b[:, 0] += np.linspace(-1e-6, 1e-6, 400).astype(np.float32)
+    b[rng.permutation(400)[:200], d - 1] += np.float32(1e-6)
+    idx, _, _ = gpu_knn(b, q, 30, "fp32", dt=dt)
+    q64, b64 = q.astype(np.float64), b.astype(np.float64)
+    full = q64 @ b64.T if dt == 16 else np.array([((x - b64) ** 2).sum(1) for x in q64])
+    got = np.take_along_axis(full, idx, 1)
+    # (the k smallest in FP64, in an order that FP64 sums in any order agree with)
+    slack = 1e-13 * np.abs(full).max()
+    assert (got <= np.sort(full, 1)[:, 29:30] + slack).all()
+    assert (np.diff(got, axis=1) >= -slack).all()

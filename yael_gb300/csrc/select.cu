@@ -267,9 +267,15 @@ __device__ __forceinline__ float lanes_dist32(const float *qv, const float *brow
 }
 
 // The same distance in pairs of floats (exact differences and products, two-sum
-// additions): within (d + 16) 2^-45 of its value (L2; of |q||b| for the inner
-// product).  This GPU's FP64 pipe runs at 1/64 of the FP32 rate; this takes about
-// 20 FP32 operations a coordinate.  The result is lane sl = 0's.
+// additions): within pair_error(d) of its value (L2; of |q||b| for the inner
+// product).  A lane adds m <= d / 8 + 5 terms; the low parts, at most u sum_i |hi_i| +
+// 3 u S <= u (m + 3) S, are rounded once or twice a term, which loses at most
+// (m^2 / 2 + 8 m) u^2 S (u = 2^-24), and the dropped square of a difference's low
+// part u^2 S more.  This GPU's FP64 pipe runs at 1/64 of the FP32 rate; this takes
+// about 20 FP32 operations a coordinate.  The result is lane sl = 0's.
+__device__ __forceinline__ double pair_error(int d) {
+  return (double)(d + 16) * 2.9e-14 + (double)d * d * 3.1e-17;
+}
 template <int LPR>
 __device__ __forceinline__ double lanes_dist_pair(const float *qv, const float *brow, int d,
                                                   int metric, int sl, unsigned gm) {
@@ -606,8 +612,8 @@ __global__ void __launch_bounds__(RT) rerank_kernel(RerankArgs a, int Mp_alloc) 
         __syncthreads();
         for (int i = tid; i < lastpair; i += RT) {
           const double e0 = ord2d(K[i]), e1 = ord2d(K[i + 1]);
-          const double tol = (double)(d + 16) * 2.9e-14 * (fabs(e0) + fabs(e1)) +
-                             (double)eta * 1e-6 + 1e-36;
+          const double tol = pair_error(d) * (fabs(e0) + fabs(e1)) +
+                             (double)eta * (1e-6 + 6e-10 * d) + 1e-36;
           if (!(e1 - e0 > tol)) sneed64 = 1;
         }
         __syncthreads();
@@ -621,9 +627,8 @@ __global__ void __launch_bounds__(RT) rerank_kernel(RerankArgs a, int Mp_alloc) 
       const unsigned long long kk = K[k - 1];
       const unsigned long long u = (kk & 0x8000000000000000ull) ? (kk & 0x7fffffffffffffffull) : ~kk;
       const double ek = __longlong_as_double((long long)u);
-      // (pairs of floats: within (d + 16) 2.9e-14 of the value and 1e-6 eta)
-      ekh = __double2float_ru(ek + (1e-12 + (double)(d + 16) * 2.9e-14) * fabs(ek) +
-                              1e-6 * (double)eta + 1e-36);
+      ekh = __double2float_ru(ek + (1e-12 + pair_error(d)) * fabs(ek) +
+                              (1e-6 + 6e-10 * d) * (double)eta + 1e-36);
       for (int r = tid; r < k; r += RT) {
         const unsigned long long kr = K[r];
         const unsigned long long ur = (kr & 0x8000000000000000ull) ? (kr & 0x7fffffffffffffffull) : ~kr;

@@ -8,8 +8,9 @@
 //     rows still in shared memory;
 //   * moments: sum_i p_ij, sum_i p_ij x_il and sum_i p_ij x_il^2 for every
 //     component and dimension (FP32 within each step of 32 vectors, pairs of
-//     floats across steps, FP64 across vector slices, summed in a fixed order:
-//     every result is reproducible), skipping zero posteriors.
+//     floats across steps, or FP64 where values are large, FP64 across vector
+//     slices, summed in a fixed order: every result is reproducible), skipping
+//     zero posteriors.
 // Fisher vectors are formed on the device from those moments; the EM update of the
 // k x d parameters and the empty-component splits are host code over them.  The posterior
 // matrix (n x k) stays on the device between the passes of an EM iteration.
@@ -251,10 +252,13 @@ __global__ void softmax_kernel(float *__restrict__ P, const float *__restrict__ 
 // left out for finite x; a row with an infinity or a NaN is never skipped.)
 // Dense posteriors are bound by the FP32 pipe: two packed multiply-adds per
 // two dimensions and component.  Sums are FP32 within each step of 32 vectors
-// and pairs of floats (two-sum) across steps: FP64 additions there held the
-// FP64 pipe, 4 of its operations per 64 multiply-adds at 1/64 the rate.  Slices are summed in FP64 in a fixed order.  n = 100k, k = 256,
-// d = 128: 1.25 ms -> 0.21 ms on average over ten EM iterations (all
-// posteriors positive in the first, 0.5% of them from the third on).
+// and pairs of floats (two-sum, 2^-48) across steps: FP64 additions there held the
+// FP64 pipe, 4 of its operations per 64 multiply-adds at 1/64 the rate.  Slices
+// are summed in FP64 in a fixed order.  Against 64-bit moments the mean error
+// is 0.77 to 1.00 of what FP64 sums across the steps gave (32 mixtures of 200 to
+// 100k vectors, d = 16 to 128, k = 4 to 256): the steps' float sums set it.
+// n = 100k, k = 256, d = 128: 1.25 ms -> 0.21 ms on average over ten EM iterations
+// (all posteriors positive in the first, 0.5% of them from the third on).
 typedef unsigned long long f32x2;
 __device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
   f32x2 r;
@@ -846,8 +850,12 @@ struct GmmDev {
     }
     // Dimensions per lane by d.  16 warps to a CTA (fewer passes over the
     // vectors) where k gives the warps components of their own and n gives
-    // every SM some steps; else 4-warp CTAs, four to an SM.
-    // n = 2000, k = 256, d = 64: 17 us on 4-warp CTAs, 30 on 16-warp ones.
+    // every SM some steps; else 4-warp CTAs, four to an SM.  Both sums' passes in
+    // us, 4-warp and 16-warp CTAs, dense posteriors, d = 64 and 128, k = 256: n = 500
+    // 26 / 44 and 23 / 40; 2,000 37 / 52 and 42 / 50; 5,000 50 / 56 and 58 / 60;
+    // 9,000 64 / 64 and 75 / 79; 20,000 93 / 93 and 130 / 126; 100,000 301 / 284 and
+    // 549 / 484 (2% of them positive: 158 / 146 and 239 / 191).  k = 32, d = 128:
+    // 121 / 118 at 100,000.
     const bool many = n >= 64L * ctx->num_sms;
     if (d > 64) {
       if (k > 32 && many) launch_moments<16, 4>(); else launch_moments<4, 4>();

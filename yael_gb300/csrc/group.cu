@@ -315,8 +315,8 @@ int wave_prepare(const yael_gpu_knn_pair *pairs, const Wave &w, int d, int k, in
   YG_CHECK(gs_get(ws, o + GS_CNT, cnt_tot, &S.cnt));
   YG_CHECK(gs_get(ws, o + GS_CANDV, cand_tot, &S.candv));
   YG_CHECK(gs_get(ws, o + GS_CANDI, cand_tot, &S.candi));
-  // the host tables are copied before they go out of scope: pageable copies
-  // are staged before cudaMemcpyAsync returns
+  // the host tables may go out of scope: a copy from pageable memory has read its
+  // source when cudaMemcpyAsync returns (copy_to_device)
   YG_CUDA(cudaMemcpyAsync(S.dpairs, hp.data(), sizeof(GroupPair) * np, cudaMemcpyHostToDevice,
                           sp));
   YG_CUDA(cudaMemcpyAsync(S.dinf, hinf.data(), np, cudaMemcpyHostToDevice, sp));

@@ -443,8 +443,7 @@ struct Engine {
   // starts from each point's distance to its previous centroid's new
   // position, an upper bound of its nearest distance: a THRESH pass with those
   // thresholds finds every possible winner with the cheapest selection, and no
-  // sample pass.  (The plain FP32 path keeps its list pass: its CUDA-core
-  // scan does not gain from the cheaper selection.)
+  // sample pass.  (The plain FP32 path runs its thresholds without a bound.)
   bool have_prev = false;
 
   void count_assign(const KnnJob &job) {
@@ -550,8 +549,13 @@ struct Engine {
       YG_CHECK(ws_get(ctx->ws, KS_MOVED, 1, &moved));
       YG_CHECK(ctx->pinned.get(5, sizeof(int), reinterpret_cast<void **>(&ph_moved)));
     }
-    // A moved row costs two rows of 64-bit atomics where the full update reads
-    // every row once: 50k x 64, k = 100: full update 34 us, 5 with few moves.
+    // A moved row costs two rows of 64-bit atomics where the full update sorts the
+    // points and reads every row once.  The update in us, full and with moves, at
+    // the share of points that had moved: 50k x 64, k = 100: 53 and 16 at 32%, 14
+    // below 4%; 200k x 128, k = 100: 170 and 69 at 23%, 22 at 9%; 1M x 64, k = 200:
+    // 429 and 66 at 20%; 300k x 128, k = 2,048: 136 and 57 at 28%.  The line
+    // keeps the full update where most rows move, as from a run's first
+    // assignment to its second.
     const int delta = track && sums_live && last_moved >= 0 && 3 * last_moved < ntot ? 1 : 0;
     // the counts, the slice sums and a flag go straight to the pinned host
     // buffers (no copies in the step); the slice sums run beside the centroids

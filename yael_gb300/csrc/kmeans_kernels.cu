@@ -1056,7 +1056,9 @@ int km_finalize(const long long *acc, const int *counts, long ncl, int d, int k,
                 int *counts_out, const int *err, int *err_out) {
   // FP64 runs at 1/64 of the FP32 rate: 32,768 rows of 96 take 84 us with a
   // division per coordinate and 38 with one per four; a few hundred rows are
-  // done sooner with more threads (2.6 and 4 us)
+  // done sooner with more threads (2.6 and 4 us).  An update of k rows of 128, one
+  // and four coordinates a division: k = 256 8.0 and 8.1 us, 1,024 23.1 and 22.5,
+  // 2,048 24.9 and 22.3, 16,384 66 and 49.
   if (ncl * d >= 1 << 18)
     finalize_kernel<4><<<(unsigned)ceil_div(ncl * ceil_div(d, 4), 256), 256, 0, st>>>(
         acc, counts, ncl, d, k, shift, active, C, counts_out, err, err_out);

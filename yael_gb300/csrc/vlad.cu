@@ -4,10 +4,11 @@
 // A VLAD sum is float arithmetic in a fixed order: the reference adds the
 // residuals (v_i - c) of a cluster's points in increasing point order (list
 // order for the subset form).  Here the point indices are sorted stably by
-// cluster (radix sort: equal keys keep their order), and one thread per
-// (cluster, coordinate) walks its cluster's points in that order with
-// round-to-nearest adds and multiplies that the compiler may not fuse, so each
-// output is the reference's own sequence of float operations.  Bag-of-features
+// cluster (radix sort: equal keys keep their order) or, for few points and
+// clusters, picked out of the assignment in order by each cluster's block, and
+// one thread per (cluster, coordinate) walks its cluster's points in that order
+// with round-to-nearest adds and multiplies that the compiler may not fuse, so
+// each output is the reference's own sequence of float operations.  Bag-of-features
 // counts are integer (or exact float) histograms.
 #include <limits.h>
 #include <string.h>

@@ -588,3 +588,18 @@ def test_near_ties_in_long_rows(d, dt):
     slack = 1e-13 * np.abs(full).max()
     assert (got <= np.sort(full, 1)[:, 29:30] + slack).all()
     assert (np.diff(got, axis=1) >= -slack).all()
+
+
+@pytest.mark.parametrize("prec", PRECS)
+@pytest.mark.parametrize("nb,k", [(100_000, 1000), (20_000, 1200), (20_000, 610)])
+def test_long_neighbour_lists_stay_within_the_candidates(nb, k, prec):
+    """A thousand neighbours and more: the expected candidates come near the limit of
+    a query's, and queries past it end in the exhaustive pass.  A few may, by the
+    sample's luck."""
+    rng = np.random.default_rng(nb)
+    b = rng.standard_normal((nb, 64)).astype(np.float32)
+    q = rng.standard_normal((200, 64)).astype(np.float32)
+    b /= np.linalg.norm(b, axis=1, keepdims=True)
+    q /= np.linalg.norm(q, axis=1, keepdims=True)
+    st = assert_exact(b, q, k, prec)
+    assert st["n_fallback"] <= 2

@@ -31,7 +31,6 @@ namespace yg {
 namespace {
 
 constexpr int kGroupTiles = 128;       // base tiles per main-pass unit
-constexpr int kSampleC = 13;           // threshold rank in the sample (knn.cu)
 
 // workspace slots of the grouped pipeline (disjoint from the per-call ones)
 enum GroupSlot : int {
@@ -111,13 +110,13 @@ void pair_layout(int nb, int stride, bool inf, int *nreg, int *cap, int *tpc) {
   if (inf) {
     *cap = pow2_ge(std::max(1, *tpc * TC_TILE_N / 2));
   } else {
-    const double er = (double)kSampleC * stride / *nreg;
+    const double er = (double)sample_rank_3(stride) * stride / *nreg;
     *cap = pow2_ge((int)(2.0 * er + 6.0 * sqrt(er) + 16.0));
   }
 }
 
 // a pair whose sample is too short for a threshold (knn.cu)
-bool pair_inf(int nb, int stride) { return nb / stride < 4 * kSampleC; }
+bool pair_inf(int nb, int stride) { return nb / stride < 4 * sample_rank_3(stride); }
 
 struct Wave {
   std::vector<int> pairs;  // indices into the caller's pair array
@@ -245,7 +244,7 @@ int wave_prepare(const yael_gpu_knn_pair *pairs, const Wave &w, int d, int k, in
   // ---- main-pass layout: chunks, regions and capacities per pair
   std::vector<GroupUnit> mu, su;
   long cnt_tot = 0, cand_tot = 0;
-  int max_cand = 4 * kSampleC * stride + 64;
+  int max_cand = 4 * sample_rank_3(stride) * stride + 64;
   for (int i = 0; i < np; i++) {
     GroupPair &g = hp[i];
     const int ntb = (int)ceil_div(g.nb, TC_TILE_N);
@@ -365,7 +364,7 @@ int wave_execute(WaveState &S, int d, int k, int metric, int max_ctas, cudaStrea
     TcOperands ops;
     YG_CHECK(tc_base_view(op, S.stride, (int)(S.brows / S.stride), &ops));
     YG_CHECK(tc_scan(ops, S.nq_all, (int)(S.brows / S.stride), ss, st));
-    YG_CHECK(thresh_from_sample(S.nq_all, 1, 16, kSampleC, S.stopv, S.eps, S.thr, st));
+    YG_CHECK(thresh_from_sample(S.nq_all, 1, 16, sample_rank_3(S.stride), S.stopv, S.eps, S.thr, st));
   }
   thr_inf_kernel<<<(unsigned)ceil_div(S.nq_all, 256), 256, 0, st>>>(S.qpair, S.dinf, S.nq_all,
                                                                     S.thr);
@@ -398,7 +397,7 @@ int wave_execute(WaveState &S, int d, int k, int metric, int max_ctas, cudaStrea
   ra.fail_cnt = &S.status->fail_cnt;
   ra.n_cand = &S.status->n_cand;
   ra.kth_out = S.kth;
-  ra.m_expect = kSampleC * S.stride;
+  ra.m_expect = sample_rank_3(S.stride) * S.stride;
   ra.qpair = S.qpair;
   ra.gpairs = S.dpairs;
   ra.max_candidates = S.max_cand;

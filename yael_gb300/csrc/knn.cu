@@ -138,8 +138,8 @@ struct SamplePlan {
   int stride, c;
   SamplePlan(int k, int nb, bool bf16) {
     const bool big = bf16 && k >= 96 && nb / (k / 6) >= kSampleMin;
-    c = big ? 19 : 13;
     stride = imax(1, k / (big ? 6 : 3));
+    c = big ? 19 : sample_rank_3(stride);
     // The FP32 pass costs its sample more than its candidates: at least a
     // 1/16 sample while it keeps 256 rows.  1,000 x 100k, d = 100, k = 20: 1/6
     // of the base and 78 candidates 270 us, 1/16 and 144 candidates 52 (the

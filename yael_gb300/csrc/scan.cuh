@@ -130,6 +130,15 @@ __host__ __device__ inline float run_slack(float eps) {
 // threshold's rank grows by less than a tenth).
 constexpr int kSampleD = 32, kSampleSuper = 32 * kSampleD, kSampleMin = 4 * kSampleSuper;
 
+// The rank of a sample of one row in stride = k / 3: 13, at which 1.6e-5 of the
+// queries find fewer than k rows; 12 (1.7e-4, and a band pass for them) from a
+// stride of 200 on, where the expected 13 strides come near the 8,192
+// candidates that a query may have, and the queries past them go to the exhaustive
+// pass: 200 queries, d = 64, 100k rows, k = 1,000: 4 of them at 13 (1.68 ms), none at 12
+// (0.91); and where a rank of 13 leaves short bases without a sample: 20k rows,
+// k = 1,200: 4.3 ms and 1.0.
+inline int sample_rank_3(int stride) { return stride >= 200 ? 12 : 13; }
+
 // FP32 CUDA-core producer.  q: nq rows (stride ldq floats); b: nb rows (stride
 // ldb floats); bn: ||b||^2 as float with stride bn_stride (L2 only).
 // Base tiles are 128 rows.  Reported base ids are j (row index in this view).

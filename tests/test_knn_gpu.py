@@ -603,3 +603,32 @@ def test_long_neighbour_lists_stay_within_the_candidates(nb, k, prec):
     q /= np.linalg.norm(q, axis=1, keepdims=True)
     st = assert_exact(b, q, k, prec)
     assert st["n_fallback"] <= 2
+
+
+def test_fp32_form_by_size():
+    """FP32, up to 8 neighbours: lists for many queries over few rows, thresholds on
+    the other side of each line (the form is read from the trace of a child process),
+    the same ids from both."""
+    import subprocess
+    import sys
+    shapes = [(6000, 896, 2, "topc"), (5999, 896, 2, "thresh"), (6000, 897, 4, "thresh"),
+              (16384, 1024, 4, "topc"), (65536, 2048, 3, "topc"), (65536, 2049, 3, "thresh"),
+              (8192, 512, 5, "topc"), (8191, 512, 5, "thresh"), (8192, 513, 8, "thresh"),
+              (65536, 896, 8, "topc"), (65536, 896, 9, "thresh"), (300, 100, 2, "thresh")]
+    code = (
+        "import numpy as np, sys, yael_gb300 as yg; sys.path.insert(0, 'tests')\n"
+        "from _util import knn_mismatches\n"
+        "rng = np.random.default_rng(7)\n"
+        "for nq, nb, k, form in %r:\n"
+        "    b = rng.standard_normal((nb, 12)).astype(np.float32)\n"
+        "    q = rng.standard_normal((nq, 12)).astype(np.float32)\n"
+        "    idx, _ = yg.knn(q, b, nnn=k, precision='fp32')\n"
+        "    assert knn_mismatches(b, q, idx)[0] == 0, (nq, nb, k)\n" % (shapes,))
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True,
+                       env=dict(os.environ, YAEL_GPU_TRACE="1"), timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
+    first = [ln for ln in r.stderr.splitlines() if "knn level=0" in ln]
+    assert len(first) == len(shapes)
+    for (nq, nb, k, form), ln in zip(shapes, first):
+        assert f"pass={form} nq={nq} nb={nb} " in ln, ln

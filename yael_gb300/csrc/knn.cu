@@ -160,6 +160,21 @@ int list_length(int k, int exact, int nb) {
   return k <= 4 ? 8 : 2 * k;
 }
 
+// FP32, up to 8 neighbours of many queries among few rows: lists of 8 (k <= 4) or
+// 16, whose re-rank is a group of lanes a query; a threshold's candidates take a
+// block a query, 10 ns each however few they are.  The pass with lists is the slower
+// one, so the line is where the rows outweigh that.  The time by thresholds
+// over that by lists, d = 64: 100k queries, k = 2: 300 rows 2.3 times, 1,024 1.44, 2,048
+// 1.09, 3,000 0.94; 20k: 300 1.56, 1,024 1.08, 1,500 0.96; 6,000: 300 1.26, 1,024 1.19,
+// 2,048 0.95; 3,000: 300 0.89.  k = 8: 100k 300 1.88, 800 1.21, 1,500 0.91; 10k 300 1.42,
+// 512 1.08, 800 0.80; 3,000: 300 0.94.  (d = 16 gains more, d = 200 less: 10k, k = 2,
+// 800 rows 1.37 and 1.11.)
+bool fp32_lists(int k, int nb, int nq) {
+  if (k < 2 || k > 8) return false;
+  if (k <= 4) return nq >= 6000 && nb <= (nq >= 65536 ? 2048 : nq >= 16384 ? 1024 : 896);
+  return nq >= 8192 && nb <= (nq >= 65536 ? 896 : 512);
+}
+
 // out[q] = the least of n rows of nq values
 __global__ void min_rows_kernel(const float *v, int nq, int n, float *out) {
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
@@ -360,15 +375,16 @@ int knn_batch(KnnJob &job, Ctx *ctx, cudaStream_t st, Small *dsmall, BaseOps *bo
   float *kth;
   YG_CHECK(ws_get(ws, WS_KTH, nq, &kth));
   ra.kth_out = kth;
-  const bool band = job.band_kth != nullptr;
-  const bool prior = !band && job.prior_kth != nullptr;
 
   const bool timed = job.timing || trace_enabled();
   const int tile_n = bf16 ? TC_TILE_N : SIMT_TILE_N;
-  const int tile_m = bf16 ? TC_TILE_M : job.lists ? 128 : simt_tile_m(nq, nb, ctx->num_sms);
+  const bool band = job.band_kth != nullptr;
+  const bool prior = !band && job.prior_kth != nullptr;
+  const bool lists = !bf16 && !band && !prior && (job.lists || fp32_lists(k, nb, nq));
+  const int tile_m = bf16 ? TC_TILE_M : lists ? 128 : simt_tile_m(nq, nb, ctx->num_sms);
   const int nqt = (int)ceil_div(nq, tile_m);
   const int ntb = (int)ceil_div(nb, tile_n);
-  const int ctas_per_sm = bf16 || job.lists ? 1 : 2;
+  const int ctas_per_sm = bf16 || lists ? 1 : 2;
   // (few CTAs in all: single tiles, so that every SM has some)
   const int min_tiles = bf16 || (long)nqt * ntb > 8L * ctx->num_sms ? 4 : 1;
   // oversampling for inexact distances: the certificate needs a margin between
@@ -437,7 +453,7 @@ int knn_batch(KnnJob &job, Ctx *ctx, cudaStream_t st, Small *dsmall, BaseOps *bo
       sel.run_eps = nullptr;
     }
     job.scan_launches++;
-  } else if ((bf16 || job.lists) && !band && !prior && c_needed <= 16) {
+  } else if ((bf16 || lists) && !band && !prior && c_needed <= 16) {
     // ---- TOPC over the full base (register lists)
     sel.mode = SCAN_TOPC;
     sel.C = pow2_at_least(c_needed);
@@ -662,7 +678,7 @@ int knn_batch(KnnJob &job, Ctx *ctx, cudaStream_t st, Small *dsmall, BaseOps *bo
   // first: 1,500 queries x 60k rows that are copies of 17, d = 128, k = 10: 152 ms by
   // the band and the exhaustive pass, 1.9 with lists (1.1 with nothing before them).
   const bool to_lists =
-      !bf16 && !band && !job.lists && k > 1 && k <= 16 && hs.bs.all_exact && job.w == nullptr;
+      !bf16 && !band && !lists && k > 1 && k <= 16 && hs.bs.all_exact && job.w == nullptr;
   const bool to_band = !band && job.w == nullptr;
   const bool to_split =
       band && (job.prec == PREC_BF16 || job.prec == PREC_FP16) && job.w == nullptr;
@@ -756,7 +772,7 @@ int knn_batches(KnnJob &job, Ctx *ctx, cudaStream_t st, Small *dsmall, BaseOps *
     const int nqt = (int)ceil_div(nq, tile_m), ntb = (int)ceil_div(nb, tile_n);
     const int C = pow2_at_least(cn);
     size_t per_query;
-    if (!bf16 && !job.lists) {
+    if (!bf16 && !job.lists && !fp32_lists(k, nb, nq)) {
       // running thresholds: up to 16 slots a region; else the regions' share of the
       // candidates, or the whole base where it is too short for a sample
       const int m = simt_tile_m(nq, nb, ctx->num_sms), nt = (int)ceil_div(nq, m);

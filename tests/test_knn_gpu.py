@@ -606,29 +606,35 @@ def test_long_neighbour_lists_stay_within_the_candidates(nb, k, prec):
 
 
 def test_fp32_form_by_size():
-    """FP32, up to 8 neighbours: lists for many queries over few rows, thresholds on
-    the other side of each line (the form is read from the trace of a child process),
-    the same ids from both."""
+    """FP32, up to 16 neighbours: lists for many queries over few rows, thresholds on
+    the other side of each line, for real values and for exact ones (the form is read
+    from the trace of a child process); the same ids from both."""
     import subprocess
     import sys
-    shapes = [(6000, 896, 2, "topc"), (5999, 896, 2, "thresh"), (6000, 897, 4, "thresh"),
-              (16384, 1024, 4, "topc"), (65536, 2048, 3, "topc"), (65536, 2049, 3, "thresh"),
-              (8192, 512, 5, "topc"), (8191, 512, 5, "thresh"), (8192, 513, 8, "thresh"),
-              (65536, 896, 8, "topc"), (65536, 896, 9, "thresh"), (300, 100, 2, "thresh")]
+    real = [(6000, 896, 2, "topc"), (5999, 896, 2, "thresh"), (6000, 897, 4, "thresh"),
+            (16384, 1024, 4, "topc"), (65536, 2048, 3, "topc"), (65536, 2049, 3, "thresh"),
+            (8192, 512, 5, "topc"), (8191, 512, 5, "thresh"), (8192, 513, 8, "thresh"),
+            (65536, 896, 8, "topc"), (65536, 896, 9, "thresh"), (300, 100, 2, "thresh")]
+    exact = [(3000, 4096, 2, "topc"), (2999, 4096, 2, "thresh"), (3000, 4097, 2, "thresh"),
+             (3000, 2048, 3, "topc"), (3000, 2049, 4, "thresh"), (6000, 1024, 5, "topc"),
+             (5999, 1024, 5, "thresh"), (6000, 1025, 8, "thresh"), (6000, 512, 16, "topc"),
+             (6000, 512, 17, "thresh"), (65536, 1024, 9, "topc"), (65536, 1025, 9, "thresh")]
     code = (
         "import numpy as np, sys, yael_gb300 as yg; sys.path.insert(0, 'tests')\n"
         "from _util import knn_mismatches\n"
         "rng = np.random.default_rng(7)\n"
-        "for nq, nb, k, form in %r:\n"
-        "    b = rng.standard_normal((nb, 12)).astype(np.float32)\n"
-        "    q = rng.standard_normal((nq, 12)).astype(np.float32)\n"
-        "    idx, _ = yg.knn(q, b, nnn=k, precision='fp32')\n"
-        "    assert knn_mismatches(b, q, idx)[0] == 0, (nq, nb, k)\n" % (shapes,))
+        "for shapes, exact in ((%r, 0), (%r, 1)):\n"
+        "    for nq, nb, k, form in shapes:\n"
+        "        b, q = rng.standard_normal((nb, 12)), rng.standard_normal((nq, 12))\n"
+        "        if exact: b, q = np.round(20 * b), np.round(20 * q)\n"
+        "        b, q = b.astype(np.float32), q.astype(np.float32)\n"
+        "        idx, _ = yg.knn(q, b, nnn=k, precision='fp32')\n"
+        "        assert knn_mismatches(b, q, idx)[0] == 0, (nq, nb, k, exact)\n" % (real, exact))
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
     r = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True,
                        env=dict(os.environ, YAEL_GPU_TRACE="1"), timeout=300)
     assert r.returncode == 0, r.stderr[-2000:]
     first = [ln for ln in r.stderr.splitlines() if "knn level=0" in ln]
-    assert len(first) == len(shapes)
-    for (nq, nb, k, form), ln in zip(shapes, first):
+    assert len(first) == len(real + exact)
+    for (nq, nb, k, form), ln in zip(real + exact, first):
         assert f"pass={form} nq={nq} nb={nb} " in ln, ln

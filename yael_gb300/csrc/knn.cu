@@ -160,19 +160,28 @@ int list_length(int k, int exact, int nb) {
   return k <= 4 ? 8 : 2 * k;
 }
 
-// FP32, up to 8 neighbours of many queries among few rows: lists of 8 (k <= 4) or
-// 16, whose re-rank is a group of lanes a query; a threshold's candidates take a
-// block a query, 10 ns each however few they are.  The pass with lists is the slower
-// one, so the line is where the rows outweigh that.  The time by thresholds
-// over that by lists, d = 64: 100k queries, k = 2: 300 rows 2.3 times, 1,024 1.44, 2,048
-// 1.09, 3,000 0.94; 20k: 300 1.56, 1,024 1.08, 1,500 0.96; 6,000: 300 1.26, 1,024 1.19,
-// 2,048 0.95; 3,000: 300 0.89.  k = 8: 100k 300 1.88, 800 1.21, 1,500 0.91; 10k 300 1.42,
-// 512 1.08, 800 0.80; 3,000: 300 0.94.  (d = 16 gains more, d = 200 less: 10k, k = 2,
-// 800 rows 1.37 and 1.11.)
-bool fp32_lists(int k, int nb, int nq) {
-  if (k < 2 || k > 8) return false;
-  if (k <= 4) return nq >= 6000 && nb <= (nq >= 65536 ? 2048 : nq >= 16384 ? 1024 : 896);
-  return nq >= 8192 && nb <= (nq >= 65536 ? 896 : 512);
+// FP32, few neighbours of many queries among few rows: lists, whose re-rank is a
+// group of lanes a query; a threshold's candidates take a block a query, 10 ns each
+// however few they are.  The pass with lists is the slower one, and the more so the
+// longer they are, so the line is where the rows outweigh that.  The time of a
+// call by thresholds over that by lists, d = 64:
+//   lists of 8, real values (k <= 4): 100k queries: 300 rows 2.3, 1,024 1.44, 2,048
+//   1.09, 3,000 0.94; 20k: 300 1.56, 1,024 1.08, 1,500 0.96; 6,000: 300 1.26, 1,024
+//   1.19, 2,048 0.95; 3,000: 300 0.89
+//   of 16, real values (k = 5 to 8): 100k: 300 1.88, 800 1.21, 1,500 0.91; 10k: 300
+//   1.42, 512 1.08, 800 0.80; 3,000: 300 0.94
+//   of 2, 4, 8 and 16, exact values (k as long): 100k: 1,024 2.1, 1.8, 1.5 and 1.08,
+//   4,000 1.14, 0.97, 0.85 and 0.67; 10k: 512 1.8, 1.6, 1.3 and 1.04, 2,048 1.4, 1.2,
+//   0.9 and 0.6; 3,000: 1,024 1.4, 1.3, 1.2 and 0.86; 1,000: 300 0.85, 0.75, 0.9 and 0.7
+// (d = 16 gains more, d = 200 less: 10k, k = 2, 800 rows, real 1.37 and 1.11.)  Whether
+// values are exact is read from the device where lists of exact ones would serve.
+bool fp32_lists(int k, int exact, int nb, int nq) {
+  if (k < 2 || k > (exact ? 16 : 8)) return false;
+  if (!exact)
+    return k <= 4 ? nq >= 6000 && nb <= (nq >= 65536 ? 2048 : nq >= 16384 ? 1024 : 896)
+                  : nq >= 8192 && nb <= (nq >= 65536 ? 896 : 512);
+  if (k <= 4) return nq >= 3000 && nb <= (k == 2 ? 4096 : 2048);
+  return nq >= 6000 && nb <= (k <= 8 ? 1024 : 512) * (nq >= 65536 ? 2 : 1);
 }
 
 // out[q] = the least of n rows of nq values
@@ -380,7 +389,7 @@ int knn_batch(KnnJob &job, Ctx *ctx, cudaStream_t st, Small *dsmall, BaseOps *bo
   const int tile_n = bf16 ? TC_TILE_N : SIMT_TILE_N;
   const bool band = job.band_kth != nullptr;
   const bool prior = !band && job.prior_kth != nullptr;
-  const bool lists = !bf16 && !band && !prior && (job.lists || fp32_lists(k, nb, nq));
+  const bool lists = !bf16 && !band && !prior && (job.lists || fp32_lists(k, bstats_exact, nb, nq));
   const int tile_m = bf16 ? TC_TILE_M : lists ? 128 : simt_tile_m(nq, nb, ctx->num_sms);
   const int nqt = (int)ceil_div(nq, tile_m);
   const int ntb = (int)ceil_div(nb, tile_n);
@@ -772,7 +781,7 @@ int knn_batches(KnnJob &job, Ctx *ctx, cudaStream_t st, Small *dsmall, BaseOps *
     const int nqt = (int)ceil_div(nq, tile_m), ntb = (int)ceil_div(nb, tile_n);
     const int C = pow2_at_least(cn);
     size_t per_query;
-    if (!bf16 && !job.lists && !fp32_lists(k, nb, nq)) {
+    if (!bf16 && !job.lists && !fp32_lists(k, bexact, nb, nq)) {
       // running thresholds: up to 16 slots a region; else the regions' share of the
       // candidates, or the whole base where it is too short for a sample
       const int m = simt_tile_m(nq, nb, ctx->num_sms), nt = (int)ceil_div(nq, m);
@@ -914,12 +923,12 @@ int knn_device(KnnJob &job, Ctx *ctx, cudaStream_t st) {
     YG_CHECK(prep_rows(job.b, job.ldb, nb, d, 1.f, nullptr, bn32, nullptr, bres, nullptr, 0,
                        nullptr, 0, &dsmall->bs, st));
   }
-  // the lists of 2 to 16 neighbours depend on whether the base is exact class
-  // (only the tensor-core passes keep lists, and k = 1 and longer k do without: no
-  // host round trip then); every later read of the small state also checks the
+  // the lists of 2 to 16 neighbours depend on whether the base is exact class (k = 1
+  // and longer k do without, and so does FP32 where no lists would serve: no host
+  // round trip then); every later read of the small state also checks the
   // tensor-core passes' error flag
   int bexact = 0;
-  if (k > 1 && k <= 16 && job.prec != PREC_FP32) {
+  if (k > 1 && k <= 16 && (job.prec != PREC_FP32 || fp32_lists(k, 1, nb, nq))) {
     Small hs;
     YG_CHECK(read_small(ctx, dsmall, st, &hs));
     bexact = hs.bs.all_exact;

@@ -638,3 +638,19 @@ def test_fp32_form_by_size():
     assert len(first) == len(real + exact)
     for (nq, nb, k, form), ln in zip(real + exact, first):
         assert f"pass={form} nq={nq} nb={nb} " in ln, ln
+
+
+@pytest.mark.parametrize("prec", PRECS)
+@pytest.mark.parametrize("nb", [50, 100, 128, 129, 256, 300, 512, 513, 1025])
+def test_rerank_at_its_candidate_counts(nb, prec):
+    """Bases in which every row, or nearly, is a candidate, at the counts where the
+    re-rank changes its form: real values, integers with many ties, and integer
+    rows against real queries."""
+    rng = np.random.default_rng(nb)
+    b = rng.standard_normal((nb, 20)).astype(np.float32)
+    q = rng.standard_normal((70, 20)).astype(np.float32)
+    bi, qi = np.round(b).astype(np.float32), np.round(q).astype(np.float32)
+    for k in (17, 33, 50):
+        assert_exact(b, q, k, prec)
+        assert assert_exact(bi, qi, k, prec)["exact_class"] == 1
+        assert_exact(bi, q, k, prec)

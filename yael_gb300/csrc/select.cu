@@ -306,7 +306,16 @@ __device__ __forceinline__ double lanes_dist_pair(const float *qv, const float *
   return (double)hi + (double)lo;
 }
 
-__global__ void __launch_bounds__(RT) rerank_kernel(RerankArgs a, int Mp_alloc) {
+// LEAN: up to kLeanMax candidate slots.  Bound by the latency of a block's barriers,
+// so eight blocks an SM (32 registers) where the others hold five, and exact candidates
+// up to kSortAll are sorted at once.  Exact values, us, before and with it (and
+// before the counting): 20k queries, 40 candidates, k = 5: 160, 107 (107); 100
+// candidates, k = 17: 206, 149 (151); 80, k = 10: 176, 137 (137); 20k x 20k, k = 20: 223,
+// 156 (154).  With many candidates to gather the five do better: 10k x 200k, d = 128,
+// k = 100, real values: 545 and 631.
+constexpr int kLeanMax = 512, kSortAll = 128;
+template <bool LEAN>
+__global__ void __launch_bounds__(RT, LEAN ? 8 : 5) rerank_kernel(RerankArgs a, int Mp_alloc) {
   extern __shared__ __align__(16) unsigned char sm_raw[];
   unsigned long long *K = reinterpret_cast<unsigned long long *>(sm_raw);
   int *I = reinterpret_cast<int *>(K + Mp_alloc);
@@ -424,7 +433,7 @@ __global__ void __launch_bounds__(RT) rerank_kernel(RerankArgs a, int Mp_alloc) 
     // Up to RK candidates per thread stay in registers: the k-th approximate value
     // is counted out, and only what can be an answer is sorted.  More than that
     // (rare) are sorted as they are.
-    const bool few = M <= RK * RT;
+    const bool few = M <= RK * RT && !(LEAN && ex && k > 1 && M <= kSortAll);
     unsigned ckey[RK], cvalid = 0;
     int cid[RK];
     unsigned akey;
@@ -1540,8 +1549,9 @@ int rerank(const RerankArgs &a, cudaStream_t st) {
   while (Mp < Mmax) Mp <<= 1;
   // K (8 B) + I (4 B) + E (4 B) per slot, then the query row
   const size_t smem = (size_t)Mp * 16 + (size_t)a.d * 4 + 16;
-  YG_CHECK(ensure_smem((const void *)rerank_kernel, smem));
-  rerank_kernel<<<a.nq, RT, smem, st>>>(a, Mp);
+  const auto kern = Mp <= kLeanMax ? rerank_kernel<true> : rerank_kernel<false>;
+  YG_CHECK(ensure_smem((const void *)kern, smem));
+  kern<<<a.nq, RT, smem, st>>>(a, Mp);
   YG_LAUNCH_CHECK();
   return OK;
 }

@@ -654,3 +654,15 @@ def test_rerank_at_its_candidate_counts(nb, prec):
         assert_exact(b, q, k, prec)
         assert assert_exact(bi, qi, k, prec)["exact_class"] == 1
         assert_exact(bi, q, k, prec)
+
+
+@pytest.mark.parametrize("nq,nb,d,k", [(1, 40_000, 33, 2), (3, 25_000, 16, 20), (130, 12_000, 40, 5)])
+def test_fp32_sample_tiles_of_their_own(nq, nb, d, k):
+    """Few queries over a base that fills the GPU with 128-row query tiles and whose
+    sample does not: the sample's tiles have 32 rows."""
+    rng = np.random.default_rng(nb + k)
+    b = rng.standard_normal((nb, d)).astype(np.float32)
+    q = rng.standard_normal((nq, d)).astype(np.float32)
+    st = assert_exact(b, q, k, "fp32")
+    assert st["n_fallback"] == 0
+    assert_exact(np.round(4 * b).astype(np.float32), np.round(4 * q).astype(np.float32), k, "fp32")

@@ -575,11 +575,14 @@ int knn_batch(KnnJob &job, Ctx *ctx, cudaStream_t st, Small *dsmall, BaseOps *bo
       ScanSel ss;
       ss.mode = SCAN_TOPV;  // only the c-th value is needed
       ss.C = 16;
-      ss.tile_m = tile_m;
+      // (the sample's tiles by its own rows: 1 x 40k, d = 128, k = 2: 41 us with
+      // 128-row tiles, whose selection works through 127 rows of padding, 16 with 32)
+      ss.tile_m = bf16 ? tile_m : simt_tile_m(nq, sns, ctx->num_sms);
+      const int snqt = (int)ceil_div(nq, ss.tile_m);
       ss.blockmin = blockmin ? 1 : 0;
       const int nts = (int)ceil_div(sns, tile_n);
-      int nch = tune_chunks(TuneKey{2, job.prec, nqt, nts, ss.C, sample_form(tile_m, blockmin)},
-                                  choose_chunks(nqt, nts, ctx->num_sms, ctas_per_sm,
+      int nch = tune_chunks(TuneKey{2, job.prec, snqt, nts, ss.C, sample_form(ss.tile_m, blockmin)},
+                                  choose_chunks(snqt, nts, ctx->num_sms, ctas_per_sm,
                                                 imin(2, min_tiles)), 64,
                                   ctx->num_sms * ctas_per_sm, &sample_ticket);
       if (c > ss.C) nch = imax(nch, 2);  // the lists together hold the c-th value

@@ -666,3 +666,15 @@ def test_fp32_sample_tiles_of_their_own(nq, nb, d, k):
     st = assert_exact(b, q, k, "fp32")
     assert st["n_fallback"] == 0
     assert_exact(np.round(4 * b).astype(np.float32), np.round(4 * q).astype(np.float32), k, "fp32")
+
+
+@pytest.mark.parametrize("prec", PRECS)
+@pytest.mark.parametrize("nq,nb,k", [(2000, 30_000, 300), (300, 30_000, 315), (2000, 9000, 250)])
+def test_rerank_slots_of_long_lists(nq, nb, k, prec):
+    """Candidate slots of 8,192 cut to 4,096 where they hold the expected candidates
+    three times: exact, with next to no rejected query."""
+    rng = np.random.default_rng(nb + k)
+    b = rng.standard_normal((nb, 24)).astype(np.float32)
+    q = rng.standard_normal((nq, 24)).astype(np.float32)
+    st = assert_exact(b, q, k, prec)
+    assert st["n_band"] <= 3 and st["n_fallback"] == 0

@@ -143,7 +143,7 @@ inline int sample_rank_3(int stride) { return stride >= 200 ? 12 : 13; }
 // ldb floats); bn: ||b||^2 as float with stride bn_stride (L2 only).
 // Base tiles are 128 rows.  Reported base ids are j (row index in this view).
 // THRESH regions are chunks (halves = 1); a TOPV pass with blockmin lists the
-// minima of 8 rows.  TOPC lists are the allocation-free call's.
+// minima of 8 rows.  TOPC: lists of 2 to 32 entries a chunk.
 constexpr int SIMT_TILE_N = 128;
 int simt_tile_m(int nq, int nb, int num_sms);
 int simt_scan(const float *q, long ldq, int nq, const float *b, long ldb, int nb,

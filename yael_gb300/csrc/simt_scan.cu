@@ -1,8 +1,9 @@
 // FP32 CUDA-core distance passes.
 //   * rows_kernel: thresholds, running thresholds (k = 1) and the threshold
 //     sample of the plain k-NN pipeline;
-//   * simt_scan_kernel: lists of C entries per chunk, for the allocation-free
-//     call, whose scratch they bound.
+//   * simt_scan_kernel: lists of C entries per chunk, for many queries among few
+//     rows (fp32_lists, knn.cu), for exact ties by the thousand, and for the
+//     allocation-free call, whose scratch they bound.
 // (See scan.cuh for the selection contract.)
 #include <limits.h>
 #include <math.h>
